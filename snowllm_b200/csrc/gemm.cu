@@ -3,7 +3,8 @@
 // This is the matrix product of the true 32-bit path (plain FFMA: no TF32, no split
 // tricks), and the reference kernel that the tensor-core products are checked against.
 // Each output element is one thread's sum over k = 0..K-1 in ascending order, so a row's
-// result does not depend on how many other rows the launch holds.
+// result does not depend on how many other rows the launch holds, nor on which of the two
+// kernels below forms it.
 //
 // Grouped form (routed experts): rows are sorted by group; group e owns rows
 // [offsets[e], offsets[e+1]) and multiplies them with W + e*N*K.  `a_rows` gathers A: the
@@ -11,10 +12,6 @@
 // (the role of snowllm/ops/gemm.py:33-41 and of the expert products in
 // snowllm/ops/inference.py:60-76)
 #include "common.cuh"
-
-#define BM 64
-#define BN 64
-#define BK 16
 
 template <typename T> struct Vec4;
 template <> struct Vec4<float> {
@@ -32,22 +29,43 @@ template <> struct Vec4<bf16> {
   }
 };
 
+// Four values from k on of a row (not ok: zeros), zeros past K; vec: by one vector load where all four are there.
 template <typename T>
-__device__ __forceinline__ void load4(const T* row, int k, int K, bool row_ok, bool vec, float (&v)[4]) {
-  if (!row_ok) { v[0] = v[1] = v[2] = v[3] = 0.f; return; }
+__device__ __forceinline__ void load4(const T* row, int k, int K, bool ok, bool vec, float (&v)[4]) {
+  if (!ok) { v[0] = v[1] = v[2] = v[3] = 0.f; return; }
   if (vec && k + 3 < K) { Vec4<T>::load(row + k, v); return; }
 #pragma unroll
   for (int i = 0; i < 4; ++i) v[i] = (k + i < K) ? to_f<T>(row[k + i]) : 0.f;
 }
 
-template <typename T, typename OutT>
-__global__ void __launch_bounds__(256)
-gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ W, OutT* __restrict__ C, int M,
+// Two independent fused multiply-adds by one instruction (fma.rn.f32x2), each rounded as fmaf rounds: acc += (a, a) * w.
+__device__ __forceinline__ void fma2(unsigned long long& acc, float a, unsigned long long w) {
+  unsigned long long aa;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(aa), "l"(w));
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// ---------------------------------------------------------------------------------------
+// Many rows: tiles of BM x BN, a thread owns TM x TN outputs (TN columns as runs of four, BN / (TN / 4) apart, so that
+// a warp's shared-memory reads are consecutive).  Bound by the FMA pipe; the multiply-adds go two to an instruction,
+// which leaves half of the issue slots to the loads from shared memory.  The next BK columns of both operands are on
+// their way to registers while the current ones are multiplied; shared memory is double buffered, one barrier a step.
+#define BK 16
+
+template <typename T, typename OutT, int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__(BM * BN / (TM * TN), BM * BN / (TM * TN) >= 256 ? 2 : (TM * TN >= 64 ? 3 : 4))
+gemm_tile_kernel(const T* __restrict__ A, const T* __restrict__ W, OutT* __restrict__ C, int M,
                  int N, int K, const int* __restrict__ a_rows, int a_div,
                  const int* __restrict__ offsets, int vec) {
+  constexpr int THREADS = BM * BN / (TM * TN), TX = BN / TN, RUNS = TN / 4;
+  constexpr int A4 = BM * (BK / 4) / THREADS, W4 = BN * (BK / 4) / THREADS;       // vectors a thread brings in a step
+  static_assert(A4 * THREADS == BM * (BK / 4) && W4 * THREADS == BN * (BK / 4) && TN % 4 == 0 && TM % 4 == 0, "tile");
   pdl_begin();
-  __shared__ __align__(16) float As[BK][BM + 4];
-  __shared__ __align__(16) float Ws[BK][BN + 4];
+  __shared__ __align__(16) float As[2][BK][BM + 4];
+  __shared__ __align__(16) float Ws[2][BK][BN + 4];
   int row_begin = 0, row_end = M;
   const T* Wg = W;
   if (offsets) {
@@ -60,55 +78,248 @@ gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ W, OutT* __restr
   const int n0 = blockIdx.x * BN;
   const int tid = threadIdx.x;
   const int lr = tid >> 2, lk = (tid & 3) * 4;       // tile-load coordinates
-  const int ty = tid >> 4, tx = tid & 15;            // 4x4 outputs at (ty*4, tx*4)
+  const int ty = tid / TX, tx = tid % TX;
 
-  const int arow = m0 + lr;
-  const bool a_ok = arow < row_end;
-  const T* a_ptr = nullptr;
-  if (a_ok) a_ptr = A + (size_t)(a_rows ? a_rows[arow] / a_div : arow) * K;
-  const int wrow = n0 + lr;
-  const bool w_ok = wrow < N;
-  const T* w_ptr = w_ok ? Wg + (size_t)wrow * K : nullptr;
+  int a_row[A4];                                     // -1: past the rows
+#pragma unroll
+  for (int i = 0; i < A4; ++i) {
+    const int r = m0 + lr + i * (THREADS / 4);
+    a_row[i] = r < row_end ? (a_rows ? a_rows[r] / a_div : r) : -1;
+  }
+  const T* w_ptr = Wg + (size_t)(n0 + lr) * K;
+  float av[A4][4], wv[W4][4];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < A4; ++i) load4<T>(A + (size_t)a_row[i] * K, k0 + lk, K, a_row[i] >= 0, vec, av[i]);
+#pragma unroll
+    for (int i = 0; i < W4; ++i)
+      load4<T>(w_ptr + (size_t)(i * (THREADS / 4)) * K, k0 + lk, K, n0 + lr + i * (THREADS / 4) < N, vec, wv[i]);
+  };
+  auto stage = [&](int b) {
+#pragma unroll
+    for (int i = 0; i < A4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) As[b][lk + j][lr + i * (THREADS / 4)] = av[i][j];
+#pragma unroll
+    for (int i = 0; i < W4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) Ws[b][lk + j][lr + i * (THREADS / 4)] = wv[i][j];
+  };
 
-  float acc[4][4];
+  unsigned long long acc[TM][TN / 2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
 
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    float av[4], wv[4];
-    load4<T>(a_ptr, k0 + lk, K, a_ok, vec, av);
-    load4<T>(w_ptr, k0 + lk, K, w_ok, vec, wv);
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      As[lk + i][lr] = av[i];
-      Ws[lk + i][lr] = wv[i];
-    }
-    __syncthreads();
+  fetch(0);
+  stage(0);
+  __syncthreads();
+  const int steps = (K + BK - 1) / BK;
+  for (int s = 0; s < steps; ++s) {
+    const int b = s & 1;
+    if (s + 1 < steps) fetch((s + 1) * BK);
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
-      const float4 a4 = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-      const float4 w4 = *reinterpret_cast<const float4*>(&Ws[k][tx * 4]);
-      const float a[4] = {a4.x, a4.y, a4.z, a4.w};
-      const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+      float a[TM];
+      unsigned long long w[TN / 2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < TM / 4; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(&As[b][k][ty * TM + 4 * i]);
+        a[4 * i] = v.x; a[4 * i + 1] = v.y; a[4 * i + 2] = v.z; a[4 * i + 3] = v.w;
+      }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+      for (int j = 0; j < RUNS; ++j) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&Ws[b][k][j * (BN / RUNS) + tx * 4]);
+        w[2 * j] = v.x; w[2 * j + 1] = v.y;
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) fma2(acc[i][j], a[i], w[j]);
+    }
+    if (s + 1 < steps) {
+      stage(b ^ 1);                                   // read last before the barrier of the step before
+      __syncthreads();
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = m0 + ty * 4 + i;
+  for (int i = 0; i < TM; ++i) {
+    const int r = m0 + ty * TM + i;
     if (r >= row_end) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int cidx = n0 + tx * 4 + j;
-      if (cidx < N) C[(size_t)r * N + cidx] = from_f<OutT>(acc[i][j]);
+    for (int j = 0; j < TN / 2; ++j) {
+      const int c = n0 + (j / 2) * (BN / RUNS) + tx * 4 + (j & 1) * 2;
+      float lo, hi;
+      unpack2(acc[i][j], lo, hi);
+      if (c < N) C[(size_t)r * N + c] = from_f<OutT>(lo);
+      if (c + 1 < N) C[(size_t)r * N + c + 1] = from_f<OutT>(hi);
     }
   }
+}
+
+// ---------------------------------------------------------------------------------------
+// Few rows (decode), float: bound by the read of W.  A block owns FR_COLS columns (rows of W); FR_STAGES chunks of
+// FR_K of their values are on their way through cp.async at a time, W's first chunks from before the wait for the
+// kernel before.  A lane owns one column and R rows: half-warps take rows of their own, warps more.  The sum over k stays one
+// thread's, in order: with K chained multiply-adds of four cycles a block cannot end sooner than 4 K cycles (4.3 us at
+// K = 2,048), which the narrow blocks of 16 columns share out over as many SMs as N gives.
+#define FR_COLS 16
+#define FR_K 128
+#define FR_STAGES 4
+#define FR_PITCH (FR_K + 4)        // an odd number of 16-byte units: eight lanes on eight rows hit different banks
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+               :: "r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem), "r"(ok ? 16 : 0));
+}
+
+template <int R, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
+gemm_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
+                const int* __restrict__ a_rows, int a_div, const int* __restrict__ offsets) {
+  constexpr int ROWS = 2 * R * WARPS, THREADS = WARPS * 32;
+  extern __shared__ __align__(16) float sm[];          // per stage: FR_COLS rows of W, then ROWS rows of A
+  constexpr int STAGE = (FR_COLS + ROWS) * FR_PITCH;
+  const int tid = threadIdx.x, n0 = blockIdx.x * FR_COLS;
+  const int chunks = (K + FR_K - 1) / FR_K;
+  const float* Wg = W;
+  int row_begin = 0, row_end = M;
+  auto load_w = [&](int c) {
+    float* to = sm + (c % FR_STAGES) * STAGE;
+    for (int i = tid; i < FR_COLS * (FR_K / 4); i += THREADS) {
+      const int r = i / (FR_K / 4), k = c * FR_K + (i % (FR_K / 4)) * 4;
+      const bool ok = n0 + r < N && k < K;             // K is a multiple of 4
+      cp_async16(to + r * FR_PITCH + (i % (FR_K / 4)) * 4, Wg + (ok ? (size_t)(n0 + r) * K + k : 0), ok);
+    }
+  };
+  if (offsets == nullptr) {                            // W is a constant: its first chunks need not wait
+#pragma unroll
+    for (int c = 0; c < FR_STAGES - 1; ++c)
+      if (c < chunks) load_w(c);
+  }
+  pdl_begin();
+  if (offsets) {
+    row_begin = offsets[blockIdx.y];
+    row_end = offsets[blockIdx.y + 1];
+    Wg = W + (size_t)blockIdx.y * N * K;
+    if (row_begin >= row_end) return;
+  }
+  const int lane = tid & 31, col = lane & 15;
+  const int first = ((tid >> 5) * 2 + (lane >> 4)) * R;              // this lane's rows of a pass
+  bool w_there = offsets == nullptr;
+  for (int m0 = row_begin; m0 < row_end; m0 += ROWS) {
+    auto load_a = [&](int c) {
+      float* to = sm + (c % FR_STAGES) * STAGE + FR_COLS * FR_PITCH;
+      for (int i = tid; i < ROWS * (FR_K / 4); i += THREADS) {
+        const int r = m0 + i / (FR_K / 4), k = c * FR_K + (i % (FR_K / 4)) * 4;
+        const bool ok = r < row_end && k < K;
+        const size_t src = ok ? (size_t)(a_rows ? a_rows[r] / a_div : r) * K + k : 0;
+        cp_async16(to + (i / (FR_K / 4)) * FR_PITCH + (i % (FR_K / 4)) * 4, A + src, ok);
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < FR_STAGES - 1; ++c) {
+      if (c < chunks) {
+        if (!w_there) load_w(c);
+        load_a(c);
+      }
+      asm volatile("cp.async.commit_group;");
+    }
+    w_there = false;
+    float acc[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) acc[i] = 0.f;
+    for (int c = 0; c < chunks; ++c) {
+      asm volatile("cp.async.wait_group %0;" :: "n"(FR_STAGES - 2));
+      __syncthreads();                                 // chunk c is there, and everyone is done with chunk c - 1
+      if (c + FR_STAGES - 1 < chunks) {
+        load_w(c + FR_STAGES - 1);
+        load_a(c + FR_STAGES - 1);
+      }
+      asm volatile("cp.async.commit_group;");
+      const float* ws = sm + (c % FR_STAGES) * STAGE + col * FR_PITCH;
+      const float* as = sm + (c % FR_STAGES) * STAGE + (FR_COLS + first) * FR_PITCH;
+#pragma unroll 8
+      for (int k = 0; k < FR_K; k += 4) {              // past K both operands are zeros
+        const float4 w = *reinterpret_cast<const float4*>(ws + k);
+        float4 a[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * FR_PITCH + k);
+#pragma unroll
+        for (int i = 0; i < R; ++i) acc[i] = fmaf(a[i].x, w.x, acc[i]);
+#pragma unroll
+        for (int i = 0; i < R; ++i) acc[i] = fmaf(a[i].y, w.y, acc[i]);
+#pragma unroll
+        for (int i = 0; i < R; ++i) acc[i] = fmaf(a[i].z, w.z, acc[i]);
+#pragma unroll
+        for (int i = 0; i < R; ++i) acc[i] = fmaf(a[i].w, w.w, acc[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int r = m0 + first + i;
+      if (r < row_end && n0 + col < N) C[(size_t)r * N + n0 + col] = acc[i];
+    }
+    asm volatile("cp.async.wait_group 0;");
+    __syncthreads();                                   // the next pass writes the stages again
+  }
+}
+
+struct SimtArgs {
+  const void *A, *W;
+  void* C;
+  int M, N, K;
+  const int* a_rows;
+  int a_div;
+  const int* offsets;
+  int groups, rows, vec;           // rows: the most that one group (or the product) can own
+  cudaStream_t stream;
+};
+
+template <typename T, typename OutT, int BM, int BN, int TM, int TN>
+static int launch_tile(const SimtArgs& p) {
+  dim3 grid((p.N + BN - 1) / BN, (p.rows + BM - 1) / BM, p.offsets ? p.groups : 1);
+  if (grid.y > 65535u || grid.z > 65535u) return SNK_ERR_SIZE;
+  snk_launch(gemm_tile_kernel<T, OutT, BM, BN, TM, TN>, grid, dim3(BM * BN / (TM * TN)), 0, p.stream,
+             static_cast<const T*>(p.A), static_cast<const T*>(p.W), static_cast<OutT*>(p.C), p.M, p.N, p.K, p.a_rows,
+             p.a_div, p.offsets, p.vec);
+  SNK_LAUNCH_CHECK();
+  return 0;
+}
+
+template <int R, int WARPS>
+static int launch_few(const SimtArgs& p) {
+  constexpr int smem = FR_STAGES * (FR_COLS + 2 * R * WARPS) * FR_PITCH * (int)sizeof(float);
+  static_assert(smem <= 227 * 1024, "stages");
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<R, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  snk_launch(gemm_few_kernel<R, WARPS>, dim3((p.N + FR_COLS - 1) / FR_COLS, p.offsets ? p.groups : 1), dim3(WARPS * 32), smem,
+             p.stream, static_cast<const float*>(p.A), static_cast<const float*>(p.W), static_cast<float*>(p.C), p.M, p.N,
+             p.K, p.a_rows, p.a_div, p.offsets);
+  SNK_LAUNCH_CHECK();
+  return 0;
+}
+
+#define FR_MAX_ROWS 16             // up to here (grouped: up to 4 rows a group on average) W's read is the bound
+
+// The tile with the least work on the busiest SM: rounds of tiles over 148 SMs times the tile's area, over the share of
+// the FMA rate that its shared-memory reads leave.
+template <typename T, typename OutT>
+static int launch_tiles(const SimtArgs& p) {
+  const int G = p.offsets ? p.groups : 1;
+  const long long mean = p.offsets ? (p.M + G - 1) / G : p.M;      // rows of a group
+  auto cost = [&](int bm, int bn, double rate) {
+    const long long tiles = (long long)G * ((mean + bm - 1) / bm) * ((p.N + bn - 1) / bn);
+    return (double)((tiles + 147) / 148) * bm * bn / rate;
+  };
+  const double c128 = cost(128, 128, 1.0), c64w = cost(64, 128, 0.95), c64 = cost(64, 64, 0.8), c32 = cost(32, 64, 0.6);
+  if (c128 <= c64w && c128 <= c64 && c128 <= c32) return launch_tile<T, OutT, 128, 128, 8, 8>(p);
+  if (c64w <= c64 && c64w <= c32) return launch_tile<T, OutT, 64, 128, 8, 8>(p);
+  if (c64 <= c32) return launch_tile<T, OutT, 64, 64, 4, 8>(p);
+  return launch_tile<T, OutT, 32, 64, 4, 4>(p);
 }
 
 // out_f32: C is float whatever the compute dtype.  groups <= 1 and offsets == nullptr: plain
@@ -120,22 +331,21 @@ SNK_API int snk_gemm_simt(const void* A, const void* W, void* C, int M, int N, i
   if (K <= 0) return SNK_ERR_SIZE;
   const int rows = offsets ? max_rows_per_group : M;
   if (rows <= 0) return 0;
-  dim3 grid((N + BN - 1) / BN, (rows + BM - 1) / BM, offsets ? groups : 1);
-  if (grid.y > 65535u || grid.z > 65535u) return SNK_ERR_SIZE;
   const size_t esz = dtype == SNK_F32 ? 4 : 2;
   const int vec = (K % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0) &&
                   (((size_t)K * esz) % 8 == 0);
-  if (a_div <= 0) a_div = 1;
+  const SimtArgs p{A, W, C, M, N, K, a_rows, a_div <= 0 ? 1 : a_div, offsets, groups, rows, vec, stream};
+  if (dtype == SNK_F32 && vec && (offsets ? (long long)M <= 4ll * groups : M <= FR_MAX_ROWS) && (!offsets || groups <= 65535)) {
+    // rows of a pass: those of the product, or about twice a group's mean (fuller groups take more passes)
+    const int pass = offsets ? 2 * ((M + groups - 1) / groups) : M;
+    if (pass <= 2) return launch_few<1, 1>(p);
+    if (pass <= 4) return launch_few<2, 1>(p);
+    if (pass <= 8) return launch_few<2, 2>(p);
+    return launch_few<4, 2>(p);
+  }
   SNK_DISPATCH(dtype, {
-    if (out_f32 || dtype == SNK_F32)
-      snk_launch(gemm_simt_kernel<T, float>, dim3(grid), dim3(256), 0, stream, 
-          static_cast<const T*>(A), static_cast<const T*>(W), static_cast<float*>(C), M, N, K,
-          a_rows, a_div, offsets, vec);
-    else
-      snk_launch(gemm_simt_kernel<T, T>, dim3(grid), dim3(256), 0, stream, 
-          static_cast<const T*>(A), static_cast<const T*>(W), static_cast<T*>(C), M, N, K, a_rows,
-          a_div, offsets, vec);
+    if (out_f32 || dtype == SNK_F32) return launch_tiles<T, float>(p);
+    return launch_tiles<T, T>(p);
   });
-  SNK_LAUNCH_CHECK();
   return 0;
 }
