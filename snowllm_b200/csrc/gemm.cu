@@ -53,6 +53,9 @@ __device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& 
 // a warp's shared-memory reads are consecutive).  Bound by the FMA pipe; the multiply-adds go two to an instruction,
 // which leaves half of the issue slots to the loads from shared memory.  The next BK columns of both operands are on
 // their way to registers while the current ones are multiplied; shared memory is double buffered, one barrier a step.
+// Measured (TFLOP/s; 74 is the pipe's rate, 34 the 64 x 64 single-buffered tile before): 2,048 x 16,384 x 2,048 53, 509 x 16,384
+// x 2,048 49, 509 x 2,048 x 2,048 32 (128 tiles: one a SM).  Tried and slower: A stored twice for the paired operand
+// (40), single multiply-adds (47), 8 columns a step (49), 16 x 8 outputs a thread.
 #define BK 16
 
 template <typename T, typename OutT, int BM, int BN, int TM, int TN>
@@ -77,13 +80,13 @@ gemm_tile_kernel(const T* __restrict__ A, const T* __restrict__ W, OutT* __restr
   if (m0 >= row_end) return;
   const int n0 = blockIdx.x * BN;
   const int tid = threadIdx.x;
-  const int lr = tid >> 2, lk = (tid & 3) * 4;       // tile-load coordinates
+  const int lr = tid / (BK / 4), lk = (tid % (BK / 4)) * 4;       // tile-load coordinates
   const int ty = tid / TX, tx = tid % TX;
 
   int a_row[A4];                                     // -1: past the rows
 #pragma unroll
   for (int i = 0; i < A4; ++i) {
-    const int r = m0 + lr + i * (THREADS / 4);
+    const int r = m0 + lr + i * (THREADS / (BK / 4));
     a_row[i] = r < row_end ? (a_rows ? a_rows[r] / a_div : r) : -1;
   }
   const T* w_ptr = Wg + (size_t)(n0 + lr) * K;
@@ -93,17 +96,17 @@ gemm_tile_kernel(const T* __restrict__ A, const T* __restrict__ W, OutT* __restr
     for (int i = 0; i < A4; ++i) load4<T>(A + (size_t)a_row[i] * K, k0 + lk, K, a_row[i] >= 0, vec, av[i]);
 #pragma unroll
     for (int i = 0; i < W4; ++i)
-      load4<T>(w_ptr + (size_t)(i * (THREADS / 4)) * K, k0 + lk, K, n0 + lr + i * (THREADS / 4) < N, vec, wv[i]);
+      load4<T>(w_ptr + (size_t)(i * (THREADS / (BK / 4))) * K, k0 + lk, K, n0 + lr + i * (THREADS / (BK / 4)) < N, vec, wv[i]);
   };
   auto stage = [&](int b) {
 #pragma unroll
     for (int i = 0; i < A4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) As[b][lk + j][lr + i * (THREADS / 4)] = av[i][j];
+      for (int j = 0; j < 4; ++j) As[b][lk + j][lr + i * (THREADS / (BK / 4))] = av[i][j];
 #pragma unroll
     for (int i = 0; i < W4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) Ws[b][lk + j][lr + i * (THREADS / 4)] = wv[i][j];
+      for (int j = 0; j < 4; ++j) Ws[b][lk + j][lr + i * (THREADS / (BK / 4))] = wv[i][j];
   };
 
   unsigned long long acc[TM][TN / 2];
@@ -159,41 +162,53 @@ gemm_tile_kernel(const T* __restrict__ A, const T* __restrict__ W, OutT* __restr
 }
 
 // ---------------------------------------------------------------------------------------
-// Few rows (decode), float: bound by the read of W.  A block owns FR_COLS columns (rows of W); FR_STAGES chunks of
-// FR_K of their values are on their way through cp.async at a time, W's first chunks from before the wait for the
-// kernel before.  A lane owns one column and R rows: half-warps take rows of their own, warps more.  The sum over k stays one
-// thread's, in order: with K chained multiply-adds of four cycles a block cannot end sooner than 4 K cycles (4.3 us at
-// K = 2,048), which the narrow blocks of 16 columns share out over as many SMs as N gives.
+// Few rows (decode), float: bound by the read of W.  A block owns FR_COLS columns (rows of W) and FR_STAGES chunks of
+// FR_K of their values, which four warps of its own bring in by cp.async (a row of a chunk is one instruction of a warp),
+// W's first chunks from before the wait for the kernel before.  The other warps multiply: a lane owns one column and R
+// rows, half-warps rows of their own.  The sum over k stays one thread's, in order: with K chained multiply-adds of four
+// cycles a block cannot end sooner than 4 K cycles (4.3 us at K = 2,048), so nothing but them and the reads of their
+// operands is left to those warps, and the narrow blocks of 16 columns share the columns out over as many SMs as N gives.
+// Measured, 4 rows (in a replayed chain; the 64 x 64 tile before): 2,048 x 2,048 9.4 us (146), 14,336 x 2,048 31 us (190),
+// 2,048 x 7,168 28 us (523), 65,536 x 2,048 108 us = 5.0 TB/s; with the loads in the warps that multiply 19, 41, 66, 130 us.
 #define FR_COLS 16
 #define FR_K 128
 #define FR_STAGES 4
 #define FR_PITCH (FR_K + 4)        // an odd number of 16-byte units: eight lanes on eight rows hit different banks
+#define FR_LOADERS 4               // warps that load
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool ok) {
+__device__ __forceinline__ void cp_async16(float* smem, const float* gmem, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
                :: "r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem), "r"(ok ? 16 : 0));
 }
 
 template <int R, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32)
+__global__ void __launch_bounds__((WARPS + FR_LOADERS) * 32)
 gemm_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
                 const int* __restrict__ a_rows, int a_div, const int* __restrict__ offsets) {
-  constexpr int ROWS = 2 * R * WARPS, THREADS = WARPS * 32;
+  constexpr int ROWS = 2 * R * WARPS;
+  constexpr int W_EACH = FR_COLS / FR_LOADERS, A_EACH = (ROWS + FR_LOADERS - 1) / FR_LOADERS;
   extern __shared__ __align__(16) float sm[];          // per stage: FR_COLS rows of W, then ROWS rows of A
   constexpr int STAGE = (FR_COLS + ROWS) * FR_PITCH;
-  const int tid = threadIdx.x, n0 = blockIdx.x * FR_COLS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n0 = blockIdx.x * FR_COLS;
+  const int loader = warp - WARPS;                     // 0..3: a warp that loads
   const int chunks = (K + FR_K - 1) / FR_K;
-  const float* Wg = W;
   int row_begin = 0, row_end = M;
-  auto load_w = [&](int c) {
-    float* to = sm + (c % FR_STAGES) * STAGE;
-    for (int i = tid; i < FR_COLS * (FR_K / 4); i += THREADS) {
-      const int r = i / (FR_K / 4), k = c * FR_K + (i % (FR_K / 4)) * 4;
-      const bool ok = n0 + r < N && k < K;             // K is a multiple of 4
-      cp_async16(to + r * FR_PITCH + (i % (FR_K / 4)) * 4, Wg + (ok ? (size_t)(n0 + r) * K + k : 0), ok);
-    }
+  const float* w_src[W_EACH];                          // a loader's rows of W (a row past N loads zeros)
+  auto point_w = [&](const float* Wg) {
+#pragma unroll
+    for (int i = 0; i < W_EACH; ++i)
+      w_src[i] = Wg + (size_t)min(n0 + loader + i * FR_LOADERS, N - 1) * K + lane * 4;
   };
-  if (offsets == nullptr) {                            // W is a constant: its first chunks need not wait
+  auto load_w = [&](int c) {
+    float* to = sm + (c % FR_STAGES) * STAGE + loader * FR_PITCH + lane * 4;
+    const bool in = c * FR_K + lane * 4 < K;           // K is a multiple of 4
+#pragma unroll
+    for (int i = 0; i < W_EACH; ++i)
+      cp_async16(to + i * (FR_LOADERS * FR_PITCH), w_src[i] + (in ? c * FR_K : -lane * 4),
+                 in && n0 + loader + i * FR_LOADERS < N);
+  };
+  if (offsets == nullptr && loader >= 0) {             // W is a constant: its first chunks need not wait
+    point_w(W);
 #pragma unroll
     for (int c = 0; c < FR_STAGES - 1; ++c)
       if (c < chunks) load_w(c);
@@ -202,45 +217,57 @@ gemm_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
   if (offsets) {
     row_begin = offsets[blockIdx.y];
     row_end = offsets[blockIdx.y + 1];
-    Wg = W + (size_t)blockIdx.y * N * K;
     if (row_begin >= row_end) return;
+    point_w(W + (size_t)blockIdx.y * N * K);
   }
-  const int lane = tid & 31, col = lane & 15;
-  const int first = ((tid >> 5) * 2 + (lane >> 4)) * R;              // this lane's rows of a pass
+  const int col = lane & 15;
+  const int first = (warp * 2 + (lane >> 4)) * R;      // a multiplying lane's rows of a pass
   bool w_there = offsets == nullptr;
   for (int m0 = row_begin; m0 < row_end; m0 += ROWS) {
-    auto load_a = [&](int c) {
-      float* to = sm + (c % FR_STAGES) * STAGE + FR_COLS * FR_PITCH;
-      for (int i = tid; i < ROWS * (FR_K / 4); i += THREADS) {
-        const int r = m0 + i / (FR_K / 4), k = c * FR_K + (i % (FR_K / 4)) * 4;
-        const bool ok = r < row_end && k < K;
-        const size_t src = ok ? (size_t)(a_rows ? a_rows[r] / a_div : r) * K + k : 0;
-        cp_async16(to + (i / (FR_K / 4)) * FR_PITCH + (i % (FR_K / 4)) * 4, A + src, ok);
-      }
-    };
+    const float* a_src[A_EACH];
+    bool a_ok[A_EACH];
 #pragma unroll
-    for (int c = 0; c < FR_STAGES - 1; ++c) {
-      if (c < chunks) {
-        if (!w_there) load_w(c);
-        load_a(c);
+    for (int i = 0; i < A_EACH; ++i) {
+      const int r = loader + i * FR_LOADERS;
+      a_ok[i] = loader >= 0 && r < ROWS && m0 + r < row_end;
+      a_src[i] = A + (a_ok[i] ? (size_t)(a_rows ? a_rows[m0 + r] / a_div : m0 + r) * K + lane * 4 : 0);
+    }
+    auto load_a = [&](int c) {
+      float* to = sm + (c % FR_STAGES) * STAGE + (FR_COLS + loader) * FR_PITCH + lane * 4;
+      const bool in = c * FR_K + lane * 4 < K;
+#pragma unroll
+      for (int i = 0; i < A_EACH; ++i)
+        if (loader + i * FR_LOADERS < ROWS)
+          cp_async16(to + i * (FR_LOADERS * FR_PITCH), in && a_ok[i] ? a_src[i] + c * FR_K : A, in && a_ok[i]);
+    };
+    if (loader >= 0) {
+#pragma unroll
+      for (int c = 0; c < FR_STAGES - 1; ++c) {
+        if (c < chunks) {
+          if (!w_there) load_w(c);
+          load_a(c);
+        }
+        asm volatile("cp.async.commit_group;");
       }
-      asm volatile("cp.async.commit_group;");
     }
     w_there = false;
     float acc[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) acc[i] = 0.f;
     for (int c = 0; c < chunks; ++c) {
-      asm volatile("cp.async.wait_group %0;" :: "n"(FR_STAGES - 2));
+      if (loader >= 0) asm volatile("cp.async.wait_group %0;" :: "n"(FR_STAGES - 2));
       __syncthreads();                                 // chunk c is there, and everyone is done with chunk c - 1
-      if (c + FR_STAGES - 1 < chunks) {
-        load_w(c + FR_STAGES - 1);
-        load_a(c + FR_STAGES - 1);
+      if (loader >= 0) {
+        if (c + FR_STAGES - 1 < chunks) {
+          load_w(c + FR_STAGES - 1);
+          load_a(c + FR_STAGES - 1);
+        }
+        asm volatile("cp.async.commit_group;");
+        continue;
       }
-      asm volatile("cp.async.commit_group;");
       const float* ws = sm + (c % FR_STAGES) * STAGE + col * FR_PITCH;
       const float* as = sm + (c % FR_STAGES) * STAGE + (FR_COLS + first) * FR_PITCH;
-#pragma unroll 8
+#pragma unroll
       for (int k = 0; k < FR_K; k += 4) {              // past K both operands are zeros
         const float4 w = *reinterpret_cast<const float4*>(ws + k);
         float4 a[R];
@@ -256,12 +283,15 @@ gemm_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
         for (int i = 0; i < R; ++i) acc[i] = fmaf(a[i].w, w.w, acc[i]);
       }
     }
+    if (loader < 0) {
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int r = m0 + first + i;
-      if (r < row_end && n0 + col < N) C[(size_t)r * N + n0 + col] = acc[i];
+      for (int i = 0; i < R; ++i) {
+        const int r = m0 + first + i;
+        if (r < row_end && n0 + col < N) C[(size_t)r * N + n0 + col] = acc[i];
+      }
+    } else {
+      asm volatile("cp.async.wait_group 0;");
     }
-    asm volatile("cp.async.wait_group 0;");
     __syncthreads();                                   // the next pass writes the stages again
   }
 }
@@ -296,7 +326,7 @@ static int launch_few(const SimtArgs& p) {
     cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<R, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
   }
-  snk_launch(gemm_few_kernel<R, WARPS>, dim3((p.N + FR_COLS - 1) / FR_COLS, p.offsets ? p.groups : 1), dim3(WARPS * 32), smem,
+  snk_launch(gemm_few_kernel<R, WARPS>, dim3((p.N + FR_COLS - 1) / FR_COLS, p.offsets ? p.groups : 1), dim3((WARPS + FR_LOADERS) * 32), smem,
              p.stream, static_cast<const float*>(p.A), static_cast<const float*>(p.W), static_cast<float*>(p.C), p.M, p.N,
              p.K, p.a_rows, p.a_div, p.offsets);
   SNK_LAUNCH_CHECK();
