@@ -27,6 +27,8 @@
 #ifndef T2_STAGES
 #define T2_STAGES 6
 #endif
+#define T2_MAX_STAGES 10              // (grouped products with few rows a group)
+static_assert(T2_STAGES <= T2_MAX_STAGES, "barriers");
 #ifndef T2_BAND
 #define T2_BAND 8
 #endif
@@ -57,8 +59,8 @@ __device__ __forceinline__ void t2_wait(uint64_t* bar, uint32_t parity, volatile
 }
 
 struct __align__(16) T2Shared {
-  uint64_t full[T2_STAGES];         // (leader) both blocks' stages hold their operands
-  uint64_t empty[T2_STAGES];        // the MMAs that read the stage have completed (both blocks)
+  uint64_t full[T2_MAX_STAGES];     // (leader) both blocks' stages hold their operands
+  uint64_t empty[T2_MAX_STAGES];    // the MMAs that read the stage have completed (both blocks)
   uint64_t acc_full[2];             // the tile's products have completed (both blocks)
   uint64_t acc_empty[2];            // (leader) both epilogues have read the accumulator: 8 arrivals
   uint32_t tmem_base;
@@ -257,46 +259,104 @@ static int launch_tc2(const CUtensorMap& map_a, const CUtensorMap& map_w, void* 
 // neighbouring items of equal modelled cost per pair, 157 -> 180 us on the experts' gate|up product of 2,048
 // tokens, as pairs side by side then read far-apart memory; items drawn from a counter as pairs get free,
 // 159 us; L2 prefetch of an item's rows of W in one piece, 184 to 198 us.)
+//
+// Groups come in the order of their row tiles' length, longest first: a round of items then has one length, and the
+// shortest make the last, partly filled one.
+//
+// Groups of few rows are bound by the read of W, and that by the bytes an SM keeps on their way: a stage's part for A
+// is as large as the longest row tile of the launch needs, and the ring has as many stages as then fit (10 of 20 KB,
+// 8 of 24 KB, 6 of 32 KB; a plain TMA read loop: 5.3 TB/s with 64 KB of an SM in flight, 6.4 with 128 KB).
+// Measured, 32 groups, gate|up of 2,048 x 3,584 (before: six stages for all, groups in their own order): 8 rows each
+// 90.5 -> 86.9 us = 5.4 TB/s, 256 rows 133 -> 129 us, 2,048 tokens with the top 4 of 32 153 -> 149 us; down 48.8 -> 47.8,
+// 72, 83 us.  (Also tried: tiles of 224 or 240 columns where they fill the last round better, 89.5 us at 8 rows and
+// slower from 256 rows on, where an item costs its full M of 256 whatever it keeps.)
 #define T2G_MAX_GROUPS 256
-#define T2G_STAGE_BYTES ((T2_BM + T2_BM) * T2_BK * 2)  // 128 rows of W and up to 128 of the tile's rows of A
+#define T2G_W_BYTES (T2_BM * T2_BK * 2)               // of a stage: 128 rows of W, then 128, 64 or 32 of the tile's rows of A
+#define T2G_RING_BYTES (10 * (T2G_W_BYTES + 32 * T2_BK * 2))     // the largest of the three rings
 #define T2G_BOXES 5                  // tensor maps of A with boxes of 128, 64, 32, 16 and 8 rows
 
 struct T2GMaps {
   CUtensorMap a[T2G_BOXES];
 };
+// What every block works out of the offsets: the groups by row-tile length, and the items before each.
+struct T2GPlan {
+  int first[T2G_MAX_GROUPS + 1];
+  int order[T2G_MAX_GROUPS];
+  int rows[T2G_MAX_GROUPS];          // rows of a full row tile of each group
+  int longest;                       // rows of the longest row tile
+};
+
+// A group's rows are dealt evenly to its row tiles (in steps of 16): every tile streams the same rows of W,
+// so a group of 270 rows as 144 + 128 costs two half-length products, where 256 + 16 costs a full one and
+// a second pass over W for 16 rows (with 2,048 tokens, top 4 of 32 experts, half the groups are just
+// above 256 rows).
+__device__ __forceinline__ int t2g_row_tiles(int cnt) { return (cnt + 2 * T2_BM - 1) / (2 * T2_BM); }
+__device__ __forceinline__ int t2g_tile_rows(int cnt) {
+  const int row_tiles = t2g_row_tiles(cnt);
+  return row_tiles ? ((cnt + row_tiles - 1) / row_tiles + 15) & ~15 : 0;
+}
+
+// By all threads of the block; ends with a barrier.
+__device__ __forceinline__ void t2g_plan(T2GPlan* plan, const int* __restrict__ offsets, int groups, int n_tiles) {
+  for (int e = threadIdx.x; e < groups; e += blockDim.x) {
+    const int cnt = offsets[e + 1] - offsets[e];
+    plan->rows[e] = t2g_tile_rows(cnt);
+    plan->first[e + 1] = t2g_row_tiles(cnt) * n_tiles;   // the group's items, in group order for now
+  }
+  __syncthreads();
+  constexpr int EACH = (T2G_MAX_GROUPS + T2_THREADS - 1) / T2_THREADS;
+  int place[EACH], before[EACH], all = 0;
+#pragma unroll
+  for (int i = 0; i < EACH; ++i) {
+    const int e = threadIdx.x + i * blockDim.x;
+    if (e >= groups) break;
+    const int mine = plan->rows[e];
+    place[i] = before[i] = all = 0;
+    for (int o = 0; o < groups; ++o) {
+      const int r = plan->rows[o], items = plan->first[o + 1];
+      if (r > mine || (r == mine && o < e)) {
+        ++place[i];
+        before[i] += items;
+      }
+      all += items;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < EACH; ++i) {
+    const int e = threadIdx.x + i * blockDim.x;
+    if (e >= groups) break;
+    plan->order[place[i]] = e;
+    plan->first[place[i]] = before[i];
+    if (place[i] == 0) plan->longest = plan->rows[e];
+    if (e == 0) plan->first[groups] = all;
+  }
+  __syncthreads();
+}
 
 struct T2GItem {
   int row0, row_end, nt, w_row0, f0;  // rows row0 .. of A (nt of them in the MMA, a multiple of 16), W rows w_row0 + f0 ..
-  bool valid;
 };
 
-// first[e]: the number of items before group e (shared memory, groups + 1 entries)
-__device__ __forceinline__ T2GItem t2g_item(int item, const int* first, const int* __restrict__ offsets, int groups,
+__device__ __forceinline__ T2GItem t2g_item(int item, const T2GPlan* plan, const int* __restrict__ offsets, int groups,
                                             int N) {
   T2GItem t;
-  t.valid = false;
-  int lo = 0, hi = groups;                               // the group e with first[e] <= item < first[e + 1]
+  int lo = 0, hi = groups;                               // the place lo with first[lo] <= item < first[lo + 1]
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (first[mid] <= item) lo = mid; else hi = mid;
+    if (plan->first[mid] <= item) lo = mid; else hi = mid;
   }
-  if (item >= first[groups]) return t;
-  const int begin = offsets[lo], cnt = offsets[lo + 1] - begin;
-  const int row_tiles = (cnt + 2 * T2_BM - 1) / (2 * T2_BM);
-  const int in_group = item - first[lo];
+  const int e = plan->order[lo];
+  const int begin = offsets[e], cnt = offsets[e + 1] - begin;
+  const int row_tiles = t2g_row_tiles(cnt), per = plan->rows[e];
+  const int in_group = item - plan->first[lo];
   const int ft = in_group / row_tiles, tt = in_group % row_tiles;
-  // A group's rows are dealt evenly to its row tiles (in steps of 16): every tile streams the same rows of W,
-  // so a group of 270 rows as 144 + 128 costs two half-length products, where 256 + 16 costs a full one and
-  // a second pass over W for 16 rows (with 2,048 tokens, top 4 of 32 experts, half the groups are just
-  // above 256 rows).
-  const int per = ((cnt + row_tiles - 1) / row_tiles + 15) & ~15;
   t.row0 = begin + tt * per;
   t.row_end = min(begin + cnt, t.row0 + per);
   const int left = t.row_end - t.row0;
   t.nt = left <= 0 ? 16 : (left + 15) & ~15;
-  t.w_row0 = lo * N;
+  t.w_row0 = e * N;
   t.f0 = ft * T2_BN;
-  t.valid = true;
   return t;
 }
 
@@ -313,17 +373,16 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
                         OutT* __restrict__ C, int N, int K, const int* __restrict__ offsets, int groups, int act) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  T2Shared* sh = reinterpret_cast<T2Shared*>(tiles + (size_t)T2_STAGES * T2G_STAGE_BYTES);
-  int* first = reinterpret_cast<int*>(sh + 1);           // groups + 1 entries
+  T2Shared* sh = reinterpret_cast<T2Shared*>(tiles + T2G_RING_BYTES);
+  T2GPlan* plan = reinterpret_cast<T2GPlan*>(sh + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int k_tiles = (K + T2_BK - 1) / T2_BK;
-  const int n_tiles = (N + T2_BN - 1) / T2_BN;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < T2_STAGES; ++s) {
+    for (int s = 0; s < T2_MAX_STAGES; ++s) {
       mbar_init(&sh->full[s], 1);
       mbar_init(&sh->empty[s], 1);
     }
@@ -346,32 +405,34 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
   const uint32_t tmem_acc = rank == 0 ? sh->tmem_base : ld_cluster_u32(&sh->tmem_base, 0);
   volatile int* aborted = &sh->aborted;
   pdl_begin();                                           // offsets are written by the kernel before this one
-  for (int e = threadIdx.x; e < groups; e += blockDim.x)  // the groups' item counts side by side, then their running sum
-    first[e + 1] = ((offsets[e + 1] - offsets[e] + 2 * T2_BM - 1) / (2 * T2_BM)) * n_tiles;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    first[0] = 0;
-    for (int e = 0; e < groups; ++e) first[e + 1] += first[e];
-  }
-  __syncthreads();
-  const int total = first[groups];
+  t2g_plan(plan, offsets, groups, (N + T2_BN - 1) / T2_BN);
+  const int total = plan->first[groups];
+  // the ring: both blocks of a pair, and every thread, come to the same one
+  const int stages = plan->longest <= 64 ? 10 : plan->longest <= 128 ? 8 : 6;
+  const int stage_bytes = T2G_W_BYTES + (plan->longest <= 64 ? 32 : plan->longest <= 128 ? 64 : 128) * T2_BK * 2;
 
-  int it = 0;                                            // k-blocks so far (producer and MMA thread)
+  int s = 0;                                             // the stage of the next k-block (producer and MMA thread)
+  uint32_t lap = 0;                                      // the parity of the ring's rounds so far
+  auto next_stage = [&]() {
+    if (++s == stages) {
+      s = 0;
+      lap ^= 1;
+    }
+  };
   const bool lose_loads = *const_cast<volatile int*>(&g_t2_lose_loads) != 0;
   auto issue_loads = [&](int item) {
-    const T2GItem t = t2g_item(item, first, offsets, groups, N);
+    const T2GItem t = t2g_item(item, plan, offsets, groups, N);
     const int half = t.nt >> 1, box = t2g_box(half);
-    const uint32_t bytes = (uint32_t)(T2_BM * T2_BK * 2 + (128 >> box) * T2_BK * 2);
-    for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-      const int s = it % T2_STAGES;
-      t2_wait(&sh->empty[s], ((it / T2_STAGES) & 1) ^ 1, aborted, T2_ERR_EMPTY);
+    const uint32_t bytes = (uint32_t)(T2G_W_BYTES + (128 >> box) * T2_BK * 2);
+    for (int kt = 0; kt < k_tiles; ++kt, next_stage()) {
+      t2_wait(&sh->empty[s], lap ^ 1, aborted, T2_ERR_EMPTY);
       if (*aborted) return;                              // a wait ran out: nothing more is issued
       if (lose_loads) continue;
       if (rank == 0) mbar_expect_tx(&sh->full[s], 2 * bytes);
       const uint32_t bar = cluster_addr(&sh->full[s], 0);
-      unsigned char* stage = tiles + (size_t)s * T2G_STAGE_BYTES;
+      unsigned char* stage = tiles + (size_t)s * stage_bytes;
       tma2_load_2d(stage, &map_w, bar, kt * T2_BK, t.w_row0 + t.f0 + (int)rank * T2_BM);
-      tma2_load_2d(stage + T2_BM * T2_BK * 2, &maps.a[box], bar, kt * T2_BK, t.row0 + (int)rank * half);
+      tma2_load_2d(stage + T2G_W_BYTES, &maps.a[box], bar, kt * T2_BK, t.row0 + (int)rank * half);
     }
   };
 
@@ -382,20 +443,19 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
     if (lane == 0 && rank == 0) {
       int local = 0;
       for (int item = pair; item < total && !*aborted; item += pairs, ++local) {
-        const T2GItem t = t2g_item(item, first, offsets, groups, N);
+        const T2GItem t = t2g_item(item, plan, offsets, groups, N);
         const uint32_t idesc = instr_desc_bf16(2 * T2_BM, t.nt);
         const int buf = local % T2_ACC_BUFFERS;
         const int use = local / T2_ACC_BUFFERS;
         t2_wait(&sh->acc_empty[buf], (use & 1) ^ 1, aborted, T2_ERR_ACC_FREE);
         tc_fence_after();
         const uint32_t d_tmem = tmem_acc + (uint32_t)(buf * T2_BN);
-        for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-          const int s = it % T2_STAGES;
-          t2_wait(&sh->full[s], (it / T2_STAGES) & 1, aborted, T2_ERR_FULL);
+        for (int kt = 0; kt < k_tiles; ++kt, next_stage()) {
+          t2_wait(&sh->full[s], lap, aborted, T2_ERR_FULL);
           if (*aborted) break;
           tc_fence_after();
-          const uint32_t w_addr = smem_u32(tiles + (size_t)s * T2G_STAGE_BYTES);
-          const uint32_t a_addr = w_addr + T2_BM * T2_BK * 2;
+          const uint32_t w_addr = smem_u32(tiles + (size_t)s * stage_bytes);
+          const uint32_t a_addr = w_addr + T2G_W_BYTES;
 #pragma unroll
           for (int k = 0; k < T2_BK / 16; ++k)
             umma2_bf16(d_tmem, smem_desc_sw128(w_addr + k * 32), smem_desc_sw128(a_addr + k * 32), idesc,
@@ -411,7 +471,7 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
     float* stage_out = sh->stage_out[warp - 2];
     int local = 0;
     for (int item = pair; item < total; item += pairs, ++local) {
-      const T2GItem t = t2g_item(item, first, offsets, groups, N);
+      const T2GItem t = t2g_item(item, plan, offsets, groups, N);
       const int buf = local % T2_ACC_BUFFERS;
       const int use = local / T2_ACC_BUFFERS;
       t2_wait(&sh->acc_full[buf], use & 1, aborted, T2_ERR_ACC);
@@ -474,7 +534,7 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
 template <typename OutT, bool SWIGLU>
 static int launch_tc2_grouped(const T2GMaps& maps, const CUtensorMap& map_w, void* C, int M, int N, int K,
                               const int* offsets, int groups, cudaStream_t stream, int act) {
-  const size_t smem = 1024 + (size_t)T2_STAGES * T2G_STAGE_BYTES + sizeof(T2Shared) + (T2G_MAX_GROUPS + 1) * sizeof(int);
+  const size_t smem = 1024 + T2G_RING_BYTES + sizeof(T2Shared) + sizeof(T2GPlan);
   static int sms = 0;
   if (sms == 0) {
     int dev = 0;
