@@ -21,7 +21,7 @@
 // A group with more than 64 rows is walked in passes of 64 (W is then re-read from L2).
 // (the role of snowllm/ops/gemm.py:33-41 and the expert products of snowllm/ops/inference.py:60-76
 // at decode shapes)
-#include "common.cuh"
+#include "tma.cuh"
 
 #ifndef SK_WARPS
 #define SK_WARPS 8
@@ -58,7 +58,7 @@ template <int MT, typename OutT, bool SWIGLU>
 __global__ void __launch_bounds__(SK_WARPS * 32)
 gemm_skinny_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, OutT* __restrict__ C, int M,
                    int N, int K, const int* __restrict__ a_rows, int a_div,
-                   const int* __restrict__ offsets, int act) {
+                   const int* __restrict__ offsets, int groups, int act) {
 #if SK_PREFETCH_LINES > 0
   if (offsets == nullptr) {
     // A plain product's W is a constant and this block's 16 rows of it are known from the block's number
@@ -84,9 +84,26 @@ gemm_skinny_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, OutT*
   int row_begin = 0, row_end = M;
   const bf16* Wg = W;
   if (offsets) {
-    row_begin = offsets[blockIdx.y];
-    row_end = offsets[blockIdx.y + 1];
-    Wg = W + (size_t)blockIdx.y * N * K;
+    // groups > gridDim.y: there are fewer rows than groups, and block y takes the y-th group that owns any (every warp
+    // looks it up for itself).  One token with the top 4 of 32 experts then starts 896 blocks and not 7,168 of which
+    // 6,272 end at once: 18.8 -> 16 us of the gate|up product in the decode step.
+    int e = blockIdx.y;
+    if (groups > (int)gridDim.y) {
+      int left = blockIdx.y;
+      e = -1;
+      for (int e0 = 0; e0 < groups; e0 += 32) {
+        const unsigned own = __ballot_sync(0xffffffffu, e0 + lane < groups && offsets[e0 + lane + 1] > offsets[e0 + lane]);
+        if (left < __popc(own)) {
+          e = e0 + __fns(own, 0, left + 1);
+          break;
+        }
+        left -= __popc(own);
+      }
+      if (e < 0) return;
+    }
+    row_begin = offsets[e];
+    row_end = offsets[e + 1];
+    Wg = W + (size_t)e * N * K;
   }
   if (row_begin >= row_end) return;
   // the two W rows of this lane (rows past N read row N-1 and are dropped at the store)
@@ -217,27 +234,6 @@ gemm_skinny_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, OutT*
   }
 }
 
-template <int MT>
-static int launch_skinny(const void* A, const void* W, void* C, int M, int N, int K, const int* a_rows,
-                         int a_div, const int* offsets, int groups, int out_f32, int swiglu, int split,
-                         cudaStream_t stream) {
-  dim3 grid((N + SK_ROWS - 1) / SK_ROWS, offsets ? groups : 1, split);
-  const dim3 block(SK_WARPS * 32);
-  const bf16 *a = static_cast<const bf16*>(A), *w = static_cast<const bf16*>(W);
-  const int unary = swiglu == SNK_ACT_RELU2 ? swiglu : 0;
-  if (swiglu && !unary)
-    snk_launch_cluster(gemm_skinny_kernel<MT, bf16, true>, grid, block, 0, stream, split, a, w,
-                       static_cast<bf16*>(C), M, N, K, a_rows, a_div, offsets, swiglu);
-  else if (out_f32)
-    snk_launch_cluster(gemm_skinny_kernel<MT, float, false>, grid, block, 0, stream, split, a, w,
-                       static_cast<float*>(C), M, N, K, a_rows, a_div, offsets, 0);
-  else
-    snk_launch_cluster(gemm_skinny_kernel<MT, bf16, false>, grid, block, 0, stream, split, a, w,
-                       static_cast<bf16*>(C), M, N, K, a_rows, a_div, offsets, unary);
-  SNK_LAUNCH_CHECK();
-  return 0;
-}
-
 // How many blocks share one strip of W (a cluster along z).  A plain product with fewer strips than
 // the GPU has SMs is split 4 ways, as long as every warp of the cluster keeps two k-blocks of its own.
 // Measured in a replayed chain of launches at 8 rows: 2048 x 2048 6.8 -> 5.1 us, 2048 x 7168 20.6 -> 9.2 us;
@@ -256,6 +252,264 @@ static int skinny_split(int N, int K, const int* offsets) {
   return (strips <= SK_SPLIT_MAX_STRIPS && kblocks >= 2 * SK_SPLIT * SK_WARPS) ? SK_SPLIT : 1;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Plain products of up to 16 rows: the same, with W streamed through shared memory.  What bounds them is the read of W,
+// and most of what a small one takes beside it is the way from the end of the kernel before to the first bytes of W.  W
+// is a constant, so here one block per SM keeps a ring of stages (16 rows x 512 columns each, one TMA box, filled by a
+// ninth warp) that starts to fill while the kernel before still runs, and goes on across the block's strips of 16 rows;
+// eight warps multiply out of it.  Ring and sums take less than half of an SM's shared memory, so that the next product
+// can start beside this one.
+//
+// The numbers are the same bits as above: warp w takes the 32-column runs w, w + 8, .. of a strip in order, the same MMAs,
+// the same order of the warps' sums (SPLIT 4: four sums a warp, as the cluster's blocks held them).  A box brings 64
+// columns of a row at a time (128 bytes, swizzled), so two warps share a block of 16 x 128 bytes.  Lane g of the MMA
+// holds row st_row(g), an order in which the eight lanes that read shared memory together find their 16 bytes in
+// different banks.
+//
+// Measured, 1 row, in a replayed chain (the kernel above): 2,048 x 2,048 5.3 -> 3.6 us, 6,144 x 2,048 8.5 -> 7.2, 16,384 x
+// 2,048 17.1 -> 14.5; in the decode steps, where the ring fills ahead, 4.1 -> 2.7 us from the end of the kernel before to
+// the end of 2,048 x 2,048 and 7.0 -> 5.6 of 6,144 x 2,048.
+// Grouped products stay above: a group's strips are few and each has other rows of A to fetch, so the eight warps of the
+// one block cannot hide that as eight blocks an SM do (20 of 32 experts with a row each: 72 us here, 54 above).
+#define ST_RUNS 16                              // runs of 32 columns of a stage (8 blocks of 64 columns)
+#define ST_BYTES (SK_ROWS * ST_RUNS * 64)
+#define ST_MAX_ROWS 16
+#define ST_WAIT_NS 1500000000ull
+
+__device__ int g_sk_status;
+static int sk_lose_loads = 0;        // test hook: producers issue no loads (the stages then never fill)
+
+__device__ __forceinline__ int st_row(int g) { return (g >> 1) | ((g & 1) << 2); }
+
+struct StShared {
+  uint64_t full[8], empty[8];
+  int aborted;
+};
+
+__device__ __forceinline__ void st_wait(uint64_t* bar, uint32_t parity, volatile int* aborted, int code) {
+  if (*aborted || mbar_try_wait(bar, parity)) return;
+  const uint64_t start = global_ns();
+  while (!mbar_try_wait(bar, parity)) {
+    if (*aborted) return;
+    if (global_ns() - start > ST_WAIT_NS) {
+      *aborted = 1;
+      atomicCAS(&g_sk_status, 0, code);
+      return;
+    }
+  }
+}
+
+template <int MT, typename OutT, bool SWIGLU, int SPLIT>
+__global__ void __launch_bounds__((SK_WARPS + 1) * 32)
+gemm_stream_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restrict__ A, OutT* __restrict__ C, int M, int N,
+                   int K, int stages, int act, int lose_loads) {
+  extern __shared__ unsigned char raw[];
+  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
+  // two sets of sums, so that one barrier a strip is enough (one where four sums a warp would take the ring's room)
+  constexpr int SETS = SPLIT == 1 ? 2 : 1;
+  float(*red)[SPLIT * SK_WARPS][MT * 8][SK_ROWS + 1] =
+      reinterpret_cast<float(*)[SPLIT * SK_WARPS][MT * 8][SK_ROWS + 1]>(ring + (size_t)stages * ST_BYTES);
+  StShared* sh = reinterpret_cast<StShared*>(red + SETS);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int strips = (N + SK_ROWS - 1) / SK_ROWS, runs = K / 32, boxes = (runs + ST_RUNS - 1) / ST_RUNS;
+  volatile int* aborted = &sh->aborted;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&sh->full[s], 1);
+      mbar_init(&sh->empty[s], SK_WARPS);
+    }
+    sh->aborted = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  int s = 0;
+  uint32_t lap = 0;
+  auto next_stage = [&]() {
+    if (++s == stages) {
+      s = 0;
+      lap ^= 1;
+    }
+  };
+
+  if (warp == SK_WARPS) {                                // the producer: reads W alone, so it waits for no kernel
+    if (lane == 0) {
+      for (int strip = blockIdx.x; strip < strips && !*aborted; strip += gridDim.x) {
+        for (int box = 0; box < boxes; ++box, next_stage()) {
+          st_wait(&sh->empty[s], lap ^ 1, aborted, 2);
+          if (*aborted) break;
+          if (lose_loads) continue;
+          mbar_expect_tx(&sh->full[s], ST_BYTES);        // a box that reaches past the last run is filled up with zeros
+          tma_load_3d(ring + (size_t)s * ST_BYTES, &map, &sh->full[s], 0, strip * SK_ROWS, box * (ST_RUNS / 2));
+        }
+      }
+    }
+    if (*aborted) drain_after_abort();
+    return;
+  }
+
+  pdl_begin();
+  const int g = lane >> 2, t = lane & 3, row_g = st_row(g);
+  // this lane's 16 bytes of row row_g in its warp's half of a block of 64 columns (rows 8..15 follow 1 KB further on)
+  const int place = (warp >> 1) * 2048 + row_g * 128 + ((((warp & 1) * 4 + t) ^ row_g) << 4);
+  const bf16* a_ptr[MT];
+#pragma unroll
+  for (int i = 0; i < MT; ++i) a_ptr[i] = A + (size_t)(i * 8 + g < M ? i * 8 + g : 0) * K + 8 * t;
+  int turn = 0;
+  for (int strip = blockIdx.x; strip < strips; strip += gridDim.x, turn ^= SETS - 1) {
+    uint4 x[2][MT];                                      // this lane's values of A for the two runs of the next box
+    auto load_x = [&](int box) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int run = box * ST_RUNS + h * SK_WARPS + warp;
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+          x[h][i] = i * 8 + g < M && run < runs ? *reinterpret_cast<const uint4*>(a_ptr[i] + (size_t)run * 32)
+                                                : make_uint4(0, 0, 0, 0);
+      }
+    };
+    float acc[SPLIT][MT][4];
+#pragma unroll
+    for (int q = 0; q < SPLIT; ++q)
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[q][i][j] = 0.f;
+    auto multiply = [&](int box, float (&lo)[MT][4], float (&hi)[MT][4]) {
+      uint4 now[2][MT];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < MT; ++i) now[h][i] = x[h][i];
+      load_x(box + 1);                                   // (past the last box: zeros)
+      st_wait(&sh->full[s], lap, aborted, 1);
+      const unsigned char* stage = ring + (size_t)s * ST_BYTES + place;
+      uint4 wl[2], wh[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        wl[h] = *reinterpret_cast<const uint4*>(stage + h * (ST_BYTES / 2));
+        wh[h] = *reinterpret_cast<const uint4*>(stage + h * (ST_BYTES / 2) + 1024);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh->empty[s]);
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        mma_bf16(lo[i], wl[0].x, wh[0].x, wl[0].y, wh[0].y, now[0][i].x, now[0][i].y);
+        mma_bf16(lo[i], wl[0].z, wh[0].z, wl[0].w, wh[0].w, now[0][i].z, now[0][i].w);
+      }
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        mma_bf16(hi[i], wl[1].x, wh[1].x, wl[1].y, wh[1].y, now[1][i].x, now[1][i].y);
+        mma_bf16(hi[i], wl[1].z, wh[1].z, wl[1].w, wh[1].w, now[1][i].z, now[1][i].w);
+      }
+      next_stage();
+    };
+    load_x(0);
+    if constexpr (SPLIT == 1) {
+      for (int box = 0; box < boxes; ++box) multiply(box, acc[0], acc[0]);
+    } else {
+      static_assert(SPLIT == 1 || SPLIT == 4, "runs 8 q .. 8 q + 7 of every 32 are sum q's");
+      for (int box = 0; box < boxes; box += 2) {
+        multiply(box, acc[0], acc[1]);
+        if (box + 1 < boxes) multiply(box + 1, acc[2], acc[3]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < SPLIT; ++q)
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        float(*mine)[SK_ROWS + 1] = red[turn][q * SK_WARPS + warp];
+        mine[i * 8 + 2 * t][row_g] = acc[q][i][0];
+        mine[i * 8 + 2 * t + 1][row_g] = acc[q][i][1];
+        mine[i * 8 + 2 * t][row_g + 8] = acc[q][i][2];
+        mine[i * 8 + 2 * t + 1][row_g + 8] = acc[q][i][3];
+      }
+    asm volatile("bar.sync 1, %0;" ::"n"(SK_WARPS * 32) : "memory");
+    auto sum_of = [&](int tok, int r) {
+      float total = 0.f;
+#pragma unroll
+      for (int q = 0; q < SPLIT; ++q) {
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < SK_WARPS; ++w) sum += red[turn][q * SK_WARPS + w][tok][r];
+        total = q == 0 ? sum : total + sum;
+      }
+      return total;
+    };
+    const int n0 = strip * SK_ROWS, toks = min(MT * 8, M);
+    if constexpr (SWIGLU) {
+      for (int idx = threadIdx.x; idx < toks * (SK_ROWS / 2); idx += SK_WARPS * 32) {
+        const int tok = idx / (SK_ROWS / 2), r = idx % (SK_ROWS / 2);
+        if (n0 + r + 8 < N)
+          C[(size_t)tok * (N / 2) + n0 / 2 + r] = from_f<OutT>(glu_out(sum_of(tok, r), sum_of(tok, r + 8), act));
+      }
+    } else {
+      for (int idx = threadIdx.x; idx < toks * SK_ROWS; idx += SK_WARPS * 32) {
+        const int tok = idx / SK_ROWS, r = idx % SK_ROWS;
+        if (n0 + r < N) C[(size_t)tok * N + n0 + r] = from_f<OutT>(unary_out(sum_of(tok, r), act));
+      }
+    }
+    if constexpr (SETS == 1) asm volatile("bar.sync 1, %0;" ::"n"(SK_WARPS * 32) : "memory");
+  }
+}
+
+template <int MT, typename OutT, bool SWIGLU, int SPLIT>
+static int launch_stream(const CUtensorMap& map, const bf16* A, void* C, int M, int N, int K, int act, cudaStream_t stream) {
+  constexpr int sums = (SPLIT == 1 ? 2 : 1) * SPLIT * SK_WARPS * MT * 8 * (SK_ROWS + 1) * (int)sizeof(float);
+  // two products' rings on one SM: 6 stages of 16 KB, fewer where the sums take the room
+  constexpr int room = (110 * 1024 - sums - (int)sizeof(StShared)) / ST_BYTES, stages = room < 6 ? room : 6;
+  constexpr int smem = 1024 + stages * ST_BYTES + sums + (int)sizeof(StShared);
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    cudaFuncSetAttribute(gemm_stream_kernel<MT, OutT, SWIGLU, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    sms = n;
+  }
+  const int strips = (N + SK_ROWS - 1) / SK_ROWS;
+  snk_launch(gemm_stream_kernel<MT, OutT, SWIGLU, SPLIT>, dim3(strips < sms ? strips : sms), dim3((SK_WARPS + 1) * 32), smem,
+             stream, map, A, static_cast<OutT*>(C), M, N, K, stages, act, sk_lose_loads);
+  SNK_LAUNCH_CHECK();
+  return 0;
+}
+
+template <int MT>
+static int stream_product(const CUtensorMap& map, const void* A, void* C, int M, int N, int K, int out_f32, int swiglu,
+                          int split, cudaStream_t stream) {
+  const bf16* a = static_cast<const bf16*>(A);
+  if (swiglu && swiglu != SNK_ACT_RELU2)
+    return split > 1 ? launch_stream<MT, bf16, true, SK_SPLIT>(map, a, C, M, N, K, swiglu, stream)
+                     : launch_stream<MT, bf16, true, 1>(map, a, C, M, N, K, swiglu, stream);
+  if (out_f32)
+    return split > 1 ? launch_stream<MT, float, false, SK_SPLIT>(map, a, C, M, N, K, 0, stream)
+                     : launch_stream<MT, float, false, 1>(map, a, C, M, N, K, 0, stream);
+  return split > 1 ? launch_stream<MT, bf16, false, SK_SPLIT>(map, a, C, M, N, K, swiglu, stream)
+                   : launch_stream<MT, bf16, false, 1>(map, a, C, M, N, K, swiglu, stream);
+}
+
+template <int MT>
+static int launch_skinny(const void* A, const void* W, void* C, int M, int N, int K, const int* a_rows,
+                         int a_div, const int* offsets, int groups, int out_f32, int swiglu, int split,
+                         cudaStream_t stream) {
+  dim3 grid((N + SK_ROWS - 1) / SK_ROWS, offsets ? (groups < M ? groups : M) : 1, split);
+  const dim3 block(SK_WARPS * 32);
+  const bf16 *a = static_cast<const bf16*>(A), *w = static_cast<const bf16*>(W);
+  const int unary = swiglu == SNK_ACT_RELU2 ? swiglu : 0;
+  if (swiglu && !unary)
+    snk_launch_cluster(gemm_skinny_kernel<MT, bf16, true>, grid, block, 0, stream, split, a, w,
+                       static_cast<bf16*>(C), M, N, K, a_rows, a_div, offsets, groups, swiglu);
+  else if (out_f32)
+    snk_launch_cluster(gemm_skinny_kernel<MT, float, false>, grid, block, 0, stream, split, a, w,
+                       static_cast<float*>(C), M, N, K, a_rows, a_div, offsets, groups, 0);
+  else
+    snk_launch_cluster(gemm_skinny_kernel<MT, bf16, false>, grid, block, 0, stream, split, a, w,
+                       static_cast<bf16*>(C), M, N, K, a_rows, a_div, offsets, groups, unary);
+  SNK_LAUNCH_CHECK();
+  return 0;
+}
+
 // rows_hint: the most rows one group (or the whole product) is expected to hold; picks how many
 // 8-token tiles a pass covers.  More rows than that still give the right result, in more passes.
 // swiglu: W is gate/up interleaved in blocks of 8 rows and C is [M, N/2] bfloat16 = silu(gate) * up (or, SNK_ACT_RELU2:
@@ -270,8 +524,38 @@ SNK_API int snk_gemm_skinny(const void* A, const void* W, void* C, int M, int N,
   if (groups > 65535) return SNK_ERR_SIZE;
   if (a_div <= 0) a_div = 1;
   const int split = skinny_split(N, K, offsets);
+  // K in whole blocks of 64 columns, one pass: W through shared memory
+  if (!offsets && !a_rows && M <= ST_MAX_ROWS && K % 64 == 0) {
+    CUtensorMap map;
+    const int rc = tensor_map(W, N, K, SK_ROWS, 0, &map, ST_RUNS / 2);
+    if (rc) return rc;
+    if (M <= 8) return stream_product<1>(map, A, C, M, N, K, out_f32, swiglu, split, stream);
+    return stream_product<2>(map, A, C, M, N, K, out_f32, swiglu, split, stream);
+  }
   if (rows_hint <= 8) return launch_skinny<1>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);
   if (rows_hint <= 16) return launch_skinny<2>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);
   if (rows_hint <= 32) return launch_skinny<4>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);
   return launch_skinny<8>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);
+}
+
+// Test hook: with on != 0 the producers of later launches issue no loads, so that the bounded waits run out
+// (about 1.5 s) and the launches return with an error status instead of a product.
+SNK_API int snk_gemm_skinny_test_lose_loads(int on) {
+  sk_lose_loads = on;
+  return 0;
+}
+
+// Queue a copy of the status word into ``host`` (pinned host memory, one int) on ``stream`` without waiting
+// for it and without clearing it.  Not for use inside a stream capture.
+SNK_API int snk_gemm_skinny_status_peek(int* host, void* stream) {
+  return (int)cudaMemcpyFromSymbolAsync(host, g_sk_status, sizeof(int), 0, cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+}
+
+// 0, or the code of a wait that ran out in any earlier launch (1: a stage never filled, 2: one never came back);
+// reading clears it.  Synchronises.
+SNK_API int snk_gemm_skinny_status() {
+  int v = 0, zero = 0;
+  if (cudaMemcpyFromSymbol(&v, g_sk_status, sizeof(int)) != cudaSuccess) return -1;
+  if (v) cudaMemcpyToSymbol(g_sk_status, &zero, sizeof(int));
+  return v;
 }

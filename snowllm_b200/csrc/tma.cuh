@@ -47,6 +47,14 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// The same of a three-dimensional map.
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+
 // After a wait has run out the block stops issuing work; before it returns it gives the copies it still has in
 // flight this long to land in its shared memory (they take microseconds when they land at all).
 #define SNK_DRAIN_NS 200000ull
@@ -93,23 +101,27 @@ struct MapKeyHash {
 #define SNK_ERR_NO_ENCODER (SNK_ERR_SIZE + 100)    // the driver gave no cuTensorMapEncodeTiled
 #define SNK_ERR_ENCODE 30000                       // + the CUresult of a refused encoding
 
-static int tensor_map(const void* ptr, long long rows, long long k, int box_rows, int box_cols, CUtensorMap* out) {
+// k_runs > 0: the matrix as runs of 64 columns, [k / 64][rows][64] (k a multiple of 64), a box being `box_rows` rows of
+// `k_runs` runs: in shared memory every run of a box is a block of box_rows x 128 bytes of its own (swizzled alike).
+static int tensor_map(const void* ptr, long long rows, long long k, int box_rows, int box_cols, CUtensorMap* out,
+                      int k_runs = 0) {
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   static std::mutex mu;
   std::lock_guard<std::mutex> lock(mu);
-  const MapKey key{ptr, rows, k, box_rows, box_cols};
+  const MapKey key{ptr, rows, k, box_rows, k_runs > 0 ? -k_runs : box_cols};
   auto it = cache.find(key);
   if (it != cache.end()) { *out = it->second; return 0; }
   EncodeTiledFn fn = encode_fn();
   if (!fn) return SNK_ERR_NO_ENCODER;
-  const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1, 1};
+  const bool runs = k_runs > 0;
+  const cuuint64_t dims[3] = {(cuuint64_t)(runs ? 64 : k), (cuuint64_t)rows, (cuuint64_t)(k / 64)};
+  const cuuint64_t strides[2] = {(cuuint64_t)k * 2, 128};
+  const cuuint32_t box[3] = {(cuuint32_t)(runs ? 64 : box_cols), (cuuint32_t)box_rows, (cuuint32_t)k_runs};
+  const cuuint32_t estr[3] = {1, 1, 1};
   CUtensorMap m;
-  const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, runs ? 3 : 2, const_cast<void*>(ptr), dims, strides, box,
+                        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return SNK_ERR_ENCODE + (int)r;
   if (cache.size() > 8192) cache.clear();
   cache.emplace(key, m);

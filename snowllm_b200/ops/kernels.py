@@ -63,6 +63,9 @@ _SIGNATURES = {
     },
     "gemm_skinny": {
         "snk_gemm_skinny": [P, P, P, I, I, I, P, I, P, I, I, I, I, P],
+        "snk_gemm_skinny_status": [],
+        "snk_gemm_skinny_status_peek": [P, P],
+        "snk_gemm_skinny_test_lose_loads": [I],
     },
     "gemm_tc": {
         "snk_gemm_tc": [P, P, P, I, I, I, P, I, I, I, I, P, P],
@@ -856,7 +859,8 @@ class StatusWatch:
     WORDS = (("gemm_tc", "snk_gemm_tc_status_peek", 1, lambda: gemm_tc_status()),
              ("gemm_tc2", "snk_gemm_tc2_status_peek", 1, lambda: gemm_tc2_status()[0]),
              ("attention_tc", "snk_attention_tc_status_peek", 1, lambda: attention_tc_status()),
-             ("attention_mma", "snk_attention_decode_status_peek", 2, lambda: attention_decode_status()))
+             ("attention_mma", "snk_attention_decode_status_peek", 2, lambda: attention_decode_status()),
+             ("gemm_skinny", "snk_gemm_skinny_status_peek", 1, lambda: gemm_skinny_status()))
 
     def __init__(self):
         self.host = torch.zeros(sum(w[2] for w in self.WORDS), dtype=torch.int32).pin_memory()
@@ -1134,12 +1138,19 @@ def gemm_tc_status() -> int:
     return int(fn("snk_gemm_tc_status")())
 
 
+def gemm_skinny_status() -> int:
+    """0, or the code of a wait that ran out inside a streaming few-rows product since the last call
+    (synchronises the device; 1: a stage never filled, 2: one never came back)."""
+    return int(fn("snk_gemm_skinny_status")())
+
+
 def lose_loads(on: bool) -> None:
-    """Test hook of the two tcgen05 product libraries: while on, their producers issue no loads, so the
-    bounded waits inside the kernels run out and a launch returns with an error status (see
-    ``gemm_tc_status``, ``gemm_tc2_status``, ``StatusWatch``) instead of a product."""
+    """Test hook of the two tcgen05 product libraries and the streaming few-rows product: while on, their producers
+    issue no loads, so the bounded waits inside the kernels run out and a launch returns with an error status (see
+    ``gemm_tc_status``, ``gemm_tc2_status``, ``gemm_skinny_status``, ``StatusWatch``) instead of a product."""
     check(fn("snk_gemm_tc_test_lose_loads")(int(on)), "gemm_tc test hook", 0)
     check(fn("snk_gemm_tc2_test_lose_loads")(int(on)), "gemm_tc2 test hook", 0)
+    check(fn("snk_gemm_skinny_test_lose_loads")(int(on)), "gemm_skinny test hook", 0)
 
 
 def gather_rows(x, rows, div=1, out=None):

@@ -1,0 +1,86 @@
+"""The few-rows products: the one that streams W through shared memory, at the edges of its boxes (512 columns), strips (16
+rows of W) and passes (8 and 16 rows), against a double-precision product and the kernel without a ring; its bounded waits;
+and grouped products with fewer rows than groups, whose blocks look up the groups that own any."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def operands(*shape, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(*shape, device="cuda", generator=gen).to(torch.bfloat16)
+
+
+def slack_of(K):
+    """What a float sum of K products of N(0, 1) values may be off by: the sum takes a step per MMA of 16 columns and
+    then 16 more (warps, halves), each rounding (or cutting off) 2^-23 of a partial sum of at most about 2 sqrt(K)."""
+    return 2.0 ** -23 * (K / 16 + 16) * 2 * K ** 0.5
+
+
+def off(got, want, K):
+    """The largest error over that slack and, for bfloat16 outputs, one rounding of the result."""
+    slack = slack_of(K) + (2.0 ** -8 * want.abs() if got.dtype == torch.bfloat16 else 0)
+    return float(((got.double() - want).abs() / slack).max())
+
+
+# K: less than a block (the kernel without a ring), a block, a part of a box, a box, a box and a block, an odd number of
+# boxes of a split sum, a deep one
+@pytest.mark.parametrize("K", [32, 64, 448, 512, 576, 2048, 2624, 10752])
+@pytest.mark.parametrize("M,N", [(1, 16), (8, 17), (9, 200), (16, 2368), (3, 2384), (5, 40)])
+def test_plain(M, N, K):
+    from snowllm_b200.ops import kernels
+    a, w = operands(M, K, seed=1), operands(N, K, seed=2)
+    want = a.double() @ w.double().T
+    out = kernels.gemm_skinny(a, w, out_dtype=torch.float32)
+    assert off(out, want, K) <= 1
+    assert off(kernels.gemm_skinny(a, w), want, K) <= 1
+    # the kernel without a ring (which takes the rows by a list) comes to the same bits, in one pass and in several
+    rows = torch.arange(M, dtype=torch.int32, device="cuda")
+    for hint in (8, 64):
+        other = kernels.gemm_skinny(a, w, out_dtype=torch.float32, a_rows=rows, rows_hint=hint)
+        assert torch.equal(other, out)
+
+
+@pytest.mark.parametrize("counts", [[1] * 5, [0, 0, 3, 0], [17, 0, 8, 9, 1], [0] * 40 + [2] + [0] * 30 + [33], [16]])
+@pytest.mark.parametrize("N,K", [(48, 128), (256, 1792)])
+def test_grouped(counts, N, K):
+    from snowllm_b200.ops import kernels
+    G, M = len(counts), sum(counts)
+    x, w = operands(2 * M + 1, K, seed=3), operands(G, N, K, seed=4)
+    rows = torch.randperm(2 * M, generator=torch.Generator().manual_seed(5))[:M].to(torch.int32).cuda()
+    offsets = torch.tensor([0] + counts).cumsum(0).to(torch.int32).cuda()
+    for hint in (8, 16):
+        out = kernels.gemm_skinny(x, w, out_dtype=torch.float32, a_rows=rows, a_div=2, offsets=offsets, rows_out=M,
+                                  rows_hint=hint)
+        glu = kernels.gemm_skinny(x, w, a_rows=rows, a_div=2, offsets=offsets, rows_out=M, rows_hint=hint, swiglu=1)
+        lo = 0
+        for e, n in enumerate(counts):
+            if n:
+                want = x[(rows[lo:lo + n] // 2).long()].double() @ w[e].double().T
+                assert off(out[lo:lo + n], want, K) <= 1
+                gate, up = want.view(n, N // 16, 2, 8).unbind(2)
+                ref = (gate * torch.sigmoid(gate) * up).reshape(n, N // 2)
+                # one rounding, and the float sums' error through the gate (its slope is at most 1.1) and the product
+                slack = 2.0 ** -8 * ref.abs() + slack_of(K) * (1.1 * up.abs() + gate.abs() + 1).reshape(n, N // 2)
+                assert ((glu[lo:lo + n].double() - ref).abs() <= slack).all()
+            lo += n
+
+
+def test_wait_that_runs_out():
+    from snowllm_b200.errors import KernelError
+    from snowllm_b200.ops import kernels
+    a, w = operands(4, 1024, seed=6), operands(4096, 1024, seed=7)
+    good = kernels.gemm_skinny(a, w)
+    watch = kernels.StatusWatch()
+    kernels.lose_loads(True)
+    try:
+        kernels.gemm_skinny(a, w)
+        watch.peek()
+        torch.cuda.synchronize()
+    finally:
+        kernels.lose_loads(False)
+    with pytest.raises(KernelError, match="bounded wait ran out.*gemm_skinny"):
+        watch.check()
+    assert kernels.gemm_skinny_status() == 0
+    assert torch.equal(kernels.gemm_skinny(a, w), good)
