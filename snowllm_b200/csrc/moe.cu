@@ -379,10 +379,20 @@ __device__ __forceinline__ void sort_pairs(const int* __restrict__ topk_ids, int
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {                                // the running sum of the counts, 32 experts at a time
     int run = 0;
-    for (int e = 0; e < E; ++e) { off[e] = run; run += cnt[e]; }
-    off[E] = run;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + threadIdx.x, mine = e < E ? cnt[e] : 0;
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int before = __shfl_up_sync(0xffffffffu, upto, o);
+        if ((int)threadIdx.x >= o) upto += before;
+      }
+      if (e < E) off[e] = run + upto - mine;
+      run += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (threadIdx.x == 0) off[E] = run;
   }
   __syncthreads();
   for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = off[e];
