@@ -64,7 +64,9 @@ gemm_skinny_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, OutT*
     // A plain product's W is a constant and this block's 16 rows of it are known from the block's number
     // alone: while the kernel before this one ends, ask L2 for the first lines of each row (128 bytes a
     // thread and round; no register is held, nothing is read into the SM).  A grouped product does not
-    // know before the wait which groups own rows.
+    // know before the wait which groups own rows.  (Told by the caller that the offsets are older than the kernel in
+    // front, the experts' second product of one token asked for its rows while the first one ran: it took as long as
+    // without, 9 us, and the first one 25 us instead of 16.)
     const int row = min((int)(blockIdx.x * SK_ROWS + (threadIdx.x >> 4)), N - 1);
     const char* base = reinterpret_cast<const char*>(W + (size_t)row * K);
     const int row_bytes = K * 2;
@@ -255,7 +257,7 @@ static int skinny_split(int N, int K, const int* offsets) {
 // ---------------------------------------------------------------------------------------------
 // Plain products of up to 16 rows: the same, with W streamed through shared memory.  What bounds them is the read of W,
 // and most of what a small one takes beside it is the way from the end of the kernel before to the first bytes of W.  W
-// is a constant, so here one block per SM keeps a ring of stages (16 rows x 512 columns each, one TMA box, filled by a
+// is a constant (the caller says so: w_ahead), so here one block per SM keeps a ring of stages (16 rows x 512 columns each, one TMA box, filled by a
 // ninth warp) that starts to fill while the kernel before still runs, and goes on across the block's strips of 16 rows;
 // eight warps multiply out of it.  Ring and sums take less than half of an SM's shared memory, so that the next product
 // can start beside this one.
@@ -302,7 +304,7 @@ __device__ __forceinline__ void st_wait(uint64_t* bar, uint32_t parity, volatile
 template <int MT, typename OutT, bool SWIGLU, int SPLIT>
 __global__ void __launch_bounds__((SK_WARPS + 1) * 32)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restrict__ A, OutT* __restrict__ C, int M, int N,
-                   int K, int stages, int act, int lose_loads) {
+                   int K, int stages, int act, int w_ahead, int lose_loads) {
   extern __shared__ unsigned char raw[];
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
   // two sets of sums, so that one barrier a strip is enough (one where four sums a warp would take the ring's room)
@@ -333,8 +335,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     }
   };
 
-  if (warp == SK_WARPS) {                                // the producer: reads W alone, so it waits for no kernel
+  if (warp == SK_WARPS) {                                // the producer: reads W alone
     if (lane == 0) {
+      if (!w_ahead) pdl_wait();
       for (int strip = blockIdx.x; strip < strips && !*aborted; strip += gridDim.x) {
         for (int box = 0; box < boxes; ++box, next_stage()) {
           st_wait(&sh->empty[s], lap ^ 1, aborted, 2);
@@ -455,7 +458,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
 }
 
 template <int MT, typename OutT, bool SWIGLU, int SPLIT>
-static int launch_stream(const CUtensorMap& map, const bf16* A, void* C, int M, int N, int K, int act, cudaStream_t stream) {
+static int launch_stream(const CUtensorMap& map, const bf16* A, void* C, int M, int N, int K, int act, int w_ahead,
+                         cudaStream_t stream) {
   constexpr int sums = (SPLIT == 1 ? 2 : 1) * SPLIT * SK_WARPS * MT * 8 * (SK_ROWS + 1) * (int)sizeof(float);
   // two products' rings on one SM: 6 stages of 16 KB, fewer where the sums take the room
   constexpr int room = (110 * 1024 - sums - (int)sizeof(StShared)) / ST_BYTES, stages = room < 6 ? room : 6;
@@ -470,23 +474,23 @@ static int launch_stream(const CUtensorMap& map, const bf16* A, void* C, int M, 
   }
   const int strips = (N + SK_ROWS - 1) / SK_ROWS;
   snk_launch(gemm_stream_kernel<MT, OutT, SWIGLU, SPLIT>, dim3(strips < sms ? strips : sms), dim3((SK_WARPS + 1) * 32), smem,
-             stream, map, A, static_cast<OutT*>(C), M, N, K, stages, act, sk_lose_loads);
+             stream, map, A, static_cast<OutT*>(C), M, N, K, stages, act, w_ahead, sk_lose_loads);
   SNK_LAUNCH_CHECK();
   return 0;
 }
 
 template <int MT>
 static int stream_product(const CUtensorMap& map, const void* A, void* C, int M, int N, int K, int out_f32, int swiglu,
-                          int split, cudaStream_t stream) {
+                          int split, int w_ahead, cudaStream_t stream) {
   const bf16* a = static_cast<const bf16*>(A);
   if (swiglu && swiglu != SNK_ACT_RELU2)
-    return split > 1 ? launch_stream<MT, bf16, true, SK_SPLIT>(map, a, C, M, N, K, swiglu, stream)
-                     : launch_stream<MT, bf16, true, 1>(map, a, C, M, N, K, swiglu, stream);
+    return split > 1 ? launch_stream<MT, bf16, true, SK_SPLIT>(map, a, C, M, N, K, swiglu, w_ahead, stream)
+                     : launch_stream<MT, bf16, true, 1>(map, a, C, M, N, K, swiglu, w_ahead, stream);
   if (out_f32)
-    return split > 1 ? launch_stream<MT, float, false, SK_SPLIT>(map, a, C, M, N, K, 0, stream)
-                     : launch_stream<MT, float, false, 1>(map, a, C, M, N, K, 0, stream);
-  return split > 1 ? launch_stream<MT, bf16, false, SK_SPLIT>(map, a, C, M, N, K, swiglu, stream)
-                   : launch_stream<MT, bf16, false, 1>(map, a, C, M, N, K, swiglu, stream);
+    return split > 1 ? launch_stream<MT, float, false, SK_SPLIT>(map, a, C, M, N, K, 0, w_ahead, stream)
+                     : launch_stream<MT, float, false, 1>(map, a, C, M, N, K, 0, w_ahead, stream);
+  return split > 1 ? launch_stream<MT, bf16, false, SK_SPLIT>(map, a, C, M, N, K, swiglu, w_ahead, stream)
+                   : launch_stream<MT, bf16, false, 1>(map, a, C, M, N, K, swiglu, w_ahead, stream);
 }
 
 template <int MT>
@@ -514,9 +518,10 @@ static int launch_skinny(const void* A, const void* W, void* C, int M, int N, in
 // 8-token tiles a pass covers.  More rows than that still give the right result, in more passes.
 // swiglu: W is gate/up interleaved in blocks of 8 rows and C is [M, N/2] bfloat16 = silu(gate) * up (or, SNK_ACT_RELU2:
 // C is [M, N] bfloat16, the square of relu of the product).
+// w_ahead: W was there before the kernel in front of this launch began, and may be read ahead of the wait for it.
 SNK_API int snk_gemm_skinny(const void* A, const void* W, void* C, int M, int N, int K, const int* a_rows,
                             int a_div, const int* offsets, int groups, int rows_hint, int out_f32, int swiglu,
-                            cudaStream_t stream) {
+                            int w_ahead, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || K % 8) return SNK_ERR_SIZE;
   if (swiglu && ((swiglu != SNK_ACT_RELU2 && N % 16) || out_f32)) return SNK_ERR_SIZE;
@@ -529,8 +534,8 @@ SNK_API int snk_gemm_skinny(const void* A, const void* W, void* C, int M, int N,
     CUtensorMap map;
     const int rc = tensor_map(W, N, K, SK_ROWS, 0, &map, ST_RUNS / 2);
     if (rc) return rc;
-    if (M <= 8) return stream_product<1>(map, A, C, M, N, K, out_f32, swiglu, split, stream);
-    return stream_product<2>(map, A, C, M, N, K, out_f32, swiglu, split, stream);
+    if (M <= 8) return stream_product<1>(map, A, C, M, N, K, out_f32, swiglu, split, w_ahead, stream);
+    return stream_product<2>(map, A, C, M, N, K, out_f32, swiglu, split, w_ahead, stream);
   }
   if (rows_hint <= 8) return launch_skinny<1>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);
   if (rows_hint <= 16) return launch_skinny<2>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);

@@ -62,18 +62,18 @@ _SIGNATURES = {
         "snk_gemm_simt": [P, P, P, I, I, I, P, I, P, I, I, I, I, P],
     },
     "gemm_skinny": {
-        "snk_gemm_skinny": [P, P, P, I, I, I, P, I, P, I, I, I, I, P],
+        "snk_gemm_skinny": [P, P, P, I, I, I, P, I, P, I, I, I, I, I, P],
         "snk_gemm_skinny_status": [],
         "snk_gemm_skinny_status_peek": [P, P],
         "snk_gemm_skinny_test_lose_loads": [I],
     },
     "gemm_tc": {
-        "snk_gemm_tc": [P, P, P, I, I, I, P, I, I, I, I, P, P],
+        "snk_gemm_tc": [P, P, P, I, I, I, P, I, I, I, I, P, I, P],
         "snk_gemm_tc_scratch_bytes": [I, I, I, I],
         "snk_gemm_tc_status": [],
         "snk_gemm_tc_status_peek": [P, P],
         "snk_gemm_tc_test_lose_loads": [I],
-        "snk_gemm_tc_parts": [P, P, P, I, I, I, P, P],
+        "snk_gemm_tc_parts": [P, P, P, I, I, I, P, I, P],
         "snk_gather_rows_bf16": [P, P, P, I, I, I, P],
     },
     "gemm_tc2": {
@@ -1006,10 +1006,11 @@ def gemm_skinny_ok(a, w) -> bool:
 
 
 def gemm_skinny(a, w, out_dtype=None, out=None, a_rows=None, a_div=1, offsets=None, rows_out=None,
-                rows_hint=None, swiglu=False, act: int = 0):
+                rows_hint=None, swiglu=False, act: int = 0, w_ahead: bool = False):
     """bfloat16 a [M, K] times w [N, K]^T (or grouped w [G, N, K]) for few rows: W streams from memory
     once into tensor-core fragments.  ``rows_hint``: rows expected per group (sets the pass size).  ``act``: the code of
-    an activation applied at the store (``UNARY_CODES``; bfloat16 output)."""
+    an activation applied at the store (``UNARY_CODES``; bfloat16 output).  ``w_ahead``: w is a weight, complete
+    before the kernel launched in front of this one began: it may be read while that one still runs."""
     _chk(a, "gemm a", torch.bfloat16)
     _chk(w, "gemm w", torch.bfloat16)
     K = a.shape[1]
@@ -1034,7 +1035,7 @@ def gemm_skinny(a, w, out_dtype=None, out=None, a_rows=None, a_div=1, offsets=No
         raise KernelError("gemm output is bfloat16 or float32 (bfloat16 with swiglu)")
     check(fn("snk_gemm_skinny")(_ptr(a), _ptr(w), _ptr(out), M, N, K, _ptr(a_rows), int(a_div), _ptr(offsets),
                                 G, int(rows_hint if rows_hint is not None else M),
-                                int(out_dtype == torch.float32), int(swiglu or act), _stream()), "gemm_skinny",
+                                int(out_dtype == torch.float32), int(swiglu or act), int(w_ahead), _stream()), "gemm_skinny",
           work=lambda: _gemm_work(M, a, w, out, offsets))
     return out
 
@@ -1055,9 +1056,10 @@ def _tc_scratch_bytes(M: int, N: int, K: int, grouped: bool) -> int:
     return int(fn("snk_gemm_tc_scratch_bytes")(M, N, K, int(grouped)))
 
 
-def gemm_tc(a, w, out_dtype=None, out=None, offsets=None, swiglu=False):
+def gemm_tc(a, w, out_dtype=None, out=None, offsets=None, swiglu=False, w_ahead: bool = False):
     """bfloat16 a [M, K] times w [N, K]^T on the tcgen05 tensor cores, float accumulation in tensor
-    memory.  Grouped: w [G, N, K], rows of ``a`` sorted by group, ``offsets`` int32 [G+1]."""
+    memory.  Grouped: w [G, N, K], rows of ``a`` sorted by group, ``offsets`` int32 [G+1].  ``w_ahead``
+    (plain products): as in ``gemm_skinny``."""
     _chk(a, "gemm a", torch.bfloat16)
     _chk(w, "gemm w", torch.bfloat16)
     M, K = a.shape
@@ -1082,7 +1084,7 @@ def gemm_tc(a, w, out_dtype=None, out=None, offsets=None, swiglu=False):
     need = _tc_scratch_bytes(M, N, K, grouped)
     scratch = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
     check(fn("snk_gemm_tc")(_ptr(a), _ptr(w), _ptr(out), M, N, K, _ptr(offsets), G, row_tiles,
-                            int(out_dtype == torch.float32), int(swiglu), _ptr(scratch), _stream()), "gemm_tc",
+                            int(out_dtype == torch.float32), int(swiglu), _ptr(scratch), int(w_ahead), _stream()), "gemm_tc",
           launches=2 if need else 1, work=lambda: _gemm_work(M, a, w, out, offsets))
     return out
 
@@ -1221,7 +1223,7 @@ def moe_route(x, router_w, bias, top_k, norm_topk_prob, scaling, scoring: str = 
         parts = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
         planes = ctypes.c_int(0)
         check(fn("snk_gemm_tc_parts")(_ptr(x), _ptr(router_w), _ptr(parts), M, E, H, ctypes.byref(planes),
-                                      _stream()), "gemm_tc_parts",
+                                      1, _stream()), "gemm_tc_parts",
               work=lambda: (_nbytes(x, router_w) + M * E * 4 * max(planes.value, 1), 2 * M * E * H))
         check(fn("snk_moe_topk")(_ptr(parts), _ptr(bias), _ptr(ids), _ptr(wts), M, E, top_k,
                                  flags, float(scaling), 0, planes.value, _stream()), "moe_topk")

@@ -34,7 +34,7 @@ def _tc(x, w, **kw):
     rows = x.shape[0]
     if TC_PAIRS and (rows >= PAIRS_MIN_ROWS if offsets is None else w.shape[0] <= PAIRS_MAX_GROUPS):
         return kernels.gemm_tc2(x, w, **kw)
-    return kernels.gemm_tc(x, w, **kw)
+    return kernels.gemm_tc(x, w, w_ahead=True, **kw)
 
 
 SKINNY_MAX_ROWS = 16       # measured crossover: up to here the few-rows kernel reads W faster than 128-row tiles
@@ -43,10 +43,11 @@ SKINNY_MAX_GROUP_ROWS = 4  # grouped: mean rows per group up to which the few-ro
 
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
            out: torch.Tensor | None = None) -> torch.Tensor:
-    """x [M, K] times w [N, K]^T -> [M, N] in ``out_dtype`` (the compute dtype or float32)."""
+    """x [M, K] times w [N, K]^T -> [M, N] in ``out_dtype`` (the compute dtype or float32).  ``w`` is a weight: the
+    products may read it while the kernel launched in front of them still runs (here and below)."""
     if kernels.gemm_skinny_ok(x, w):
         if x.shape[0] <= SKINNY_MAX_ROWS:
-            return kernels.gemm_skinny(x, w, out_dtype=out_dtype, out=out)
+            return kernels.gemm_skinny(x, w, out_dtype=out_dtype, out=out, w_ahead=True)
         return _tc(x, w, out_dtype=out_dtype, out=out)
     return kernels.gemm_simt(x, w, out_dtype=out_dtype, out=out)
 
@@ -127,7 +128,7 @@ def linear_glu(x: torch.Tensor, w13: torch.Tensor, interleaved: bool, activation
     if interleaved and kernels.gemm_skinny_ok(x, w13):
         code = glu_code(activation, limit)
         if x.shape[0] <= SKINNY_MAX_ROWS:
-            return kernels.gemm_skinny(x, w13, swiglu=code)
+            return kernels.gemm_skinny(x, w13, swiglu=code, w_ahead=True)
         return _tc(x, w13, swiglu=code)
     return _gated(linear(x, w13), interleaved, activation, limit)
 
