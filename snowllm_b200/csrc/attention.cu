@@ -215,20 +215,16 @@ __global__ void paged_attention_kernel(
 
 // Merge the chunks of one (row, head).  The first warp finds the running maximum and the normaliser
 // over the chunks (lanes take chunks in turns, then a butterfly) and leaves the chunks' factors in shared memory.  The
-// chunks are then cut into MERGE_ZG runs; a thread sums four neighbouring elements of the output over one run in chunk
-// order, and the runs' sums are added in run order: many short chains of loads instead of one long one.  Bound by
+// chunks are then cut into MERGE_ZG runs; a thread sums four neighbouring elements of the output (one, where hd is no
+// multiple of four) over one run in chunk order, and the runs' sums are added in run order: many short chains of loads instead of one long one.  Bound by
 // the latency of those loads, so the blocks are small and all of a step's are on the SMs at once: with a thread per
 // element and run, and the factors formed by each, 64 rows of
 // 32 heads and up to 33 chunks took 18.4 us from the end of the attention to the end of the merge, now 7.7.
 #define MERGE_ZG 4
-#define MERGE_MAX_FACTORS 8192      // chunks whose factors fit beside the sums; more are formed where they are used
+#define MERGE_MAX_FACTORS 4096      // chunks whose factors fit beside the sums; more are formed where they are used
 
-static int merge_threads(int hd) { return hd <= 32 ? 32 : (hd <= 512 ? (hd + 31) & ~31 : 512); }
-static size_t merge_smem(int hd, int num_chunks) {
-  return (size_t)(MERGE_ZG * hd + (num_chunks <= MERGE_MAX_FACTORS ? num_chunks : 0)) * sizeof(float);
-}
-
-template <typename T>
+// VEC 4: hd is a multiple of 4 and part_o lies on 16 bytes; otherwise VEC 1, an element at a time.
+template <typename T, int VEC>
 __global__ void attention_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                        const int* __restrict__ positions, T* __restrict__ out, int nh,
                                        int hd, int window, int chunk, int num_chunks,
@@ -260,19 +256,27 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
   __syncthreads();
   // `gate`: the head's output times sigmoid of its own logit, gate[m * gate_ld + head]
   const float mx = s_mx, inv = gate ? s_inv / (1.f + expf(-to_f<T>(gate[(size_t)m * gate_ld + head]))) : s_inv;
-  const int per = (n + MERGE_ZG - 1) / MERGE_ZG, quads = hd / 4;     // hd is a multiple of 4
-  for (int i = threadIdx.x; i < MERGE_ZG * quads; i += blockDim.x) {
-    const int zg = i / quads, d = (i % quads) * 4;
+  const int per = (n + MERGE_ZG - 1) / MERGE_ZG, units = hd / VEC;
+  for (int i = threadIdx.x; i < MERGE_ZG * units; i += blockDim.x) {
+    const int zg = i / units, d = (i % units) * VEC;
     const int z0 = min(n, zg * per), z1 = min(n, z0 + per);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float acc[VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) acc[v] = 0.f;
 #pragma unroll 8
     for (int z = z0; z < z1; ++z) {
-      const float4 o = *reinterpret_cast<const float4*>(part_o + (base + z) * hd + d);
+      const float* from = part_o + (base + z) * hd + d;
       const float f = kept ? factors[z] : expf(part_ml[(base + z) * 2] - mx);
-      acc.x = fmaf(o.x, f, acc.x); acc.y = fmaf(o.y, f, acc.y);
-      acc.z = fmaf(o.z, f, acc.z); acc.w = fmaf(o.w, f, acc.w);
+      if constexpr (VEC == 4) {
+        const float4 o = *reinterpret_cast<const float4*>(from);
+        acc[0] = fmaf(o.x, f, acc[0]); acc[1] = fmaf(o.y, f, acc[1]);
+        acc[2] = fmaf(o.z, f, acc[2]); acc[3] = fmaf(o.w, f, acc[3]);
+      } else {
+        acc[0] = fmaf(*from, f, acc[0]);
+      }
     }
-    *reinterpret_cast<float4*>(merge_sh + zg * hd + d) = acc;
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) merge_sh[zg * hd + d + v] = acc[v];
   }
   __syncthreads();
   for (int d = threadIdx.x; d < hd; d += blockDim.x) {
@@ -281,6 +285,20 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
     for (int r = 1; r < MERGE_ZG; ++r) acc += merge_sh[r * hd + d];
     out[((size_t)m * nh + head) * hd + d] = from_f<T>(acc * inv);
   }
+}
+
+template <typename T>
+static void launch_merge(const float* part_o, const float* part_ml, const int* positions, void* out, int M, int nh, int hd,
+                         int window, int chunk, int num_chunks, const int* row_list, int keep, const void* gate,
+                         long long gate_ld, cudaStream_t stream) {
+  const int threads = hd <= 32 ? 32 : (hd <= 512 ? (hd + 31) & ~31 : 512);
+  const size_t smem = (size_t)(MERGE_ZG * hd + (num_chunks <= MERGE_MAX_FACTORS ? num_chunks : 0)) * sizeof(float);
+  auto launch = [&](auto kernel) {
+    snk_launch(kernel, dim3(M, nh), dim3(threads), smem, stream, part_o, part_ml, positions, static_cast<T*>(out), nh, hd,
+               window, chunk, num_chunks, row_list, keep, static_cast<const T*>(gate), gate_ld);
+  };
+  if (hd % 4 == 0 && (uintptr_t)part_o % 16 == 0) launch(attention_merge_kernel<T, 4>);
+  else launch(attention_merge_kernel<T, 1>);
 }
 
 // Bytes of scratch the launch below needs for `num_chunks` > 1 (0 for one chunk).
@@ -330,12 +348,8 @@ SNK_API int snk_paged_attention_rows(const void* q, const void* pool, const int*
 #undef ATT_LAUNCH
   SNK_LAUNCH_CHECK();
   if (num_chunks > 1) {
-    dim3 mgrid(M, nh);
-    const int threads = merge_threads(hd);
-    SNK_DISPATCH(dtype, snk_launch(attention_merge_kernel<T>, dim3(mgrid), dim3(threads),
-                                   merge_smem(hd, num_chunks), stream, 
-                            part_o, part_ml, positions, static_cast<T*>(out), nh, hd, window,
-                            chunk, num_chunks, row_list, 0, static_cast<const T*>(nullptr), 0LL));
+    SNK_DISPATCH(dtype, launch_merge<T>(part_o, part_ml, positions, out, M, nh, hd, window, chunk, num_chunks,
+                                         row_list, 0, nullptr, 0LL, stream));
     SNK_LAUNCH_CHECK();
   }
   return 0;
@@ -349,12 +363,8 @@ SNK_API int snk_attention_merge(const void* scratch, const int* positions, void*
   if (M <= 0 || num_chunks <= 1) return 0;
   const float* part_o = static_cast<const float*>(scratch);
   const float* part_ml = part_o + (size_t)M * nh * num_chunks * hd;
-  dim3 mgrid(M, nh);
-  const int threads = merge_threads(hd);
-  SNK_DISPATCH(dtype, snk_launch(attention_merge_kernel<T>, dim3(mgrid), dim3(threads),
-                                 merge_smem(hd, num_chunks), stream, 
-                          part_o, part_ml, positions, static_cast<T*>(out), nh, hd, window, chunk, num_chunks,
-                          row_list, 0, static_cast<const T*>(nullptr), 0LL));
+  SNK_DISPATCH(dtype, launch_merge<T>(part_o, part_ml, positions, out, M, nh, hd, window, chunk, num_chunks,
+                                       row_list, 0, nullptr, 0LL, stream));
   SNK_LAUNCH_CHECK();
   return 0;
 }
@@ -368,12 +378,8 @@ SNK_API int snk_attention_merge_gated(const void* scratch, const int* positions,
   if (M <= 0 || num_chunks <= 1) return 0;
   const float* part_o = static_cast<const float*>(scratch);
   const float* part_ml = part_o + (size_t)M * nh * num_chunks * hd;
-  dim3 mgrid(M, nh);
-  const int threads = merge_threads(hd);
-  SNK_DISPATCH(dtype, snk_launch(attention_merge_kernel<T>, dim3(mgrid), dim3(threads),
-                                 merge_smem(hd, num_chunks), stream,
-                                 part_o, part_ml, positions, static_cast<T*>(out), nh, hd, window, chunk, num_chunks,
-                                 row_list, keep, static_cast<const T*>(gate), gate_ld));
+  SNK_DISPATCH(dtype, launch_merge<T>(part_o, part_ml, positions, out, M, nh, hd, window, chunk, num_chunks,
+                                       row_list, keep, gate, gate_ld, stream));
   SNK_LAUNCH_CHECK();
   return 0;
 }

@@ -88,15 +88,18 @@ gemm_skinny_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, OutT*
   if (offsets) {
     // groups > gridDim.y: there are fewer rows than groups, and block y takes the y-th group that owns any (every warp
     // looks it up for itself).  One token with the top 4 of 32 experts then starts 896 blocks and not 7,168 of which
-    // 6,272 end at once: 18.8 -> 16 us of the gate|up product in the decode step.
+    // 6,272 end at once: 18.8 -> 16 us of the gate|up product in the decode step.  (With as many rows as groups, 8 such
+    // tokens, the look-up cost as much as it saved.)
     int e = blockIdx.y;
     if (groups > (int)gridDim.y) {
       int left = blockIdx.y;
       e = -1;
       for (int e0 = 0; e0 < groups; e0 += 32) {
-        const unsigned own = __ballot_sync(0xffffffffu, e0 + lane < groups && offsets[e0 + lane + 1] > offsets[e0 + lane]);
-        if (left < __popc(own)) {
-          e = e0 + __fns(own, 0, left + 1);
+        const bool owns = e0 + lane < groups && offsets[e0 + lane + 1] > offsets[e0 + lane];
+        const unsigned own = __ballot_sync(0xffffffffu, owns);
+        const unsigned it = __ballot_sync(0xffffffffu, owns && __popc(own & ((1u << lane) - 1)) == left);
+        if (it) {
+          e = e0 + __ffs(it) - 1;
           break;
         }
         left -= __popc(own);
