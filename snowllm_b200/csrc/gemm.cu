@@ -164,7 +164,7 @@ gemm_tile_kernel(const T* __restrict__ A, const T* __restrict__ W, OutT* __restr
 // ---------------------------------------------------------------------------------------
 // Few rows (decode), float: bound by the read of W.  A block owns FR_COLS columns (rows of W) and FR_STAGES chunks of
 // FR_K of their values, which four warps of its own bring in by cp.async (a row of a chunk is one instruction of a warp),
-// W's first chunks from before the wait for the kernel before.  The other warps multiply: a lane owns one column and R
+// W's first chunks from before the wait for the kernel before where W is a weight (w_ahead).  The other warps multiply: a lane owns one column and R
 // rows, half-warps rows of their own.  The sum over k stays one thread's, in order: with K chained multiply-adds of four
 // cycles a block cannot end sooner than 4 K cycles (4.3 us at K = 2,048), so nothing but them and the reads of their
 // operands is left to those warps, and the narrow blocks of 16 columns share the columns out over as many SMs as N gives.
@@ -184,7 +184,7 @@ __device__ __forceinline__ void cp_async16(float* smem, const float* gmem, bool 
 template <int R, int WARPS>
 __global__ void __launch_bounds__((WARPS + FR_LOADERS) * 32)
 gemm_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
-                const int* __restrict__ a_rows, int a_div, const int* __restrict__ offsets) {
+                const int* __restrict__ a_rows, int a_div, const int* __restrict__ offsets, int w_ahead) {
   constexpr int ROWS = 2 * R * WARPS;
   constexpr int W_EACH = FR_COLS / FR_LOADERS, A_EACH = (ROWS + FR_LOADERS - 1) / FR_LOADERS;
   extern __shared__ __align__(16) float sm[];          // per stage: FR_COLS rows of W, then ROWS rows of A
@@ -207,7 +207,8 @@ gemm_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
       cp_async16(to + i * (FR_LOADERS * FR_PITCH), w_src[i] + (in ? c * FR_K : -lane * 4),
                  in && n0 + loader + i * FR_LOADERS < N);
   };
-  if (offsets == nullptr && loader >= 0) {             // W is a constant: its first chunks need not wait
+  bool w_there = offsets == nullptr && w_ahead;        // W is a weight: its first chunks need not wait
+  if (w_there && loader >= 0) {
     point_w(W);
 #pragma unroll
     for (int c = 0; c < FR_STAGES - 1; ++c)
@@ -219,10 +220,11 @@ gemm_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
     row_end = offsets[blockIdx.y + 1];
     if (row_begin >= row_end) return;
     point_w(W + (size_t)blockIdx.y * N * K);
+  } else if (!w_there) {
+    point_w(W);
   }
   const int col = lane & 15;
   const int first = (warp * 2 + (lane >> 4)) * R;      // a multiplying lane's rows of a pass
-  bool w_there = offsets == nullptr;
   for (int m0 = row_begin; m0 < row_end; m0 += ROWS) {
     const float* a_src[A_EACH];
     bool a_ok[A_EACH];
@@ -304,6 +306,7 @@ struct SimtArgs {
   int a_div;
   const int* offsets;
   int groups, rows, vec;           // rows: the most that one group (or the product) can own
+  int w_ahead;
   cudaStream_t stream;
 };
 
@@ -328,7 +331,7 @@ static int launch_few(const SimtArgs& p) {
   }
   snk_launch(gemm_few_kernel<R, WARPS>, dim3((p.N + FR_COLS - 1) / FR_COLS, p.offsets ? p.groups : 1), dim3((WARPS + FR_LOADERS) * 32), smem,
              p.stream, static_cast<const float*>(p.A), static_cast<const float*>(p.W), static_cast<float*>(p.C), p.M, p.N,
-             p.K, p.a_rows, p.a_div, p.offsets);
+             p.K, p.a_rows, p.a_div, p.offsets, p.w_ahead);
   SNK_LAUNCH_CHECK();
   return 0;
 }
@@ -353,10 +356,11 @@ static int launch_tiles(const SimtArgs& p) {
 }
 
 // out_f32: C is float whatever the compute dtype.  groups <= 1 and offsets == nullptr: plain
-// product.  max_rows_per_group bounds the rows any one group can own (for the grid).
+// product.  max_rows_per_group bounds the rows any one group can own (for the grid).  w_ahead (plain products): W was
+// there before the kernel in front of this launch began, and may be read ahead of the wait for it.
 SNK_API int snk_gemm_simt(const void* A, const void* W, void* C, int M, int N, int K,
                           const int* a_rows, int a_div, const int* offsets, int groups,
-                          int max_rows_per_group, int out_f32, int dtype, cudaStream_t stream) {
+                          int max_rows_per_group, int out_f32, int dtype, int w_ahead, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return SNK_ERR_SIZE;
   const int rows = offsets ? max_rows_per_group : M;
@@ -364,7 +368,7 @@ SNK_API int snk_gemm_simt(const void* A, const void* W, void* C, int M, int N, i
   const size_t esz = dtype == SNK_F32 ? 4 : 2;
   const int vec = (K % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0) &&
                   (((size_t)K * esz) % 8 == 0);
-  const SimtArgs p{A, W, C, M, N, K, a_rows, a_div <= 0 ? 1 : a_div, offsets, groups, rows, vec, stream};
+  const SimtArgs p{A, W, C, M, N, K, a_rows, a_div <= 0 ? 1 : a_div, offsets, groups, rows, vec, w_ahead, stream};
   if (dtype == SNK_F32 && vec && (offsets ? (long long)M <= 4ll * groups : M <= FR_MAX_ROWS) && (!offsets || groups <= 65535)) {
     // rows of a pass: those of the product, or about twice a group's mean (fuller groups take more passes)
     const int pass = offsets ? 2 * ((M + groups - 1) / groups) : M;

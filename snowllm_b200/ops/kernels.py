@@ -59,7 +59,7 @@ _SIGNATURES = {
         "snk_attention_tc_status_peek": [P, P],
     },
     "gemm": {
-        "snk_gemm_simt": [P, P, P, I, I, I, P, I, P, I, I, I, I, P],
+        "snk_gemm_simt": [P, P, P, I, I, I, P, I, P, I, I, I, I, I, P],
     },
     "gemm_skinny": {
         "snk_gemm_skinny": [P, P, P, I, I, I, P, I, P, I, I, I, I, I, P],
@@ -967,9 +967,9 @@ def _gemm_work(rows, a, w, out, offsets):
 
 
 def gemm_simt(a, w, out_dtype=None, out=None, a_rows=None, a_div=1, offsets=None, rows_out=None,
-              max_rows_per_group=None):
+              max_rows_per_group=None, w_ahead: bool = False):
     """a [M, K] times w [N, K]^T (or, grouped, w [G, N, K] over rows sorted by group) with float
-    accumulation in k order on the CUDA cores."""
+    accumulation in k order on the CUDA cores.  ``w_ahead`` (plain products): as in ``gemm_skinny``."""
     dtype = a.dtype
     _chk(a, "gemm a", (torch.float32, torch.bfloat16))
     _chk(w, "gemm w", dtype)
@@ -994,7 +994,7 @@ def gemm_simt(a, w, out_dtype=None, out=None, a_rows=None, a_div=1, offsets=None
         raise KernelError("gemm output is the compute dtype or float32")
     check(fn("snk_gemm_simt")(_ptr(a), _ptr(w), _ptr(out), M, N, K, _ptr(a_rows), int(a_div), _ptr(offsets),
                               G, int(max_rows_per_group if grouped else M),
-                              int(out_dtype == torch.float32), code_of(dtype), _stream()), "gemm_simt",
+                              int(out_dtype == torch.float32), code_of(dtype), int(w_ahead), _stream()), "gemm_simt",
           work=lambda: _gemm_work(M, a, w, out, offsets))
     return out
 

@@ -49,7 +49,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
         if x.shape[0] <= SKINNY_MAX_ROWS:
             return kernels.gemm_skinny(x, w, out_dtype=out_dtype, out=out, w_ahead=True)
         return _tc(x, w, out_dtype=out_dtype, out=out)
-    return kernels.gemm_simt(x, w, out_dtype=out_dtype, out=out)
+    return kernels.gemm_simt(x, w, out_dtype=out_dtype, out=out, w_ahead=True)
 
 
 def _few_rows_per_group(rows_out: int, groups: int) -> bool:
