@@ -458,6 +458,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     }
     if constexpr (SETS == 1) asm volatile("bar.sync 1, %0;" ::"n"(SK_WARPS * 32) : "memory");
   }
+  // the producer may have issued its last box and gone before a wait ran out here: the warp that gave up keeps the
+  // block's shared memory until the boxes on their way have landed
+  if (*aborted) drain_after_abort();
 }
 
 template <int MT, typename OutT, bool SWIGLU, int SPLIT>

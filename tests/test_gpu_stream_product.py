@@ -84,3 +84,22 @@ def test_wait_that_runs_out():
         watch.check()
     assert kernels.gemm_skinny_status() == 0
     assert torch.equal(kernels.gemm_skinny(a, w), good)
+
+
+def test_a_block_that_gave_up_stays_until_its_copies_have_landed():
+    """At most two boxes a block, fewer than stages: the producer is gone when the multiplying warps' wait runs out, and
+    they give the copies on their way their 200 us themselves.  The launch takes the wait and those."""
+    from snowllm_b200.ops import kernels
+    a, w = operands(4, 1024, seed=8), operands(16 * 100, 1024, seed=9)
+    kernels.gemm_skinny(a, w)
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    kernels.lose_loads(True)
+    try:
+        begin.record()
+        kernels.gemm_skinny(a, w)
+        end.record()
+        torch.cuda.synchronize()
+    finally:
+        kernels.lose_loads(False)
+    assert kernels.gemm_skinny_status() == 1
+    assert begin.elapsed_time(end) >= 1500 + 0.2
