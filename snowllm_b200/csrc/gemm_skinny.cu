@@ -340,9 +340,12 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
 
   if (warp == SK_WARPS) {                                // the producer: reads W alone
     if (lane == 0) {
-      if (!w_ahead) pdl_wait();
+      // Boxes that go out ahead of the wait for the kernel in front: one ring, whose stages are empty.  The next one waits
+      // for warps that wait for that kernel, and its time is not to run while they do.
+      int ahead = w_ahead ? stages : 0;
       for (int strip = blockIdx.x; strip < strips && !*aborted; strip += gridDim.x) {
         for (int box = 0; box < boxes; ++box, next_stage()) {
+          if (ahead-- == 0) pdl_wait();
           st_wait(&sh->empty[s], lap ^ 1, aborted, 2);
           if (*aborted) break;
           if (lose_loads) continue;

@@ -103,3 +103,25 @@ def test_a_block_that_gave_up_stays_until_its_copies_have_landed():
         kernels.lose_loads(False)
     assert kernels.gemm_skinny_status() == 1
     assert begin.elapsed_time(end) >= 1500 + 0.2
+
+
+def test_a_slow_kernel_in_front_is_not_a_wait_that_ran_out():
+    """The kernel in front takes longer than a wait may: 1.5 s and the time it gives its copies (a tcgen05 product whose
+    loads are lost).  The rings of the product behind it are full all the while, and its own waits begin after it."""
+    from snowllm_b200.ops import kernels
+    a, w = operands(4, 2048, seed=10), operands(16384, 2048, seed=11)      # 7 strips of 4 boxes a block
+    x, v = operands(128, 64, seed=12), operands(128, 64, seed=13)
+    good = kernels.gemm_skinny(a, w)
+    kernels.gemm_tc(x, v)
+    assert kernels.gemm_tc_status() == 0 and kernels.gemm_skinny_status() == 0
+    lose = kernels.fn("snk_gemm_tc_test_lose_loads")
+    lose(1)
+    try:
+        kernels.gemm_tc(x, v)
+        out = kernels.gemm_skinny(a, w, w_ahead=True)
+        torch.cuda.synchronize()
+    finally:
+        lose(0)
+    assert kernels.gemm_tc_status() != 0
+    assert kernels.gemm_skinny_status() == 0
+    assert torch.equal(out, good)
