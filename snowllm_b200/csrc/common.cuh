@@ -175,7 +175,8 @@ __device__ __forceinline__ float ld_cluster_f32(const float* local, uint32_t ran
 }
 
 // Programmatic dependent launch.  pdl_wait() holds a kernel until the kernels before it have completed
-// and their writes are visible; before it a kernel touches no memory.  pdl_trigger() lets the next
+// and their writes are visible; before it a kernel touches no memory but a weight that its caller has said (w_ahead)
+// was complete before the kernel in front began, which it may read.  pdl_trigger() lets the next
 // kernel of the stream be scheduled while this one still runs, so that its launch latency hides behind
 // this kernel's tail.  The trigger always comes after the wait: a kernel that triggered first would let
 // the one after it trigger too, and a whole chain of waiting kernels would take the SMs from the one

@@ -1199,11 +1199,13 @@ def _route_flags(norm_topk_prob, scoring: str, bias=None, groups=(1, 1), group_s
     return int(bool(norm_topk_prob)) | softmax | limits
 
 
-def moe_route(x, router_w, bias, top_k, norm_topk_prob, scaling, scoring: str = "sigmoid", groups=(1, 1), **choice):
+def moe_route(x, router_w, bias, top_k, norm_topk_prob, scaling, scoring: str = "sigmoid", groups=(1, 1),
+              w_ahead: bool = False, **choice):
     """(ids int32 [M, k], weights float [M, k]) of the router, computed in float: a sigmoid per expert, or
     (``scoring`` "softmax") a softmax over all experts' logits; the k largest of score + ``bias`` are picked, among
     the experts of the best ``groups[1]`` of ``groups[0]`` equal groups; the weights are the scores.
-    ``choice``: ``group_score`` and ``renorm_eps`` of ``_route_flags``."""
+    ``w_ahead``: as in ``gemm_skinny``, of ``router_w``.  ``choice``: ``group_score`` and ``renorm_eps`` of
+    ``_route_flags``."""
     M, H = x.shape
     dtype = x.dtype
     _chk(x, "router input", (torch.float32, torch.bfloat16))
@@ -1223,7 +1225,7 @@ def moe_route(x, router_w, bias, top_k, norm_topk_prob, scaling, scoring: str = 
         parts = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
         planes = ctypes.c_int(0)
         check(fn("snk_gemm_tc_parts")(_ptr(x), _ptr(router_w), _ptr(parts), M, E, H, ctypes.byref(planes),
-                                      1, _stream()), "gemm_tc_parts",
+                                      int(w_ahead), _stream()), "gemm_tc_parts",
               work=lambda: (_nbytes(x, router_w) + M * E * 4 * max(planes.value, 1), 2 * M * E * H))
         check(fn("snk_moe_topk")(_ptr(parts), _ptr(bias), _ptr(ids), _ptr(wts), M, E, top_k,
                                  flags, float(scaling), 0, planes.value, _stream()), "moe_topk")
@@ -1246,14 +1248,14 @@ ROUTE_FUSED_MAX_ROWS = 32      # up to here: logits spread over the GPU, selecti
 
 
 def moe_route_sort(x, router_w, bias, top_k, norm_topk_prob, scaling, scoring: str = "sigmoid", groups=(1, 1),
-                   identity: int = 0, **choice):
+                   identity: int = 0, w_ahead: bool = False, **choice):
     """Routing and the sort by expert together: (ids, weights, offsets, pair_pos, sorted_pair) as
     `moe_route` and `moe_sort` give them.  The few rows of a decode step take two launches made for
     them; a row's logits are the same numbers on every path but the tensor-core one."""
     M, H = x.shape
     E = router_w.shape[0]
     if M > ROUTE_FUSED_MAX_ROWS or 8 * E * min(M, 32) + 8 * M * top_k > 48 * 1024:
-        ids, wts = moe_route(x, router_w, bias, top_k, norm_topk_prob, scaling, scoring, groups, **choice)
+        ids, wts = moe_route(x, router_w, bias, top_k, norm_topk_prob, scaling, scoring, groups, w_ahead, **choice)
         return (ids, wts) + moe_sort(ids, E, identity)
     dtype = x.dtype
     _chk(x, "router input", (torch.float32, torch.bfloat16))

@@ -28,13 +28,13 @@ PAIRS_MIN_ROWS = 4096             # plain products
 PAIRS_MAX_GROUPS = 256            # grouped products always run on pairs (a group's rows are the N side of the MMA)
 
 
-def _tc(x, w, **kw):
+def _tc(x, w, w_ahead=False, **kw):
     """The tcgen05 product: on pairs of SMs where there are rows enough."""
     offsets = kw.get("offsets")
     rows = x.shape[0]
     if TC_PAIRS and (rows >= PAIRS_MIN_ROWS if offsets is None else w.shape[0] <= PAIRS_MAX_GROUPS):
         return kernels.gemm_tc2(x, w, **kw)
-    return kernels.gemm_tc(x, w, w_ahead=True, **kw)
+    return kernels.gemm_tc(x, w, w_ahead=w_ahead, **kw)
 
 
 SKINNY_MAX_ROWS = 16       # measured crossover: up to here the few-rows kernel reads W faster than 128-row tiles
@@ -42,14 +42,15 @@ SKINNY_MAX_GROUP_ROWS = 4  # grouped: mean rows per group up to which the few-ro
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
-           out: torch.Tensor | None = None) -> torch.Tensor:
-    """x [M, K] times w [N, K]^T -> [M, N] in ``out_dtype`` (the compute dtype or float32).  ``w`` is a weight: the
-    products may read it while the kernel launched in front of them still runs (here and below)."""
+           out: torch.Tensor | None = None, w_ahead: bool = False) -> torch.Tensor:
+    """x [M, K] times w [N, K]^T -> [M, N] in ``out_dtype`` (the compute dtype or float32).  ``w_ahead``: w is a weight,
+    complete before the kernel launched in front of this product began, and may be read while that one still runs; without it
+    w may come from that kernel, as x may."""
     if kernels.gemm_skinny_ok(x, w):
         if x.shape[0] <= SKINNY_MAX_ROWS:
-            return kernels.gemm_skinny(x, w, out_dtype=out_dtype, out=out, w_ahead=True)
-        return _tc(x, w, out_dtype=out_dtype, out=out)
-    return kernels.gemm_simt(x, w, out_dtype=out_dtype, out=out, w_ahead=True)
+            return kernels.gemm_skinny(x, w, out_dtype=out_dtype, out=out, w_ahead=w_ahead)
+        return _tc(x, w, w_ahead, out_dtype=out_dtype, out=out)
+    return kernels.gemm_simt(x, w, out_dtype=out_dtype, out=out, w_ahead=w_ahead)
 
 
 def _few_rows_per_group(rows_out: int, groups: int) -> bool:
@@ -119,23 +120,23 @@ def _gated(h: torch.Tensor, interleaved: bool, activation: str, limit: float) ->
 
 
 def linear_glu(x: torch.Tensor, w13: torch.Tensor, interleaved: bool, activation: str = "silu",
-               limit: float = 0.0) -> torch.Tensor:
+               limit: float = 0.0, w_ahead: bool = False) -> torch.Tensor:
     """act(x Wg^T) * (x Wu^T) -> [M, I] with Wg, Wu held in one matrix w13 [2I, K] (plain halves, or
     interleaved by 8) and ``activation`` one of silu, relu, gelu_tanh, or swish_clamp with its ``limit``
     (g = min(gate, limit), u = clamp(up, -limit, limit), g * sigmoid(1.702 g) * (u + 1)).  With the
     interleaved layout the bfloat16 products apply the gate at their store; otherwise one elementwise kernel
-    follows the product."""
+    follows the product.  ``w_ahead``: as in ``linear``."""
     if interleaved and kernels.gemm_skinny_ok(x, w13):
         code = glu_code(activation, limit)
         if x.shape[0] <= SKINNY_MAX_ROWS:
-            return kernels.gemm_skinny(x, w13, swiglu=code, w_ahead=True)
-        return _tc(x, w13, swiglu=code)
-    return _gated(linear(x, w13), interleaved, activation, limit)
+            return kernels.gemm_skinny(x, w13, swiglu=code, w_ahead=w_ahead)
+        return _tc(x, w13, w_ahead, swiglu=code)
+    return _gated(linear(x, w13, w_ahead=w_ahead), interleaved, activation, limit)
 
 
-def linear_swiglu(x: torch.Tensor, w13: torch.Tensor, interleaved: bool) -> torch.Tensor:
+def linear_swiglu(x: torch.Tensor, w13: torch.Tensor, interleaved: bool, w_ahead: bool = False) -> torch.Tensor:
     """``linear_glu`` with silu."""
-    return linear_glu(x, w13, interleaved, "silu")
+    return linear_glu(x, w13, interleaved, "silu", w_ahead=w_ahead)
 
 
 def grouped_linear_glu(x, w13, offsets, rows_out, max_rows_per_group, a_rows, a_div, interleaved: bool,

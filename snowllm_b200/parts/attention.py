@@ -62,7 +62,7 @@ class Attention(Part):
             self.q_norm, self.k_norm = self.q_norm.float(), self.k_norm.float()
 
     def forward(self, ctx, x, cache, owns_cache=True):
-        qkv = linear(x, self.wqkv if owns_cache else self.wq)
+        qkv = linear(x, self.wqkv if owns_cache else self.wq, w_ahead=True)
         inv_freq, rot_dim = self.position.rotary(x.device)
         q = kernels.qk_norm_rope_cache(
             qkv, self.q_norm, self.k_norm, self.qk_norm_eps or 0.0, inv_freq, rot_dim, ctx.positions,
@@ -83,7 +83,7 @@ class Attention(Part):
                 kernels.attention_prefill(q, cache.pool, cache.block_table, cache.page_size, tiles, self.scale, o,
                                           window=self.window)
             if not rows_host:
-                return linear(o, self.wo, out_dtype=torch.float32)
+                return linear(o, self.wo, out_dtype=torch.float32, w_ahead=True)
         served = ctx.M if rows_host is None else len(rows_host)
         if kernels.attention_decode_mma_ok(q, self.num_kv_heads):
             # rows of decoded tokens on the tensor cores: keys in chunks of 256, merged in order
@@ -93,14 +93,14 @@ class Attention(Part):
             kernels.attention_decode_mma(q, cache.pool, cache.block_table, cache.page_size, ctx.positions,
                                          ctx.row_seg, self.scale, num_chunks, o, window=self.window,
                                          scratch=scratch, rows=rows)
-            return linear(o, self.wo, out_dtype=torch.float32)
+            return linear(o, self.wo, out_dtype=torch.float32, w_ahead=True)
         chunk, num_chunks = plan.plan(ctx, self.window, rows_host)
         scratch = ctx.scratch(kernels.attention_scratch_bytes(
             served, self.num_heads, self.head_dim, num_chunks)) if num_chunks > 1 else None
         kernels.paged_attention(q, cache.pool, cache.block_table, cache.page_size, ctx.positions,
                                 ctx.row_seg, self.scale, window=self.window, chunk=chunk,
                                 num_chunks=num_chunks, scratch=scratch, out=o, rows=rows)
-        return linear(o, self.wo, out_dtype=torch.float32)
+        return linear(o, self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 register_mixer("attention", Attention)

@@ -127,10 +127,10 @@ class LatentAttention(Part):
             raise KernelError("a layer without a latent projection must read another layer's cache, "
                               "and one with it must own its cache")
         H, M, r, rd = self.num_heads, ctx.M, self.kv_rank, self.rot_dim
-        proj = linear(x, self.w_in)
+        proj = linear(x, self.w_in, w_ahead=True)
         q_col, kv_col = self._columns()
         if self.q_rank:
-            q = linear(kernels.rms_cols(proj, q_col, self.q_rank, self.q_norm, self.norm_eps), self.w_uq)
+            q = linear(kernels.rms_cols(proj, q_col, self.q_rank, self.q_norm, self.norm_eps), self.w_uq, w_ahead=True)
             q_off = 0
         else:
             q, q_off = proj, q_col
@@ -161,7 +161,7 @@ class LatentAttention(Part):
         v = grouped_linear(o_lat.view(M * H, r), self.w_uv, offsets, H * M, M, a_rows=head_major)
         heads = kernels.heads_to_rows(v.view(H, M, self.v_head_dim))
         ctx.tap("attention_heads", heads)
-        return linear(heads, self.wo, out_dtype=torch.float32)
+        return linear(heads, self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 register_mixer("latent_attention", LatentAttention)

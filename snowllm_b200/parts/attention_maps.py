@@ -231,7 +231,7 @@ class MapsAttention(Part):
         if owns_cache == self.reads_cache:
             raise KernelError("a layer without key and value tensors must read another layer's cache, "
                               "and one with them must own its cache")
-        proj = linear(x, self.w_in)
+        proj = linear(x, self.w_in, w_ahead=True)
         if self._lends_rows:
             ctx.memo[("input_rows", id(self))] = proj
         q_off, k_off, v_off, g_off, _ = self._columns()
@@ -379,7 +379,7 @@ class BiasAttention(MapsAttention):
 
     def forward(self, ctx, x, cache, owns_cache=True):
         _, out = self._attend(ctx, x, cache, owns_cache, self.dtype)
-        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32)
+        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 class DiffAttention(MapsAttention):
@@ -415,7 +415,7 @@ class DiffAttention(MapsAttention):
         heads = kernels.head_norm_gate(maps, self.num_heads, dv, self.head_norm_eps, self.dtype, second=dv,
                                        lam=self.lam, gate=proj, gate_col=gate_col, mult=1.0 - self.offset)
         ctx.tap("attention_heads", heads)
-        return linear(heads, self.wo, out_dtype=torch.float32)
+        return linear(heads, self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 class SinkAttention(MapsAttention):
@@ -447,7 +447,7 @@ class SinkAttention(MapsAttention):
 
     def forward(self, ctx, x, cache, owns_cache=True):
         _, out = self._attend(ctx, x, cache, owns_cache, self.dtype)
-        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32)
+        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 class SlopeAttention(MapsAttention):
@@ -468,7 +468,7 @@ class SlopeAttention(MapsAttention):
 
     def forward(self, ctx, x, cache, owns_cache=True):
         _, out = self._attend(ctx, x, cache, owns_cache, self.dtype)
-        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32)
+        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 class ConvGateAttention(MapsAttention):
@@ -535,7 +535,7 @@ class ConvGateAttention(MapsAttention):
 
     def forward(self, ctx, x, cache, owns_cache=True):
         _, out = self._attend(ctx, x, cache, owns_cache, self.dtype)
-        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32)
+        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 class RotaryAttention(MapsAttention):
@@ -618,7 +618,7 @@ class RotaryAttention(MapsAttention):
 
     def forward(self, ctx, x, cache, owns_cache=True):
         _, out = self._attend(ctx, x, cache, owns_cache, self.dtype)
-        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32)
+        return linear(out.view(ctx.M, -1), self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 register_mixer("rotary_attention", RotaryAttention)

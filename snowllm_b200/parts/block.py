@@ -314,7 +314,7 @@ class OutputGate(Part):
         if self._rides is not None:
             sublayer, col = self._rides
             return sublayer.input_rows(ctx), col, self.bias
-        return linear(h, self.weight), 0, self.bias
+        return linear(h, self.weight, w_ahead=True), 0, self.bias
 
 
 class DepthAverage(Part):

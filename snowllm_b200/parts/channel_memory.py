@@ -49,7 +49,7 @@ class LowRank:
 
     def __call__(self, x):
         """Float [M, out], the pairs' outputs side by side."""
-        return linear(linear(x, self.a), self.b, out_dtype=torch.float32)
+        return linear(linear(x, self.a, w_ahead=True), self.b, out_dtype=torch.float32, w_ahead=True)
 
 
 class _ChannelMemory(Part):
@@ -74,7 +74,7 @@ class _ChannelMemory(Part):
         if self._rides is not None:
             host, col = self._rides
             return host.input_rows(ctx), col
-        return linear(x, self.w_in), 0
+        return linear(x, self.w_in, w_ahead=True), 0
 
     def _low_rank(self, rank) -> tuple:
         """(rank as a tensor dimension, what a TensorSpec says about it): the checkpoint's to choose unless given."""
@@ -119,7 +119,7 @@ class GatedLinear(_ChannelMemory):
         ctx.tap("memory_raw", raw)
         heads = kernels.head_norm_gate(raw, H, dv, self.head_norm_eps, self.dtype, weight=self.norm, gate=proj,
                                        gate_col=col + 2 * H * dk + H * dv, gate_act="silu")
-        return linear(heads, self.wo, out_dtype=torch.float32)
+        return linear(heads, self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 class DeltaRule(_ChannelMemory):
@@ -183,7 +183,7 @@ class DeltaRule(_ChannelMemory):
         ctx.tap("memory_raw", raw)
         heads = kernels.head_norm_gate(raw, H, dv, self.head_norm_eps, self.dtype, weight=self.norm, gate=low,
                                        gate_col=H * dk)
-        return linear(heads, self.wo, out_dtype=torch.float32)
+        return linear(heads, self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 register_mixer("gated_linear", GatedLinear)

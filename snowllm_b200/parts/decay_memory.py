@@ -122,13 +122,13 @@ class Hgrn2(_DecayMemory):
 
     def forward(self, ctx, x, cache, owns_cache=True):
         H, dk, dv = self.num_heads, self.head_dim, self.v_head_dim
-        proj = linear(x, self.w_in, out_dtype=torch.float32)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, w_ahead=True)
         raw = kernels.decay_memory(proj, 0, H * dk, 2 * H * dk, ctx.cu_seqlens, ctx.seg_start, ctx.seg_slot,
                                    cache.tensors[0], H, dk, dv, gate_bias=self.f_bias, gate_low=self.lower,
                                    pieces=self._pieces(ctx))
         ctx.tap("memory_raw", raw)
         heads = kernels.head_norm_gate(raw, H, dv, self.head_norm_eps, self.dtype, weight=self.norm)
-        return linear(heads, self.wo, out_dtype=torch.float32)
+        return linear(heads, self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 class Retention(_DecayMemory):
@@ -157,7 +157,7 @@ class Retention(_DecayMemory):
 
     def forward(self, ctx, x, cache, owns_cache=True):
         H, dk, dv = self.num_heads, self.head_dim, self.v_head_dim
-        proj = linear(x, self.w_in, out_dtype=torch.float32)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, w_ahead=True)
         inv_freq, rot_dim = self.position.rotary(x.device)
         raw = kernels.decay_memory(proj, 0, H * dk, 2 * H * dk, ctx.cu_seqlens, ctx.seg_start, ctx.seg_slot,
                                    cache.tensors[0], H, dk, dv, decay=self.decay, inv_freq=inv_freq, rot_dim=rot_dim,
@@ -165,7 +165,7 @@ class Retention(_DecayMemory):
         ctx.tap("memory_raw", raw)
         heads = kernels.head_norm_gate(raw, H, dv, self.head_norm_eps, self.dtype, gate=proj,
                                        gate_col=2 * H * dk + H * dv, gate_act="silu")
-        return linear(heads, self.wo, out_dtype=torch.float32)
+        return linear(heads, self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 register_mixer("hgrn2", Hgrn2)

@@ -105,7 +105,7 @@ class LinearHead(Part):
         return self.weight.numel() * self.weight.element_size() if self.weight is not None else 0
 
     def forward(self, ctx, x):
-        logits = linear(x, self.weight, out_dtype=torch.float32)
+        logits = linear(x, self.weight, out_dtype=torch.float32, w_ahead=True)
         return kernels.softcap(logits, self.softcap) if self.softcap else logits
 
 

@@ -34,8 +34,8 @@ class SwiGLU(Part):
         self.w2 = tensors["down"]
 
     def forward(self, ctx, x):
-        act = linear_swiglu(x, self.w13, self.interleaved)
-        return linear(act, self.w2, out_dtype=torch.float32)
+        act = linear_swiglu(x, self.w13, self.interleaved, w_ahead=True)
+        return linear(act, self.w2, out_dtype=torch.float32, w_ahead=True)
 
 
 class GatedFFN(SwiGLU):
@@ -55,8 +55,8 @@ class GatedFFN(SwiGLU):
         self.activation, self.limit = activation, float(limit or 0.0)
 
     def forward(self, ctx, x):
-        act = linear_glu(x, self.w13, self.interleaved, self.activation, self.limit)
-        return linear(act, self.w2, out_dtype=torch.float32)
+        act = linear_glu(x, self.w13, self.interleaved, self.activation, self.limit, w_ahead=True)
+        return linear(act, self.w2, out_dtype=torch.float32, w_ahead=True)
 
 
 class MLP(Part):
@@ -79,8 +79,8 @@ class MLP(Part):
         self.w1, self.w2 = tensors["up"], tensors["down"]
 
     def forward(self, ctx, x):
-        u = linear(x, self.w1)
-        return linear(kernels.act_rows(u, self.activation), self.w2, out_dtype=torch.float32)
+        u = linear(x, self.w1, w_ahead=True)
+        return linear(kernels.act_rows(u, self.activation), self.w2, out_dtype=torch.float32, w_ahead=True)
 
 
 register_ffn("swiglu", SwiGLU)

@@ -143,7 +143,7 @@ class SigmoidMoE(Part):
 
     def route(self, x):
         return kernels.moe_route(x, self.router, self.bias, self.top_k, self.norm_topk_prob,
-                                 self.routed_scaling_factor, self.scoring, self.groups, **self.choice)
+                                 self.routed_scaling_factor, self.scoring, self.groups, w_ahead=True, **self.choice)
 
     def forward_from_residual(self, ctx, residual, delta, norm):
         """The norm that precedes this feed-forward, the router and the sort in one launch, for the few rows
@@ -169,16 +169,16 @@ class SigmoidMoE(Part):
     def forward(self, ctx, x):
         routed = self._experts(ctx, x, *kernels.moe_route_sort(
             x, self.router, self.bias, self.top_k, self.norm_topk_prob, self.routed_scaling_factor, self.scoring,
-            self.groups, self.identity, **self.choice))
+            self.groups, self.identity, w_ahead=True, **self.choice))
         if self.shared is None:
             return routed
-        act = linear_glu(x, self.shared_w13, self.shared_interleaved, self.activation, self.shared["limit"])
+        act = linear_glu(x, self.shared_w13, self.shared_interleaved, self.activation, self.shared["limit"], w_ahead=True)
         gate = None
         if self.shared_row_gate is not None:
             gate = kernels.row_dot(x, self.shared_row_gate)        # float [M, 1]: one logit per token
             if ctx is not None:
                 ctx.tap("shared_row_gate", gate)
-        return kernels.DeltaSum(linear(act, self.shared_w2, out_dtype=torch.float32), routed, a_gate=gate)
+        return kernels.DeltaSum(linear(act, self.shared_w2, out_dtype=torch.float32, w_ahead=True), routed, a_gate=gate)
 
     def _gate_up(self, x, offsets, rows_out, cap, a_rows, a_div):
         """The experts' activated gate|up product over the rows in expert order."""

@@ -68,7 +68,7 @@ class MLstm(Part):
 
     def forward(self, ctx, x, cache, owns_cache=True):
         H, dk, dv = self.num_heads, self.head_dim, self.v_head_dim
-        proj = linear(x, self.w_in, out_dtype=torch.float32)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, w_ahead=True)
         q, k, v, g, i, f = self._columns()
         s_mat, s_vec, s_max = cache.tensors
         raw = kernels.mlstm(proj, q, k, v, i, f, self.bias_i, self.bias_f, self.gate_cap, ctx.cu_seqlens,
@@ -76,7 +76,7 @@ class MLstm(Part):
         ctx.tap("mlstm_raw", raw)
         heads = kernels.head_norm_gate(raw, H, dv, self.head_norm_eps, self.dtype, weight=self.norm, gate=proj,
                                        gate_col=g)
-        return linear(heads, self.wo, out_dtype=torch.float32)
+        return linear(heads, self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 register_mixer("mlstm", MLstm)

@@ -34,10 +34,10 @@ class ShortConv(Part):
         self.conv = tensors["conv"].reshape(self.hidden_size, self.kernel_size).contiguous()
 
     def forward(self, ctx, x, cache, owns_cache=True):
-        bcx = linear(x, self.in_proj)
+        bcx = linear(x, self.in_proj, w_ahead=True)
         y = kernels.short_conv(bcx, self.conv, cache.tensors[0], ctx.cu_seqlens, ctx.seg_start,
                                ctx.seg_slot, ctx.row_seg)
-        return linear(y, self.out_proj, out_dtype=torch.float32)
+        return linear(y, self.out_proj, out_dtype=torch.float32, w_ahead=True)
 
 
 register_mixer("short_conv", ShortConv)

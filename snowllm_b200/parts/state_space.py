@@ -96,7 +96,7 @@ class Mamba2(Part):
         return ctx.memo.pop(("input_rows", id(self)))
 
     def forward(self, ctx, x, cache, owns_cache=True):
-        proj = linear(x, self.w_in)
+        proj = linear(x, self.w_in, w_ahead=True)
         if self._lends_rows:
             ctx.memo[("input_rows", id(self))] = proj
         z_col, dt_col = self._columns()
@@ -111,7 +111,7 @@ class Mamba2(Part):
                                 self.num_groups, max(ctx.host_seg_len))
         ctx.tap("state_space_out", y)
         heads = kernels.gate_group_norm(y, proj, z_col, self.norm, self.norm_groups, self.norm_eps)
-        return linear(heads, self.wo, out_dtype=torch.float32)
+        return linear(heads, self.wo, out_dtype=torch.float32, w_ahead=True)
 
 
 register_mixer("mamba2", Mamba2)

@@ -40,8 +40,8 @@ class TokenSide(Part):
         if TABLE not in ctx.memo:
             raise KernelError("a layer with an input from the token ids needs an embedding with side rows")
         x = kernels.layer_norm(residual, delta, None, 0.0, self.dtype)
-        g = linear(x, self.gate, out_dtype=torch.float32)
+        g = linear(x, self.gate, out_dtype=torch.float32, w_ahead=True)
         act = kernels.side_gate(g, ctx.memo[TABLE], ctx.token_ids, self.index * self.dim, self.dtype,
                                 pending=ctx.pending_tokens)
         ctx.tap("token_side_gate", act)
-        return kernels.NormedDelta(linear(act, self.proj, out_dtype=torch.float32), weight=self.norm, eps=self.eps)
+        return kernels.NormedDelta(linear(act, self.proj, out_dtype=torch.float32, w_ahead=True), weight=self.norm, eps=self.eps)

@@ -125,3 +125,29 @@ def test_a_slow_kernel_in_front_is_not_a_wait_that_ran_out():
     assert kernels.gemm_tc_status() != 0
     assert kernels.gemm_skinny_status() == 0
     assert torch.equal(out, good)
+
+
+@pytest.mark.parametrize("M,dtype", [(4, torch.bfloat16), (64, torch.bfloat16), (4, torch.float32)])
+def test_w_may_come_from_the_kernel_in_front(M, dtype):
+    """Without ``w_ahead``, products whose w the launch in front of them writes, replayed without a gap; the numbers of
+    the same products launched one by one."""
+    from snowllm_b200.ops import linear
+    x, v = operands(M, 2048, seed=14).to(dtype), operands(2048, 64, seed=15).to(dtype)
+    us = [operands(2048, 64, seed=16 + i).to(dtype) for i in range(4)]
+    w = torch.zeros(2048, 2048, dtype=dtype, device="cuda")
+    want = []
+    for u in us:
+        linear(u, v, out=w)
+        torch.cuda.synchronize()
+        want.append(linear(x, w))
+        torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = []
+        for u in us:
+            linear(u, v, out=w)
+            got.append(linear(x, w))
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))

@@ -1,0 +1,51 @@
+"""Which products may read w while the kernel in front still runs: those whose caller says that w is a weight, no others.
+The kernels' wrappers are replaced by ones that write down what they are told."""
+import pytest
+import torch
+
+from snowllm_b200.ops import kernels, linear, linear_glu, linear_swiglu
+
+
+@pytest.fixture
+def told(monkeypatch):
+    calls = []
+    for name in ("gemm_skinny", "gemm_simt", "gemm_tc"):
+        monkeypatch.setattr(kernels, name, lambda x, w, name=name, **kw: calls.append((name, kw["w_ahead"])) or x)
+    monkeypatch.setattr(kernels, "gemm_skinny_ok", lambda x, w: x.dtype == torch.bfloat16)
+    for name in ("swiglu", "gated_act"):
+        monkeypatch.setattr(kernels, name, lambda h, *a, **kw: h)
+    return calls
+
+
+@pytest.mark.parametrize("rows,dtype,kernel", [(3, torch.bfloat16, "gemm_skinny"), (40, torch.bfloat16, "gemm_tc"),
+                                               (3, torch.float32, "gemm_simt"), (40, torch.float32, "gemm_simt")])
+def test_w_is_read_ahead_only_where_the_caller_says_it_is_a_weight(told, rows, dtype, kernel):
+    x, w = torch.zeros(rows, 64, dtype=dtype), torch.zeros(32, 64, dtype=dtype)
+    for said in (False, True):
+        kw = {"w_ahead": True} if said else {}
+        linear(x, w, **kw)
+        linear_glu(x, w, True, **kw)
+        linear_glu(x, w, False, "relu", **kw)
+        linear_swiglu(x, w, True, **kw)
+        assert told == [(kernel, said)] * 4
+        told.clear()
+
+
+@pytest.mark.parametrize("entry", ["moe_route", "moe_route_sort"])
+def test_a_router_is_read_ahead_only_where_the_caller_says_so(monkeypatch, entry):
+    parts = []
+
+    def fn(name):
+        return lambda *args: parts.append(args[7]) or 0 if name == "snk_gemm_tc_parts" else 0
+
+    monkeypatch.setattr(kernels, "fn", fn)
+    for name in ("_chk", "check"):
+        monkeypatch.setattr(kernels, name, lambda *a, **kw: None)
+    monkeypatch.setattr(kernels, "_stream", lambda: 0)
+    monkeypatch.setattr(kernels, "gemm_tc_ok", lambda x, w: True)
+    monkeypatch.setattr(kernels, "gemm_tc_is_split", lambda M, N, K: True)
+    monkeypatch.setattr(kernels, "_tc_scratch_bytes", lambda *a: 64)
+    x, w = torch.zeros(65, 64, dtype=torch.bfloat16), torch.zeros(32, 64, dtype=torch.bfloat16)
+    getattr(kernels, entry)(x, w, None, 2, True, 1.0)
+    getattr(kernels, entry)(x, w, None, 2, True, 1.0, w_ahead=True)
+    assert parts == [0, 1]
