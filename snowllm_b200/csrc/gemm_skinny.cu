@@ -21,6 +21,7 @@
 // A group with more than 64 rows is walked in passes of 64 (W is then re-read from L2).
 // (the role of snowllm/ops/gemm.py:33-41 and the expert products of snowllm/ops/inference.py:60-76
 // at decode shapes)
+#include "per_device.h"
 #include "tma.cuh"
 
 #ifndef SK_WARPS
@@ -473,14 +474,15 @@ static int launch_stream(const CUtensorMap& map, const bf16* A, void* C, int M, 
   // two products' rings on one SM: 6 stages of 16 KB, fewer where the sums take the room
   constexpr int room = (110 * 1024 - sums - (int)sizeof(StShared)) / ST_BYTES, stages = room < 6 ? room : 6;
   constexpr int smem = 1024 + stages * ST_BYTES + sums + (int)sizeof(StShared);
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(gemm_stream_kernel<MT, OutT, SWIGLU, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    sms = n;
-  }
+  static std::atomic<int> sms_of[SNK_MAX_DEVICES];
+  int device = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  const int rc = snk_per_device(sms_of, device, &sms, [&](int* n) {
+    e = cudaFuncSetAttribute(gemm_stream_kernel<MT, OutT, SWIGLU, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return (int)(e != cudaSuccess ? e : cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, device));
+  });
+  if (rc) return rc;
   const int strips = (N + SK_ROWS - 1) / SK_ROWS;
   snk_launch(gemm_stream_kernel<MT, OutT, SWIGLU, SPLIT>, dim3(strips < sms ? strips : sms), dim3((SK_WARPS + 1) * 32), smem,
              stream, map, A, static_cast<OutT*>(C), M, N, K, stages, act, w_ahead, sk_lose_loads);
