@@ -12,6 +12,7 @@
 // (the role of snowllm/ops/gemm.py:33-41 and of the expert products in
 // snowllm/ops/inference.py:60-76)
 #include "common.cuh"
+#include "per_device.h"
 
 template <typename T> struct Vec4;
 template <> struct Vec4<float> {
@@ -338,21 +339,49 @@ static int launch_few(const SimtArgs& p) {
 
 #define FR_MAX_ROWS 16             // up to here (grouped: up to 4 rows a group on average) W's read is the bound
 
-// The tile with the least work on the busiest SM: rounds of tiles over 148 SMs times the tile's area, over the share of
-// the FMA rate that its shared-memory reads leave.
+// The tile with the least work on the busiest SM: rounds of tiles over the SMs times the tile's area, over the share of
+// the FMA rate that its shared-memory reads leave.  The shares are those at 4,096 x 16,384 x 2,048 (128 x 128 5.16 ms, 64 x 128 5.28,
+// 64 x 64 6.64, 32 x 64 8.56).  Against all four tiles at 135 sizes (17 to 8,192 rows; N 64 to 16,384; K 640 to 8,192) the
+// choice was within 2 % of the fastest at 127, 3 to 6 % off at six, 9 and 12 % off at one each.
+// mean: rows of a group (of the product); sms: the device's.  0 to 3: 128 x 128, 64 x 128, 64 x 64, 32 x 64.
+static int pick_tile(int groups, long long mean, int N, int sms) {
+  static const int bm[4] = {128, 64, 64, 32}, bn[4] = {128, 128, 64, 64};
+  static const double rate[4] = {1.0, 0.95, 0.8, 0.6};
+  int best = 0;
+  double least = 0.0;
+  for (int t = 0; t < 4; ++t) {
+    const long long tiles = (long long)groups * ((mean + bm[t] - 1) / bm[t]) * ((N + bn[t] - 1) / bn[t]);
+    const double cost = (double)((tiles + sms - 1) / sms) * bm[t] * bn[t] / rate[t];
+    if (t == 0 || cost < least) {
+      best = t;
+      least = cost;
+    }
+  }
+  return best;
+}
+
+// For tests: the tile that a product of M rows (of `groups` groups, 0: plain) takes on a device of that many SMs.
+SNK_API int snk_gemm_simt_tile(int M, int N, int groups, int sms) {
+  return pick_tile(groups ? groups : 1, groups ? (M + groups - 1) / groups : M, N, sms);
+}
+
 template <typename T, typename OutT>
 static int launch_tiles(const SimtArgs& p) {
+  static std::atomic<int> sms_of[SNK_MAX_DEVICES];
+  int device = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  const int rc = snk_per_device(sms_of, device, &sms, [&](int* n) {
+    return (int)cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, device);
+  });
+  if (rc) return rc;
   const int G = p.offsets ? p.groups : 1;
-  const long long mean = p.offsets ? (p.M + G - 1) / G : p.M;      // rows of a group
-  auto cost = [&](int bm, int bn, double rate) {
-    const long long tiles = (long long)G * ((mean + bm - 1) / bm) * ((p.N + bn - 1) / bn);
-    return (double)((tiles + 147) / 148) * bm * bn / rate;
-  };
-  const double c128 = cost(128, 128, 1.0), c64w = cost(64, 128, 0.95), c64 = cost(64, 64, 0.8), c32 = cost(32, 64, 0.6);
-  if (c128 <= c64w && c128 <= c64 && c128 <= c32) return launch_tile<T, OutT, 128, 128, 8, 8>(p);
-  if (c64w <= c64 && c64w <= c32) return launch_tile<T, OutT, 64, 128, 8, 8>(p);
-  if (c64 <= c32) return launch_tile<T, OutT, 64, 64, 4, 8>(p);
-  return launch_tile<T, OutT, 32, 64, 4, 4>(p);
+  switch (pick_tile(G, p.offsets ? (p.M + G - 1) / G : p.M, p.N, sms)) {
+    case 0: return launch_tile<T, OutT, 128, 128, 8, 8>(p);
+    case 1: return launch_tile<T, OutT, 64, 128, 8, 8>(p);
+    case 2: return launch_tile<T, OutT, 64, 64, 4, 8>(p);
+    default: return launch_tile<T, OutT, 32, 64, 4, 4>(p);
+  }
 }
 
 // out_f32: C is float whatever the compute dtype.  groups <= 1 and offsets == nullptr: plain

@@ -49,3 +49,19 @@ def test_a_router_is_read_ahead_only_where_the_caller_says_so(monkeypatch, entry
     getattr(kernels, entry)(x, w, None, 2, True, 1.0)
     getattr(kernels, entry)(x, w, None, 2, True, 1.0, w_ahead=True)
     assert parts == [0, 1]
+
+
+TILES = ((128, 128, 1.0), (64, 128, 0.95), (64, 64, 0.8), (32, 64, 0.6))       # rows, columns, share of the FMA rate
+
+
+@pytest.mark.parametrize("sms", [148, 132])
+def test_the_float_tile_is_the_one_with_the_least_work_on_the_busiest_sm(sms):
+    pick = kernels.fn("snk_gemm_simt_tile")
+    seen = set()
+    for M, N, groups in [(17, 56, 0), (200, 2049, 0), (509, 2050, 0), (509, 8195, 0), (300, 6147, 0), (2048, 2048, 0),
+                         (8192, 64, 0), (40, 56, 8), (900, 3584, 32), (4096, 3584, 32)]:
+        mean = -(-M // groups) if groups else M
+        cost = [-(-(max(groups, 1) * -(-mean // bm) * -(-N // bn)) // sms) * bm * bn / rate for bm, bn, rate in TILES]
+        assert pick(M, N, groups, sms) == cost.index(min(cost))
+        seen.add(pick(M, N, groups, sms))
+    assert seen == {0, 1, 2, 3}
