@@ -343,13 +343,15 @@ static int launch_few(const SimtArgs& p) {
 // the FMA rate that its shared-memory reads leave.  The shares are those at 4,096 x 16,384 x 2,048 (128 x 128 5.16 ms, 64 x 128 5.28,
 // 64 x 64 6.64, 32 x 64 8.56).  Against all four tiles at 135 sizes (17 to 8,192 rows; N 64 to 16,384; K 640 to 8,192) the
 // choice was within 2 % of the fastest at 127, 3 to 6 % off at six, 9 and 12 % off at one each.
-// mean: rows of a group (of the product); sms: the device's.  0 to 3: 128 x 128, 64 x 128, 64 x 64, 32 x 64.
-static int pick_tile(int groups, long long mean, int N, int sms) {
+// rows: the most that one group can own, which the grid's 65,535 blocks along y have to hold (a lower tile that would not is
+// left out); mean: rows of a group (of the product); sms: the device's.  0 to 3: 128 x 128, 64 x 128, 64 x 64, 32 x 64.
+static int pick_tile(int groups, int rows, long long mean, int N, int sms) {
   static const int bm[4] = {128, 64, 64, 32}, bn[4] = {128, 128, 64, 64};
   static const double rate[4] = {1.0, 0.95, 0.8, 0.6};
   int best = 0;
   double least = 0.0;
   for (int t = 0; t < 4; ++t) {
+    if (t > 0 && (rows + bm[t] - 1ll) / bm[t] > 65535) continue;
     const long long tiles = (long long)groups * ((mean + bm[t] - 1) / bm[t]) * ((N + bn[t] - 1) / bn[t]);
     const double cost = (double)((tiles + sms - 1) / sms) * bm[t] * bn[t] / rate[t];
     if (t == 0 || cost < least) {
@@ -360,9 +362,10 @@ static int pick_tile(int groups, long long mean, int N, int sms) {
   return best;
 }
 
-// For tests: the tile that a product of M rows (of `groups` groups, 0: plain) takes on a device of that many SMs.
-SNK_API int snk_gemm_simt_tile(int M, int N, int groups, int sms) {
-  return pick_tile(groups ? groups : 1, groups ? (M + groups - 1) / groups : M, N, sms);
+// For tests: the tile that a product of M rows takes on a device of that many SMs (groups 0: plain; otherwise one group owns
+// `rows` rows at most).
+SNK_API int snk_gemm_simt_tile(int M, int N, int groups, int rows, int sms) {
+  return groups ? pick_tile(groups, rows, (M + groups - 1) / groups, N, sms) : pick_tile(1, M, M, N, sms);
 }
 
 template <typename T, typename OutT>
@@ -376,7 +379,7 @@ static int launch_tiles(const SimtArgs& p) {
   });
   if (rc) return rc;
   const int G = p.offsets ? p.groups : 1;
-  switch (pick_tile(G, p.offsets ? (p.M + G - 1) / G : p.M, p.N, sms)) {
+  switch (pick_tile(G, p.rows, p.offsets ? (p.M + G - 1) / G : p.M, p.N, sms)) {
     case 0: return launch_tile<T, OutT, 128, 128, 8, 8>(p);
     case 1: return launch_tile<T, OutT, 64, 128, 8, 8>(p);
     case 2: return launch_tile<T, OutT, 64, 64, 4, 8>(p);

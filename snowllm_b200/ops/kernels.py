@@ -60,7 +60,7 @@ _SIGNATURES = {
     },
     "gemm": {
         "snk_gemm_simt": [P, P, P, I, I, I, P, I, P, I, I, I, I, I, P],
-        "snk_gemm_simt_tile": [I, I, I, I],
+        "snk_gemm_simt_tile": [I, I, I, I, I],
     },
     "gemm_skinny": {
         "snk_gemm_skinny": [P, P, P, I, I, I, P, I, P, I, I, I, I, I, P],

@@ -62,6 +62,17 @@ def test_the_float_tile_is_the_one_with_the_least_work_on_the_busiest_sm(sms):
                          (8192, 64, 0), (40, 56, 8), (900, 3584, 32), (4096, 3584, 32)]:
         mean = -(-M // groups) if groups else M
         cost = [-(-(max(groups, 1) * -(-mean // bm) * -(-N // bn)) // sms) * bm * bn / rate for bm, bn, rate in TILES]
-        assert pick(M, N, groups, sms) == cost.index(min(cost))
-        seen.add(pick(M, N, groups, sms))
+        assert pick(M, N, groups, M, sms) == cost.index(min(cost))
+        seen.add(pick(M, N, groups, M, sms))
     assert seen == {0, 1, 2, 3}
+
+
+def test_a_float_product_of_millions_of_rows_keeps_a_tile_that_the_grid_can_hold():
+    """25,013 groups of 96 rows on average, one of which may own them all: of 32 x 64 tiles, the cheapest by their count, the
+    grid would need 75,039 along y.  A launch of 64-row tiles holds up to 4,194,240 rows."""
+    pick = kernels.fn("snk_gemm_simt_tile")
+    G, M = 25013, 25013 * 96
+    assert TILES[pick(M, 64, G, 1000, 148)][0] == 32
+    assert TILES[pick(M, 64, G, M, 148)][0] >= 64
+    for rows in (32 * 65535, 32 * 65535 + 1, 64 * 65535):
+        assert -(-rows // TILES[pick(rows, 64, rows // 75, rows, 148)][0]) <= 65535
