@@ -59,10 +59,10 @@ template <int MT, typename OutT, bool SWIGLU>
 __global__ void __launch_bounds__(SK_WARPS * 32)
 gemm_skinny_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, OutT* __restrict__ C, int M,
                    int N, int K, const int* __restrict__ a_rows, int a_div,
-                   const int* __restrict__ offsets, int groups, int act) {
+                   const int* __restrict__ offsets, int groups, int act, int w_ahead) {
 #if SK_PREFETCH_LINES > 0
-  if (offsets == nullptr) {
-    // A plain product's W is a constant and this block's 16 rows of it are known from the block's number
+  if (w_ahead && offsets == nullptr) {
+    // W is a weight (the caller says so) and this block's 16 rows of it are known from the block's number
     // alone: while the kernel before this one ends, ask L2 for the first lines of each row (128 bytes a
     // thread and round; no register is held, nothing is read into the SM).  A grouped product does not
     // know before the wait which groups own rows.  (Told by the caller that the offsets are older than the kernel in
@@ -507,20 +507,20 @@ static int stream_product(const CUtensorMap& map, const void* A, void* C, int M,
 template <int MT>
 static int launch_skinny(const void* A, const void* W, void* C, int M, int N, int K, const int* a_rows,
                          int a_div, const int* offsets, int groups, int out_f32, int swiglu, int split,
-                         cudaStream_t stream) {
+                         int w_ahead, cudaStream_t stream) {
   dim3 grid((N + SK_ROWS - 1) / SK_ROWS, offsets ? (groups < M ? groups : M) : 1, split);
   const dim3 block(SK_WARPS * 32);
   const bf16 *a = static_cast<const bf16*>(A), *w = static_cast<const bf16*>(W);
   const int unary = swiglu == SNK_ACT_RELU2 ? swiglu : 0;
   if (swiglu && !unary)
     snk_launch_cluster(gemm_skinny_kernel<MT, bf16, true>, grid, block, 0, stream, split, a, w,
-                       static_cast<bf16*>(C), M, N, K, a_rows, a_div, offsets, groups, swiglu);
+                       static_cast<bf16*>(C), M, N, K, a_rows, a_div, offsets, groups, swiglu, w_ahead);
   else if (out_f32)
     snk_launch_cluster(gemm_skinny_kernel<MT, float, false>, grid, block, 0, stream, split, a, w,
-                       static_cast<float*>(C), M, N, K, a_rows, a_div, offsets, groups, 0);
+                       static_cast<float*>(C), M, N, K, a_rows, a_div, offsets, groups, 0, w_ahead);
   else
     snk_launch_cluster(gemm_skinny_kernel<MT, bf16, false>, grid, block, 0, stream, split, a, w,
-                       static_cast<bf16*>(C), M, N, K, a_rows, a_div, offsets, groups, unary);
+                       static_cast<bf16*>(C), M, N, K, a_rows, a_div, offsets, groups, unary, w_ahead);
   SNK_LAUNCH_CHECK();
   return 0;
 }
@@ -548,10 +548,10 @@ SNK_API int snk_gemm_skinny(const void* A, const void* W, void* C, int M, int N,
     if (M <= 8) return stream_product<1>(map, A, C, M, N, K, out_f32, swiglu, split, w_ahead, stream);
     return stream_product<2>(map, A, C, M, N, K, out_f32, swiglu, split, w_ahead, stream);
   }
-  if (rows_hint <= 8) return launch_skinny<1>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);
-  if (rows_hint <= 16) return launch_skinny<2>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);
-  if (rows_hint <= 32) return launch_skinny<4>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);
-  return launch_skinny<8>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, stream);
+  if (rows_hint <= 8) return launch_skinny<1>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, w_ahead, stream);
+  if (rows_hint <= 16) return launch_skinny<2>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, w_ahead, stream);
+  if (rows_hint <= 32) return launch_skinny<4>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, w_ahead, stream);
+  return launch_skinny<8>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, w_ahead, stream);
 }
 
 // Test hook: with on != 0 the producers of later launches issue no loads, so that the bounded waits run out
