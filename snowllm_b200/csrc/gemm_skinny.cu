@@ -467,20 +467,57 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
   if (*aborted) drain_after_abort();
 }
 
+static int device_sms(int* sms) {
+  static std::atomic<int> sms_of[SNK_MAX_DEVICES];
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  return snk_per_device(sms_of, device, sms, [&](int* n) {
+    return (int)cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, device);
+  });
+}
+
+// Where the ring is the faster of the two kernels.  It gains at the start of a product and where N gives the kernel above
+// one to three blocks an SM, too few loads on their way; it loses where that one fills the SMs (4 and more strips an SM: 16 KB
+// a stage and 0.5 us of multiplying 8 rows hold a block to 4.9 TB/s of all SMs, there 5.9), where a strip is a short walk
+// (a round of strips costs more than its bytes), and where few strips are long walks, which the cluster above divides by four.
+// Measured in replayed chains of a norm and the product, M 1 / 4 / 8 / 16, us here (there):
+//   one round   2,048 x 2,048 5.7 (6.5) / 5.7 (6.6) / 5.9 (7.1) / 6.7 (8.9); 512 x 1,024 3.5 (4.0) / 3.8 (4.6) / 4.0 (4.7) / 4.2 (6.2);
+//               512 x 4,096 1.04 to 1.15 times there, 256 x 16,384 1.23 to 1.47, 2,048 x 10,752 0.94 / 1.04 / 1.04 / 0.89,
+//               2,048 x 20,480 1.04 to 1.18
+//   two         4,096 x 4,096 0.69 / 0.75 / 0.80 / 0.75 times there, x 1,024 0.98 / 0.99 / 1.02 / 0.90, x 256 1.07 / 1.04 / 1.05 / 0.99
+//   three       6,144 x 2,048 0.96 / 0.98 / 1.03 / 1.00, x 4,096 0.82 / 0.90 / 0.96 / 0.96, x 1,024 1.05 / 1.07 / 1.14 / 1.06,
+//               x 20,480 0.84 / 1.05 / 1.12 / 1.07
+//   more        8,192 x 2,048 1.02 / 1.06 / 1.13 / 1.11, 16,384 x 2,048 0.91 / 0.99 / 1.08 / 1.04 (but gate|up and down of 2,048 and 7,168
+//               together 25.7 / 27.8 / 29.8 / 35.3 us with gate|up here, 24.1 / 25.0 / 25.7 / 31.4 with it there), 65,536 x 2,048 1.12 /
+//               1.12 / 1.28 / 1.26, 128,256 x 1,024 1.39 to 1.51
+static bool stream_pays(int N, int K, int sms) {
+  const int strips = (N + SK_ROWS - 1) / SK_ROWS, rounds = (strips + sms - 1) / sms;
+  if (rounds <= 1) return K <= 2560 || (strips >= sms * 3 / 4 && K <= 12288);
+  if (rounds == 2) return K >= 512;
+  return rounds == 3 && K >= 2048 && K <= 16384;
+}
+
+// For tests: whether a plain product of these sizes streams W through shared memory on a device of that many SMs.
+SNK_API int snk_gemm_skinny_streams(int M, int N, int K, int sms) {
+  return M <= ST_MAX_ROWS && K % 64 == 0 && stream_pays(N, K, sms);
+}
+
 template <int MT, typename OutT, bool SWIGLU, int SPLIT>
-static int launch_stream(const CUtensorMap& map, const bf16* A, void* C, int M, int N, int K, int act, int w_ahead,
+static int launch_stream(const CUtensorMap& map, const bf16* A, void* C, int M, int N, int K, int act, int w_ahead, int sms,
                          cudaStream_t stream) {
   constexpr int sums = (SPLIT == 1 ? 2 : 1) * SPLIT * SK_WARPS * MT * 8 * (SK_ROWS + 1) * (int)sizeof(float);
   // two products' rings on one SM: 6 stages of 16 KB, fewer where the sums take the room
   constexpr int room = (110 * 1024 - sums - (int)sizeof(StShared)) / ST_BYTES, stages = room < 6 ? room : 6;
   constexpr int smem = 1024 + stages * ST_BYTES + sums + (int)sizeof(StShared);
-  static std::atomic<int> sms_of[SNK_MAX_DEVICES];
-  int device = 0, sms = 0;
+  static std::atomic<int> limit_set[SNK_MAX_DEVICES];
+  int device = 0, set = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return (int)e;
-  const int rc = snk_per_device(sms_of, device, &sms, [&](int* n) {
-    e = cudaFuncSetAttribute(gemm_stream_kernel<MT, OutT, SWIGLU, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return (int)(e != cudaSuccess ? e : cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, device));
+  const int rc = snk_per_device(limit_set, device, &set, [&](int* n) {
+    *n = 1;
+    return (int)cudaFuncSetAttribute(gemm_stream_kernel<MT, OutT, SWIGLU, SPLIT>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   });
   if (rc) return rc;
   const int strips = (N + SK_ROWS - 1) / SK_ROWS;
@@ -492,16 +529,16 @@ static int launch_stream(const CUtensorMap& map, const bf16* A, void* C, int M, 
 
 template <int MT>
 static int stream_product(const CUtensorMap& map, const void* A, void* C, int M, int N, int K, int out_f32, int swiglu,
-                          int split, int w_ahead, cudaStream_t stream) {
+                          int split, int w_ahead, int sms, cudaStream_t stream) {
   const bf16* a = static_cast<const bf16*>(A);
   if (swiglu && swiglu != SNK_ACT_RELU2)
-    return split > 1 ? launch_stream<MT, bf16, true, SK_SPLIT>(map, a, C, M, N, K, swiglu, w_ahead, stream)
-                     : launch_stream<MT, bf16, true, 1>(map, a, C, M, N, K, swiglu, w_ahead, stream);
+    return split > 1 ? launch_stream<MT, bf16, true, SK_SPLIT>(map, a, C, M, N, K, swiglu, w_ahead, sms, stream)
+                     : launch_stream<MT, bf16, true, 1>(map, a, C, M, N, K, swiglu, w_ahead, sms, stream);
   if (out_f32)
-    return split > 1 ? launch_stream<MT, float, false, SK_SPLIT>(map, a, C, M, N, K, 0, w_ahead, stream)
-                     : launch_stream<MT, float, false, 1>(map, a, C, M, N, K, 0, w_ahead, stream);
-  return split > 1 ? launch_stream<MT, bf16, false, SK_SPLIT>(map, a, C, M, N, K, swiglu, w_ahead, stream)
-                   : launch_stream<MT, bf16, false, 1>(map, a, C, M, N, K, swiglu, w_ahead, stream);
+    return split > 1 ? launch_stream<MT, float, false, SK_SPLIT>(map, a, C, M, N, K, 0, w_ahead, sms, stream)
+                     : launch_stream<MT, float, false, 1>(map, a, C, M, N, K, 0, w_ahead, sms, stream);
+  return split > 1 ? launch_stream<MT, bf16, false, SK_SPLIT>(map, a, C, M, N, K, swiglu, w_ahead, sms, stream)
+                   : launch_stream<MT, bf16, false, 1>(map, a, C, M, N, K, swiglu, w_ahead, sms, stream);
 }
 
 template <int MT>
@@ -540,13 +577,18 @@ SNK_API int snk_gemm_skinny(const void* A, const void* W, void* C, int M, int N,
   if (groups > 65535) return SNK_ERR_SIZE;
   if (a_div <= 0) a_div = 1;
   const int split = skinny_split(N, K, offsets);
-  // K in whole blocks of 64 columns, one pass: W through shared memory
+  // K in whole blocks of 64 columns, one pass: W through shared memory, where that is the faster way
   if (!offsets && !a_rows && M <= ST_MAX_ROWS && K % 64 == 0) {
-    CUtensorMap map;
-    const int rc = tensor_map(W, N, K, SK_ROWS, 0, &map, ST_RUNS / 2);
+    int sms = 0;
+    int rc = device_sms(&sms);
     if (rc) return rc;
-    if (M <= 8) return stream_product<1>(map, A, C, M, N, K, out_f32, swiglu, split, w_ahead, stream);
-    return stream_product<2>(map, A, C, M, N, K, out_f32, swiglu, split, w_ahead, stream);
+    if (stream_pays(N, K, sms)) {
+      CUtensorMap map;
+      rc = tensor_map(W, N, K, SK_ROWS, 0, &map, ST_RUNS / 2);
+      if (rc) return rc;
+      if (M <= 8) return stream_product<1>(map, A, C, M, N, K, out_f32, swiglu, split, w_ahead, sms, stream);
+      return stream_product<2>(map, A, C, M, N, K, out_f32, swiglu, split, w_ahead, sms, stream);
+    }
   }
   if (rows_hint <= 8) return launch_skinny<1>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, w_ahead, stream);
   if (rows_hint <= 16) return launch_skinny<2>(A, W, C, M, N, K, a_rows, a_div, offsets, groups, out_f32, swiglu, split, w_ahead, stream);

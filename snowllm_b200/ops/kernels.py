@@ -64,6 +64,7 @@ _SIGNATURES = {
     },
     "gemm_skinny": {
         "snk_gemm_skinny": [P, P, P, I, I, I, P, I, P, I, I, I, I, I, P],
+        "snk_gemm_skinny_streams": [I, I, I, I],
         "snk_gemm_skinny_status": [],
         "snk_gemm_skinny_status_peek": [P, P],
         "snk_gemm_skinny_test_lose_loads": [I],

@@ -76,3 +76,14 @@ def test_a_float_product_of_millions_of_rows_keeps_a_tile_that_the_grid_can_hold
     assert TILES[pick(M, 64, G, M, 148)][0] >= 64
     for rows in (32 * 65535, 32 * 65535 + 1, 64 * 65535):
         assert -(-rows // TILES[pick(rows, 64, rows // 75, rows, 148)][0]) <= 65535
+
+
+def test_which_few_rows_products_stream_w_through_shared_memory():
+    """148 SMs: up to 2,368 rows of W are one round of strips, up to 4,736 two, up to 7,104 three."""
+    streams = kernels.fn("snk_gemm_skinny_streams")
+    for (N, K), want in {(16, 2560): 1, (16, 2624): 0, (1760, 4096): 0, (1776, 4096): 1, (2368, 12288): 1, (2368, 12352): 0,
+                         (2369, 448): 0, (2369, 512): 1, (4736, 65536): 1, (4737, 512): 0, (4737, 2048): 1, (7104, 16384): 1,
+                         (7104, 16448): 0, (7105, 2048): 0, (65536, 2048): 0, (2048, 2080): 0}.items():
+        for M in (1, 16):
+            assert streams(M, N, K, 148) == want, (N, K)
+        assert streams(17, N, K, 148) == 0
