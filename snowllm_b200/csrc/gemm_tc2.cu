@@ -279,10 +279,13 @@ struct T2GMaps {
   CUtensorMap a[T2G_BOXES];
 };
 // What every block works out of the offsets: the groups by row-tile length, and the items before each.
+#define T2G_LENGTHS (2 * T2_BM / 16 + 1)
 struct T2GPlan {
   int first[T2G_MAX_GROUPS + 1];
   int order[T2G_MAX_GROUPS];
   int rows[T2G_MAX_GROUPS];          // rows of a full row tile of each group
+  int items[T2G_MAX_GROUPS];         // tiles of each group
+  int place[T2G_LENGTHS];            // where the next group of a row-tile length goes
   int longest;                       // rows of the longest row tile
 };
 
@@ -296,40 +299,86 @@ __device__ __forceinline__ int t2g_tile_rows(int cnt) {
   return row_tiles ? ((cnt + row_tiles - 1) / row_tiles + 15) & ~15 : 0;
 }
 
-// By all threads of the block; ends with a barrier.
+// The sum over the lanes up to this one.
+__device__ __forceinline__ int t2g_running(int v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int before = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += before;
+  }
+  return v;
+}
+
+// By all threads of the block; ends with a barrier.  One warp sorts the groups, equal lengths in the groups' own order (every block
+// comes to the same plan).  Up to 32 groups: a lane per group, which compares its own with all others in registers.  More:
+// by counting (a row tile is 0, 16, .. or 256 rows long), 32 groups at a time.  Measured against each group's thread
+// comparing it with all others through shared memory: 256 groups of 512 x 512, 1,032 rows 41.5 -> 37.1 us (35.6 in the groups' own
+// order), 8 groups of 512 x 256, 128 rows 8.5 -> 8.4 us (9.0 by counting).
 __device__ __forceinline__ void t2g_plan(T2GPlan* plan, const int* __restrict__ offsets, int groups, int n_tiles) {
+  if (groups <= 32) {
+    const int lane = threadIdx.x;                        // (only the first warp's threads have a group)
+    const int cnt = lane < groups ? offsets[lane + 1] - offsets[lane] : 0;
+    const int mine = t2g_tile_rows(cnt), items = t2g_row_tiles(cnt) * n_tiles;
+    int place = 0, before = 0, all = 0;
+    for (int o = 0; o < groups && threadIdx.x < 32; ++o) {
+      const int rows = __shfl_sync(0xffffffffu, mine, o), its = __shfl_sync(0xffffffffu, items, o);
+      if (rows > mine || (rows == mine && o < lane)) {
+        ++place;
+        before += its;
+      }
+      all += its;
+    }
+    if (lane < groups) {
+      plan->rows[lane] = mine;
+      plan->order[place] = lane;
+      plan->first[place] = before;
+      if (place == 0) plan->longest = mine;
+    }
+    if (lane == 0) plan->first[groups] = all;
+    __syncthreads();
+    return;
+  }
   for (int e = threadIdx.x; e < groups; e += blockDim.x) {
     const int cnt = offsets[e + 1] - offsets[e];
     plan->rows[e] = t2g_tile_rows(cnt);
-    plan->first[e + 1] = t2g_row_tiles(cnt) * n_tiles;   // the group's items, in group order for now
+    plan->items[e] = t2g_row_tiles(cnt) * n_tiles;
   }
   __syncthreads();
-  constexpr int EACH = (T2G_MAX_GROUPS + T2_THREADS - 1) / T2_THREADS;
-  int place[EACH], before[EACH], all = 0;
-#pragma unroll
-  for (int i = 0; i < EACH; ++i) {
-    const int e = threadIdx.x + i * blockDim.x;
-    if (e >= groups) break;
-    const int mine = plan->rows[e];
-    place[i] = before[i] = all = 0;
-    for (int o = 0; o < groups; ++o) {
-      const int r = plan->rows[o], items = plan->first[o + 1];
-      if (r > mine || (r == mine && o < e)) {
-        ++place[i];
-        before[i] += items;
-      }
-      all += items;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const unsigned below = (1u << lane) - 1;
+    if (lane < T2G_LENGTHS) plan->place[lane] = 0;
+    __syncwarp();
+    for (int e0 = 0; e0 < groups; e0 += 32) {            // how many groups have a length
+      const int e = e0 + lane, len = e < groups ? plan->rows[e] >> 4 : -1;
+      const unsigned same = __match_any_sync(0xffffffffu, len);
+      if (len >= 0 && !(same & below)) plan->place[len] += __popc(same);
+      __syncwarp();
     }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < EACH; ++i) {
-    const int e = threadIdx.x + i * blockDim.x;
-    if (e >= groups) break;
-    plan->order[place[i]] = e;
-    plan->first[place[i]] = before[i];
-    if (place[i] == 0) plan->longest = plan->rows[e];
-    if (e == 0) plan->first[groups] = all;
+    const int len_here = T2G_LENGTHS - 1 - lane;         // longest first
+    const int have = lane < T2G_LENGTHS ? plan->place[len_here] : 0;
+    const int upto_here = t2g_running(have, lane);
+    if (lane < T2G_LENGTHS) plan->place[len_here] = upto_here - have;
+    __syncwarp();
+    for (int e0 = 0; e0 < groups; e0 += 32) {
+      const int e = e0 + lane, len = e < groups ? plan->rows[e] >> 4 : -1;
+      const unsigned same = __match_any_sync(0xffffffffu, len);
+      if (len >= 0) plan->order[plan->place[len] + __popc(same & below)] = e;
+      __syncwarp();
+      if (len >= 0 && !(same & below)) plan->place[len] += __popc(same);
+      __syncwarp();
+    }
+    int run = 0;
+    for (int p0 = 0; p0 < groups; p0 += 32) {
+      const int p = p0 + lane, mine = p < groups ? plan->items[plan->order[p]] : 0;
+      const int upto = t2g_running(mine, lane);
+      if (p < groups) plan->first[p] = run + upto - mine;
+      run += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (lane == 0) {
+      plan->first[groups] = run;
+      plan->longest = plan->rows[plan->order[0]];
+    }
   }
   __syncthreads();
 }

@@ -671,6 +671,27 @@ def test_gemm_tc2_grouped_rows_on_the_n_side(K, N, K_):
     assert K.gemm_tc2_status()[0] == 0
 
 
+@pytest.mark.parametrize("counts", [[64, 3, 0, 49], [65, 1, 64], [128, 17, 0, 96, 112], [129, 64, 5], [256] + [16] * 40, [257],
+                                    [(7 * e) % 23 * (e % 5 != 0) for e in range(200)], [(e % 13) * (e % 29) for e in range(256)]])
+def test_gemm_tc2_grouped_rings_and_plans(K, counts):
+    """The grouped pair product where its ring changes (row tiles of up to 64, up to 128 and more rows: 10, 8 and 6 stages),
+    with more than two rounds of the ring (26 k-blocks), and its plan of many groups, longest row tiles first."""
+    G, M, N, K_ = len(counts), sum(counts), 264, 26 * 64
+    gen = torch.Generator(device="cuda").manual_seed(41)
+    a = torch.randn(M, K_, device="cuda", generator=gen).to(torch.bfloat16)
+    w = torch.randn(G, N, K_, device="cuda", generator=gen).to(torch.bfloat16)
+    offsets = torch.tensor([0] + counts).cumsum(0).to(torch.int32).cuda()
+    out = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    K.gemm_tc2(a, w, out_dtype=torch.float32, offsets=offsets, out=out)
+    assert K.gemm_tc2_status()[0] == 0
+    lo = 0
+    for e, n in enumerate(counts):
+        want = a[lo:lo + n].double() @ w[e].double().T
+        # a step of the float sum per 16 columns, each rounding 2^-23 of a partial sum of at most about 4 sqrt(K)
+        assert n == 0 or float((out[lo:lo + n].double() - want).abs().max()) <= 2.0 ** -23 * (K_ / 16) * 4 * K_ ** 0.5
+        lo += n
+
+
 def test_gemm_tc_grouped_after_gather(K):
     torch.manual_seed(31)
     dtype = torch.bfloat16
