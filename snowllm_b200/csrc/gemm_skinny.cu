@@ -90,25 +90,31 @@ gemm_skinny_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, OutT*
     // groups > gridDim.y: there are fewer rows than groups, and block y takes the y-th group that owns any (every warp
     // looks it up for itself).  One token with the top 4 of 32 experts then starts 896 blocks and not 7,168 of which
     // 6,272 end at once: 18.8 -> 16 us of the gate|up product in the decode step.  (With as many rows as groups, 8 such
-    // tokens, the look-up cost as much as it saved.)
+    // tokens, the look-up cost as much as it saved.)  The look-up has the group's rows in its registers: no second read.
     int e = blockIdx.y;
     if (groups > (int)gridDim.y) {
       int left = blockIdx.y;
       e = -1;
       for (int e0 = 0; e0 < groups; e0 += 32) {
-        const bool owns = e0 + lane < groups && offsets[e0 + lane + 1] > offsets[e0 + lane];
+        const bool in = e0 + lane < groups;
+        const int begin = in ? offsets[e0 + lane] : 0, end = in ? offsets[e0 + lane + 1] : 0;
+        const bool owns = end > begin;
         const unsigned own = __ballot_sync(0xffffffffu, owns);
         const unsigned it = __ballot_sync(0xffffffffu, owns && __popc(own & ((1u << lane) - 1)) == left);
         if (it) {
-          e = e0 + __ffs(it) - 1;
+          const int from = __ffs(it) - 1;
+          e = e0 + from;
+          row_begin = __shfl_sync(0xffffffffu, begin, from);
+          row_end = __shfl_sync(0xffffffffu, end, from);
           break;
         }
         left -= __popc(own);
       }
       if (e < 0) return;
+    } else {
+      row_begin = offsets[e];
+      row_end = offsets[e + 1];
     }
-    row_begin = offsets[e];
-    row_end = offsets[e + 1];
     Wg = W + (size_t)e * N * K;
   }
   if (row_begin >= row_end) return;
