@@ -260,7 +260,7 @@ static int launch_tc2(const CUtensorMap& map_a, const CUtensorMap& map_w, void* 
 // tokens, as pairs side by side then read far-apart memory; items drawn from a counter as pairs get free,
 // 159 us; L2 prefetch of an item's rows of W in one piece, 184 to 198 us.)
 //
-// Groups come in the order of their row tiles' length, longest first: a round of items then has one length, and the
+// Up to 32 groups come in the order of their row tiles' length, longest first: a round of items then has one length, and the
 // shortest make the last, partly filled one.
 //
 // Groups of few rows are bound by the read of W, and that by the bytes an SM keeps on their way: a stage's part for A
@@ -278,14 +278,11 @@ static int launch_tc2(const CUtensorMap& map_a, const CUtensorMap& map_w, void* 
 struct T2GMaps {
   CUtensorMap a[T2G_BOXES];
 };
-// What every block works out of the offsets: the groups by row-tile length, and the items before each.
-#define T2G_LENGTHS (2 * T2_BM / 16 + 1)
+// What every block works out of the offsets: the groups in the order they are taken, and the items before each.
 struct T2GPlan {
   int first[T2G_MAX_GROUPS + 1];
   int order[T2G_MAX_GROUPS];
   int rows[T2G_MAX_GROUPS];          // rows of a full row tile of each group
-  int items[T2G_MAX_GROUPS];         // tiles of each group
-  int place[T2G_LENGTHS];            // where the next group of a row-tile length goes
   int longest;                       // rows of the longest row tile
 };
 
@@ -299,21 +296,12 @@ __device__ __forceinline__ int t2g_tile_rows(int cnt) {
   return row_tiles ? ((cnt + row_tiles - 1) / row_tiles + 15) & ~15 : 0;
 }
 
-// The sum over the lanes up to this one.
-__device__ __forceinline__ int t2g_running(int v, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int before = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += before;
-  }
-  return v;
-}
-
-// By all threads of the block; ends with a barrier.  One warp sorts the groups, equal lengths in the groups' own order (every block
-// comes to the same plan).  Up to 32 groups: a lane per group, which compares its own with all others in registers.  More:
-// by counting (a row tile is 0, 16, .. or 256 rows long), 32 groups at a time.  Measured against each group's thread
-// comparing it with all others through shared memory: 256 groups of 512 x 512, 1,032 rows 41.5 -> 37.1 us (35.6 in the groups' own
-// order), 8 groups of 512 x 256, 128 rows 8.5 -> 8.4 us (9.0 by counting).
+// By all threads of the block; ends with a barrier.  Up to 32 groups are put in order, equal lengths in the groups' own order (every
+// block comes to the same plan), by a lane per group that compares its own with all others in registers.  More groups stay in
+// their own order: what the other order gains there, 0 to 3 %, is less than it costs.  Measured, us: groups in their own order
+// for all, their sum by one thread / every group in order, compared through shared memory / so: 256 groups of 512 x 512, 1,032 rows
+// 35.5 / 41.5 / 35.1; 40 of 512 x 1,024, half of 8,192 rows in one group 28.1 / 32.4 / 28.7; 64 of 768 x 2,048, 16,384 rows 87.4 /
+// 85.6 / 88.2; 8 of 512 x 256, 128 rows 8.2 / 8.5 / 8.4.
 __device__ __forceinline__ void t2g_plan(T2GPlan* plan, const int* __restrict__ offsets, int groups, int n_tiles) {
   if (groups <= 32) {
     const int lane = threadIdx.x;                        // (only the first warp's threads have a group)
@@ -341,43 +329,30 @@ __device__ __forceinline__ void t2g_plan(T2GPlan* plan, const int* __restrict__ 
   for (int e = threadIdx.x; e < groups; e += blockDim.x) {
     const int cnt = offsets[e + 1] - offsets[e];
     plan->rows[e] = t2g_tile_rows(cnt);
-    plan->items[e] = t2g_row_tiles(cnt) * n_tiles;
+    plan->order[e] = e;
+    plan->first[e] = t2g_row_tiles(cnt) * n_tiles;       // the group's items, for now
   }
   __syncthreads();
   if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    const unsigned below = (1u << lane) - 1;
-    if (lane < T2G_LENGTHS) plan->place[lane] = 0;
-    __syncwarp();
-    for (int e0 = 0; e0 < groups; e0 += 32) {            // how many groups have a length
-      const int e = e0 + lane, len = e < groups ? plan->rows[e] >> 4 : -1;
-      const unsigned same = __match_any_sync(0xffffffffu, len);
-      if (len >= 0 && !(same & below)) plan->place[len] += __popc(same);
-      __syncwarp();
-    }
-    const int len_here = T2G_LENGTHS - 1 - lane;         // longest first
-    const int have = lane < T2G_LENGTHS ? plan->place[len_here] : 0;
-    const int upto_here = t2g_running(have, lane);
-    if (lane < T2G_LENGTHS) plan->place[len_here] = upto_here - have;
-    __syncwarp();
-    for (int e0 = 0; e0 < groups; e0 += 32) {
-      const int e = e0 + lane, len = e < groups ? plan->rows[e] >> 4 : -1;
-      const unsigned same = __match_any_sync(0xffffffffu, len);
-      if (len >= 0) plan->order[plan->place[len] + __popc(same & below)] = e;
-      __syncwarp();
-      if (len >= 0 && !(same & below)) plan->place[len] += __popc(same);
-      __syncwarp();
-    }
-    int run = 0;
-    for (int p0 = 0; p0 < groups; p0 += 32) {
-      const int p = p0 + lane, mine = p < groups ? plan->items[plan->order[p]] : 0;
-      const int upto = t2g_running(mine, lane);
-      if (p < groups) plan->first[p] = run + upto - mine;
+    int run = 0, longest = 0;
+    for (int e = threadIdx.x; e - (int)threadIdx.x < groups; e += 32) {
+      const int items = e < groups ? plan->first[e] : 0;
+      int upto = items;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int before = __shfl_up_sync(0xffffffffu, upto, o);
+        if ((int)threadIdx.x >= o) upto += before;
+      }
+      if (e < groups) {
+        plan->first[e] = run + upto - items;
+        longest = max(longest, plan->rows[e]);
+      }
       run += __shfl_sync(0xffffffffu, upto, 31);
     }
-    if (lane == 0) {
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (threadIdx.x == 0) {
       plan->first[groups] = run;
-      plan->longest = plan->rows[plan->order[0]];
+      plan->longest = longest;
     }
   }
   __syncthreads();
