@@ -1,5 +1,6 @@
-"""float32 products at the edges of their kernels (chunks of 128 columns, strips of 16, passes of 2 to 16 rows; tiles of 32 to
-128): every output is one thread's sum in order of k, so few rows and many come to the same bits."""
+"""float32 products at the edges of their kernels (chunks of 128 columns, strips of 16, passes of 2 to 16 rows; each of the four
+tiles with ragged edges): every output is one thread's sum in order of k, so few rows and many come to the same bits, and so do
+bfloat16 operands and the same values in float32."""
 import pytest
 import torch
 
@@ -36,4 +37,43 @@ def test_groups(counts):
     for e, n in enumerate(counts):
         if n:
             assert torch.equal(out[lo:lo + n], kernels.gemm_simt(x[(rows[lo:lo + n] // 2).long()].contiguous(), w[e]))
+        lo += n
+
+
+def tile_of(M, N, groups, rows):
+    from snowllm_b200.ops import kernels
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return kernels.fn("snk_gemm_simt_tile")(M, N, groups, rows, sms)
+
+
+# tiles 128 x 128, 64 x 128, 64 x 64 and 32 x 64; K in vectors of four, odd (element by element), less than a step of 16
+@pytest.mark.parametrize("K", [12, 132, 645])
+@pytest.mark.parametrize("M,N,tile", [(300, 6147, 0), (1000, 1999, 0), (509, 2050, 1), (130, 4099, 1), (200, 2049, 2),
+                                      (1100, 2051, 2), (33, 130, 3)])
+def test_every_tile_at_its_edges(M, N, tile, K):
+    from snowllm_b200.ops import kernels
+    assert tile_of(M, N, 0, M) == tile
+    a, w = operands(M, K, seed=6).to(torch.bfloat16), operands(N, K, seed=7).to(torch.bfloat16)
+    out = kernels.gemm_simt(a.float(), w.float())
+    want = a.double() @ w.double().T
+    assert float((out.double() - want).abs().max()) <= 2.0 ** -24 * K * 4 * K ** 0.5
+    for lo in (0, M // 2, M - 16):                     # the few-rows kernel (K a multiple of 4) or a lower tile
+        assert torch.equal(kernels.gemm_simt(a[lo:lo + 16].float(), w.float()), out[lo:lo + 16])
+    assert torch.equal(kernels.gemm_simt(a, w, out_dtype=torch.float32), out)
+    assert torch.equal(kernels.gemm_simt(a, w), out.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("N,tile", [(2051, 0), (1027, 1), (515, 2)])
+def test_groups_on_the_larger_tiles(N, tile):
+    from snowllm_b200.ops import kernels
+    counts, K = [300, 0, 517, 129], 132
+    G, M = len(counts), sum(counts)
+    assert tile_of(M, N, G, M) == tile
+    x, w = operands(M, K, seed=8), operands(G, N, K, seed=9)
+    offsets = torch.tensor([0] + counts).cumsum(0).to(torch.int32).cuda()
+    out = kernels.gemm_simt(x, w, offsets=offsets, rows_out=M, max_rows_per_group=M)
+    lo = 0
+    for e, n in enumerate(counts):
+        if n:
+            assert torch.equal(out[lo:lo + n], kernels.gemm_simt(x[lo:lo + n], w[e]))
         lo += n
