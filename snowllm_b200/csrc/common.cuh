@@ -11,6 +11,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include "per_device.h"
+
 #define SNK_API extern "C" __attribute__((visibility("default")))
 
 enum { SNK_F32 = 0, SNK_BF16 = 1 };
@@ -245,6 +247,17 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t snk_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               Args&&... args) {
   return snk_launch_cluster(kernel, grid, block, smem, stream, 1, static_cast<Args&&>(args)...);
+}
+
+// The SMs of the current device; 0 or the CUDA error.
+inline int snk_device_sms(int* sms) {
+  static std::atomic<int> sms_of[SNK_MAX_DEVICES];
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  return snk_per_device(sms_of, device, sms, [&](int* n) {
+    return (int)cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, device);
+  });
 }
 
 #define SNK_LAUNCH_CHECK()                       \

@@ -12,7 +12,6 @@
 // (the role of snowllm/ops/gemm.py:33-41 and of the expert products in
 // snowllm/ops/inference.py:60-76)
 #include "common.cuh"
-#include "per_device.h"
 
 // Four values of a row as they are fetched, to be turned into floats where they are used: what is computed from a load ends
 // the time in which the load may be on its way.  (bfloat16, K = 2,044, converted at the fetch / at the store to shared memory: 17 x
@@ -390,13 +389,8 @@ SNK_API int snk_gemm_simt_tile(int M, int N, int groups, int rows, int sms) {
 
 template <typename T, typename OutT>
 static int launch_tiles(const SimtArgs& p) {
-  static std::atomic<int> sms_of[SNK_MAX_DEVICES];
-  int device = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return (int)e;
-  const int rc = snk_per_device(sms_of, device, &sms, [&](int* n) {
-    return (int)cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, device);
-  });
+  int sms = 0;
+  const int rc = snk_device_sms(&sms);
   if (rc) return rc;
   const int G = p.offsets ? p.groups : 1;
   switch (pick_tile(G, p.rows, p.offsets ? (p.M + G - 1) / G : p.M, p.N, sms)) {

@@ -21,7 +21,6 @@
 // A group with more than 64 rows is walked in passes of 64 (W is then re-read from L2).
 // (the role of snowllm/ops/gemm.py:33-41 and the expert products of snowllm/ops/inference.py:60-76
 // at decode shapes)
-#include "per_device.h"
 #include "tma.cuh"
 
 #ifndef SK_WARPS
@@ -473,16 +472,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
   if (*aborted) drain_after_abort();
 }
 
-static int device_sms(int* sms) {
-  static std::atomic<int> sms_of[SNK_MAX_DEVICES];
-  int device = 0;
-  const cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return (int)e;
-  return snk_per_device(sms_of, device, sms, [&](int* n) {
-    return (int)cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, device);
-  });
-}
-
 // Where the ring is the faster of the two kernels.  It gains at the start of a product and where N gives the kernel above
 // one to three blocks an SM, too few loads on their way; it loses where that one fills the SMs (4 and more strips an SM: 16 KB
 // a stage and 0.5 us of multiplying 8 rows hold a block to 4.9 TB/s of all SMs, there 5.9), where a strip is a short walk
@@ -586,7 +575,7 @@ SNK_API int snk_gemm_skinny(const void* A, const void* W, void* C, int M, int N,
   // K in whole blocks of 64 columns, one pass: W through shared memory, where that is the faster way
   if (!offsets && !a_rows && M <= ST_MAX_ROWS && K % 64 == 0) {
     int sms = 0;
-    int rc = device_sms(&sms);
+    int rc = snk_device_sms(&sms);
     if (rc) return rc;
     if (stream_pays(N, K, sms)) {
       CUtensorMap map;
