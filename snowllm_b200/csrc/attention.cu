@@ -215,16 +215,20 @@ __global__ void paged_attention_kernel(
 
 // Merge the chunks of one (row, head).  The first warp finds the running maximum and the normaliser
 // over the chunks (lanes take chunks in turns, then a butterfly) and leaves the chunks' factors in shared memory.  The
-// chunks are then cut into MERGE_ZG runs; a thread sums four neighbouring elements of the output (one, where hd is no
-// multiple of four) over one run in chunk order, and the runs' sums are added in run order: many short chains of loads instead of one long one.  Bound by
-// the latency of those loads, so the blocks are small and all of a step's are on the SMs at once: with a thread per
-// element and run, and the factors formed by each, 64 rows of
-// 32 heads and up to 33 chunks took 18.4 us from the end of the attention to the end of the merge, now 7.7.
+// chunks are then cut into MERGE_ZG runs; a thread sums a few neighbouring elements of the output over one run in chunk
+// order, and the runs' sums are added in run order: many short chains of loads instead of one long one.  Bound by the
+// latency of those loads.  With many rows the blocks are small, four elements a thread, so that all of a step's are on the
+// SMs at once: with a thread per element and run, and the factors formed by each, 64 rows of 32 heads and up to 33 chunks
+// took 18.4 us from the end of the attention to the end of the merge, now 7.7.  With few rows (launch_merge) there is room,
+// and two elements a thread keep eight chunks' loads on their way at once where four would need the registers of eight
+// 16-byte loads: 32 heads of 64, 1 row, 33 / 128 / 600 chunks 3.3 / 3.2 / 9.4 us, with four 3.9 / 4.2 / 13.1.
 #define MERGE_ZG 4
 #define MERGE_MAX_FACTORS 4096      // chunks whose factors fit beside the sums; more are formed where they are used
+#define MERGE_AHEAD 4               // chunks a lane of the first warp holds in registers
 
-// VEC 4: hd is a multiple of 4 and part_o lies on 16 bytes; otherwise VEC 1, an element at a time.
-template <typename T, int VEC>
+// VEC elements a thread: 4 (or 2) where hd is a multiple of that and part_o lies on as many floats, otherwise 1.  KEPT: num_chunks is
+// at most MERGE_MAX_FACTORS (known at compile time for the registers' sake: 56 a thread, with the choice inside 66).
+template <typename T, int VEC, bool KEPT>
 __global__ void attention_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                        const int* __restrict__ positions, T* __restrict__ out, int nh,
                                        int hd, int window, int chunk, int num_chunks,
@@ -233,7 +237,6 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
   pdl_begin();
   extern __shared__ __align__(16) float merge_sh[];        // [MERGE_ZG][hd], then the factors
   float* factors = merge_sh + MERGE_ZG * hd;
-  const bool kept = num_chunks <= MERGE_MAX_FACTORS;
   __shared__ float s_mx, s_inv;
   const int m = row_list ? row_list[blockIdx.x] : blockIdx.x, head = blockIdx.y;
   const int pos = positions[m];
@@ -241,14 +244,31 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
   const size_t base = ((size_t)blockIdx.x * nh + head) * num_chunks;
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
-    float mx = -INFINITY;
-    for (int z = lane; z < n; z += 32) mx = fmaxf(mx, part_ml[(base + z) * 2]);
+    float first_mx[MERGE_AHEAD], first_l[MERGE_AHEAD], mx = -INFINITY;       // the lane's first chunks, read once
+#pragma unroll
+    for (int i = 0; i < MERGE_AHEAD; ++i) {
+      const int z = lane + 32 * i;
+      first_mx[i] = z < n ? part_ml[(base + z) * 2] : -INFINITY;
+      first_l[i] = z < n ? part_ml[(base + z) * 2 + 1] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < MERGE_AHEAD; ++i) mx = fmaxf(mx, first_mx[i]);
+    for (int z = lane + 32 * MERGE_AHEAD; z < n; z += 32) mx = fmaxf(mx, part_ml[(base + z) * 2]);
     mx = warp_max(mx);
     float l = 0.f;
-    for (int z = lane; z < n; z += 32) {
+#pragma unroll
+    for (int i = 0; i < MERGE_AHEAD; ++i) {
+      const int z = lane + 32 * i;
+      if (z >= n) break;
+      const float f = expf(first_mx[i] - mx);
+      l += first_l[i] * f;
+      if constexpr (KEPT) factors[z] = f;
+    }
+#pragma unroll 4
+    for (int z = lane + 32 * MERGE_AHEAD; z < n; z += 32) {
       const float f = expf(part_ml[(base + z) * 2] - mx);
       l += part_ml[(base + z) * 2 + 1] * f;
-      if (kept) factors[z] = f;
+      if constexpr (KEPT) factors[z] = f;
     }
     l = warp_sum(l);
     if (lane == 0) { s_mx = mx; s_inv = 1.f / l; }
@@ -266,11 +286,16 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
 #pragma unroll 8
     for (int z = z0; z < z1; ++z) {
       const float* from = part_o + (base + z) * hd + d;
-      const float f = kept ? factors[z] : expf(part_ml[(base + z) * 2] - mx);
+      float f;
+      if constexpr (KEPT) f = factors[z];
+      else f = expf(part_ml[(base + z) * 2] - mx);
       if constexpr (VEC == 4) {
         const float4 o = *reinterpret_cast<const float4*>(from);
         acc[0] = fmaf(o.x, f, acc[0]); acc[1] = fmaf(o.y, f, acc[1]);
         acc[2] = fmaf(o.z, f, acc[2]); acc[3] = fmaf(o.w, f, acc[3]);
+      } else if constexpr (VEC == 2) {
+        const float2 o = *reinterpret_cast<const float2*>(from);
+        acc[0] = fmaf(o.x, f, acc[0]); acc[1] = fmaf(o.y, f, acc[1]);
       } else {
         acc[0] = fmaf(*from, f, acc[0]);
       }
@@ -287,18 +312,30 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
   }
 }
 
+// Two elements a thread where a block is then one task a thread (hd up to 256) and all blocks together are at most 512 threads
+// an SM; beyond, their larger number costs more than their loads gain (64 rows of 32 heads of 64: 1.06 to 1.27 times four's time;
+// 8 rows 0.81 to 0.96 times).
 template <typename T>
-static void launch_merge(const float* part_o, const float* part_ml, const int* positions, void* out, int M, int nh, int hd,
-                         int window, int chunk, int num_chunks, const int* row_list, int keep, const void* gate,
-                         long long gate_ld, cudaStream_t stream) {
-  const int threads = hd <= 32 ? 32 : (hd <= 512 ? (hd + 31) & ~31 : 512);
-  const size_t smem = (size_t)(MERGE_ZG * hd + (num_chunks <= MERGE_MAX_FACTORS ? num_chunks : 0)) * sizeof(float);
+static int launch_merge(const float* part_o, const float* part_ml, const int* positions, void* out, int M, int nh, int hd,
+                        int window, int chunk, int num_chunks, const int* row_list, int keep, const void* gate,
+                        long long gate_ld, cudaStream_t stream) {
+  int sms = 0;
+  const int rc = snk_device_sms(&sms);
+  if (rc) return rc;
+  const bool kept = num_chunks <= MERGE_MAX_FACTORS;
+  const bool two = kept && hd % 2 == 0 && (uintptr_t)part_o % 8 == 0 && hd <= 256 && 2ll * hd * M * nh <= 512ll * sms;
+  const bool four = hd % 4 == 0 && (uintptr_t)part_o % 16 == 0;
+  const int tasks = two ? 2 * hd : hd, threads = tasks < 512 ? (tasks + 31) & ~31 : 512;
+  const size_t smem = (size_t)(MERGE_ZG * hd + (kept ? num_chunks : 0)) * sizeof(float);
   auto launch = [&](auto kernel) {
     snk_launch(kernel, dim3(M, nh), dim3(threads), smem, stream, part_o, part_ml, positions, static_cast<T*>(out), nh, hd,
                window, chunk, num_chunks, row_list, keep, static_cast<const T*>(gate), gate_ld);
   };
-  if (hd % 4 == 0 && (uintptr_t)part_o % 16 == 0) launch(attention_merge_kernel<T, 4>);
-  else launch(attention_merge_kernel<T, 1>);
+  if (two) launch(attention_merge_kernel<T, 2, true>);
+  else if (kept) launch(four ? attention_merge_kernel<T, 4, true> : attention_merge_kernel<T, 1, true>);
+  else launch(four ? attention_merge_kernel<T, 4, false> : attention_merge_kernel<T, 1, false>);
+  SNK_LAUNCH_CHECK();
+  return 0;
 }
 
 // Bytes of scratch the launch below needs for `num_chunks` > 1 (0 for one chunk).
@@ -348,9 +385,8 @@ SNK_API int snk_paged_attention_rows(const void* q, const void* pool, const int*
 #undef ATT_LAUNCH
   SNK_LAUNCH_CHECK();
   if (num_chunks > 1) {
-    SNK_DISPATCH(dtype, launch_merge<T>(part_o, part_ml, positions, out, M, nh, hd, window, chunk, num_chunks,
-                                         row_list, 0, nullptr, 0LL, stream));
-    SNK_LAUNCH_CHECK();
+    SNK_DISPATCH(dtype, return launch_merge<T>(part_o, part_ml, positions, out, M, nh, hd, window, chunk, num_chunks,
+                                                row_list, 0, nullptr, 0LL, stream));
   }
   return 0;
 }
@@ -363,9 +399,8 @@ SNK_API int snk_attention_merge(const void* scratch, const int* positions, void*
   if (M <= 0 || num_chunks <= 1) return 0;
   const float* part_o = static_cast<const float*>(scratch);
   const float* part_ml = part_o + (size_t)M * nh * num_chunks * hd;
-  SNK_DISPATCH(dtype, launch_merge<T>(part_o, part_ml, positions, out, M, nh, hd, window, chunk, num_chunks,
-                                       row_list, 0, nullptr, 0LL, stream));
-  SNK_LAUNCH_CHECK();
+  SNK_DISPATCH(dtype, return launch_merge<T>(part_o, part_ml, positions, out, M, nh, hd, window, chunk, num_chunks,
+                                              row_list, 0, nullptr, 0LL, stream));
   return 0;
 }
 
@@ -378,9 +413,8 @@ SNK_API int snk_attention_merge_gated(const void* scratch, const int* positions,
   if (M <= 0 || num_chunks <= 1) return 0;
   const float* part_o = static_cast<const float*>(scratch);
   const float* part_ml = part_o + (size_t)M * nh * num_chunks * hd;
-  SNK_DISPATCH(dtype, launch_merge<T>(part_o, part_ml, positions, out, M, nh, hd, window, chunk, num_chunks,
-                                       row_list, keep, gate, gate_ld, stream));
-  SNK_LAUNCH_CHECK();
+  SNK_DISPATCH(dtype, return launch_merge<T>(part_o, part_ml, positions, out, M, nh, hd, window, chunk, num_chunks,
+                                              row_list, keep, gate, gate_ld, stream));
   return 0;
 }
 

@@ -1130,3 +1130,38 @@ def test_norm_route_sort_in_one_launch(K, dtype, M, H, E, k, bias, norm_topk, sc
     tk = g((1,), torch.int32, fill=0)
     K.norm_route_sort(res, torch.randn(M, H, device="cuda"), gamma, eps, dtype, wr, b, k, norm_topk, scaling, tk)
     g.check("norm_route_sort")
+
+
+# chunks: one run each, past a warp's first four rounds (128), past what is kept of their factors (4,096)
+@pytest.mark.parametrize("chunks", [2, 33, 129, 4096, 4097])
+@pytest.mark.parametrize("nh,hd", [(3, 64), (2, 50), (3, 33), (1, 260), (2, 512)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_attention_merge(K, dtype, nh, hd, chunks):
+    """Partial results of rows of all lengths against their sum in double precision; a row alone (a few elements a thread)
+    and the same row among many (more of them) come to the same bits."""
+    gen = torch.Generator(device="cuda").manual_seed(43)
+    M, chunk = (9 if chunks > 1000 else 700), 64
+    part = torch.randn(M * nh * chunks * (hd + 2), device="cuda", generator=gen)
+    o, ml = part[:M * nh * chunks * hd].view(M, nh, chunks, hd), part[M * nh * chunks * hd:].view(M, nh, chunks, 2)
+    ml[..., 1].abs_().add_(0.5)
+    lengths = [1 + (m * 131 + chunks - 1) % chunks for m in range(M)]              # chunks of a row; row 0 has all
+    positions = i32([n * chunk - 1 - m % chunk for m, n in enumerate(lengths)])
+
+    def merge(rows):
+        scratch = torch.cat((o[rows].reshape(-1), ml[rows].reshape(-1)))
+        at, out = positions[rows].contiguous(), torch.full((len(rows), nh * hd), float("nan"), dtype=dtype, device="cuda")
+        K.check(K.fn("snk_attention_merge")(scratch.data_ptr(), at.data_ptr(), out.data_ptr(), len(rows), nh, hd, 0, chunk,
+                                            chunks, K.code_of(dtype), 0, K._stream()), "attention_merge")
+        return out.view(len(rows), nh, hd)
+
+    out = merge(list(range(M)))
+    there = (torch.arange(chunks, device="cuda")[None, :] < i32(lengths)[:, None])[:, None, :, None]
+    weight = torch.where(there, (ml[..., :1].double() - ml[..., :1].double().amax(2, keepdim=True)).exp(), 0.0)
+    total = (weight * ml[..., 1:].double()).sum(2)
+    want = (weight * o.double()).sum(2) / total
+    # a rounding of 2^-24 of the partial sum at every chunk's addition, of its factor (expf: 2 ulp) and of the division
+    slack = 2.0 ** -24 * (chunks + 8) * (weight * o.double().abs()).sum(2) / total + 2.0 ** -23 * want.abs()
+    slack += 2.0 ** -24 * (chunks / 32 + 8) * want.abs() + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)
+    assert bool(((out.double() - want).abs() <= slack).all())
+    for m in (0, 1, M - 1):
+        assert torch.equal(merge([m])[0], out[m])
