@@ -240,7 +240,8 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
   __shared__ float s_mx, s_inv;
   const int m = row_list ? row_list[blockIdx.x] : blockIdx.x, head = blockIdx.y;
   const int pos = positions[m];
-  const int n = row_chunks(pos, window, keep, chunk);      // chunks this row really has
+  // chunks this row really has; a position past the launch's chunks takes all of them (there are factors for no more)
+  const int n = min(row_chunks(pos, window, keep, chunk), num_chunks);
   const size_t base = ((size_t)blockIdx.x * nh + head) * num_chunks;
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;

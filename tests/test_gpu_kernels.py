@@ -1165,3 +1165,17 @@ def test_attention_merge(K, dtype, nh, hd, chunks):
     assert bool(((out.double() - want).abs() <= slack).all())
     for m in (0, 1, M - 1):
         assert torch.equal(merge([m])[0], out[m])
+
+
+def test_attention_merge_of_a_position_past_its_chunks(K):
+    """takes the launch's chunks and nothing beyond them"""
+    nh, hd, chunks, chunk = 2, 64, 5, 64
+    gen = torch.Generator(device="cuda").manual_seed(44)
+    part = torch.randn(nh * chunks * (hd + 2), device="cuda", generator=gen)
+    part[nh * chunks * hd:].abs_().add_(0.5)
+    out = []
+    for position in (chunks * chunk - 1, chunks * chunk, 1000 * chunk):
+        out.append(torch.zeros(1, nh * hd, device="cuda"))
+        K.check(K.fn("snk_attention_merge")(part.data_ptr(), i32([position]).data_ptr(), out[-1].data_ptr(), 1, nh, hd, 0, chunk,
+                                            chunks, K.code_of(torch.float32), 0, K._stream()), "attention_merge")
+    assert torch.equal(out[1], out[0]) and torch.equal(out[2], out[0])
