@@ -356,7 +356,16 @@ static int launch_few(const SimtArgs& p) {
   return 0;
 }
 
-#define FR_MAX_ROWS 16             // up to here (grouped: up to 4 rows a group on average) W's read is the bound
+// Up to here W's read is the bound.  Measured, in replayed chains over rotating weights, this kernel / the tiles, us: 2,048 x 2,048 1 row
+// 8.6 / 95, 4 rows 10.0 / 95, 8 rows 12.6 / 95, 16 rows 21.5 / 95; 6,144 x 2,048 14 / 87, 19 / 88, 22 / 89, 45 / 88; 16,384 x 2,048
+// 27 / 94, 35 / 95, 50 / 94, 91 / 95; 65,536 x 2,048 96 / 272, 111 / 274, 165 / 275, 316 / 279 (there the tiles are ahead from 10 rows on);
+// 20 rows 58 / 89 at 6,144 x 2,048 and 118 / 97 at 16,384 x 2,048.
+// Grouped, up to 4 rows a group on average (32 groups, 3,584 x 2,048, each token in 4 of them at random): 4 tokens 80 / 240 us, 8 128 / 313,
+// 16 174 / 421, 32 272 / 461; 128 groups of 768 x 512: 16 tokens 25 / 58, 100 74 / 102.  A group far above the average is walked in
+// passes that read W again: all 32 tokens in the same 4 of 32 groups 195 / 174 us, 100 tokens in the same 4 of 128 groups 69 / 36,
+// all 400 rows in one of 128 groups 250 / 54 (such a group would need tiles of its own: a second launch whose blocks find no such
+// group in every ordinary step).
+#define FR_MAX_ROWS 16
 
 // The tile with the least work on the busiest SM: rounds of tiles over the SMs times the tile's area, over the share of
 // the FMA rate that its shared-memory reads leave.  The shares are those at 4,096 x 16,384 x 2,048 (128 x 128 5.16 ms, 64 x 128 5.28,
@@ -416,7 +425,9 @@ SNK_API int snk_gemm_simt(const void* A, const void* W, void* C, int M, int N, i
                   (((size_t)K * esz) % 8 == 0);
   const SimtArgs p{A, W, C, M, N, K, a_rows, a_div <= 0 ? 1 : a_div, offsets, groups, rows, vec, w_ahead, stream};
   if (dtype == SNK_F32 && vec && (offsets ? (long long)M <= 4ll * groups : M <= FR_MAX_ROWS) && (!offsets || groups <= 65535)) {
-    // rows of a pass: those of the product, or about twice a group's mean (fuller groups take more passes)
+    // Rows of a pass: those of the product, or about twice a group's mean (fuller groups take more passes).  32 groups of 3,584 x 2,048,
+    // passes of 2 / 4 / 8 / 16 rows: 1 row a group on average 128 / 128 / 186 / 364 us, 2 rows 194 / 174 / 252 / 498, 4 rows 325 / 244 /
+    // 272 / 539; plain 2,048 x 2,048 of 4 rows 15.6 / 10.0 / 12.6 / 21.5, of 8 rows 28.8 / 18.2 / 12.6 / 21.8.
     const int pass = offsets ? 2 * ((M + groups - 1) / groups) : M;
     if (pass <= 2) return launch_few<1, 1>(p);
     if (pass <= 4) return launch_few<2, 1>(p);

@@ -1175,7 +1175,8 @@ def test_attention_merge_of_a_position_past_its_chunks(K):
     part[nh * chunks * hd:].abs_().add_(0.5)
     out = []
     for position in (chunks * chunk - 1, chunks * chunk, 1000 * chunk):
+        at = i32([position])
         out.append(torch.zeros(1, nh * hd, device="cuda"))
-        K.check(K.fn("snk_attention_merge")(part.data_ptr(), i32([position]).data_ptr(), out[-1].data_ptr(), 1, nh, hd, 0, chunk,
+        K.check(K.fn("snk_attention_merge")(part.data_ptr(), at.data_ptr(), out[-1].data_ptr(), 1, nh, hd, 0, chunk,
                                             chunks, K.code_of(torch.float32), 0, K._stream()), "attention_merge")
     assert torch.equal(out[1], out[0]) and torch.equal(out[2], out[0])
