@@ -14,8 +14,35 @@ The class knows nothing of CUDA: what captures, what measures memory and what an
 are given to it, so its decisions are tested on the CPU."""
 from __future__ import annotations
 
+import contextlib
+import gc
+import threading
 from collections import OrderedDict
 from typing import Callable
+
+_collector = threading.Lock()
+_captures_now = 0
+_was_enabled = False
+
+
+@contextlib.contextmanager
+def collector_off():
+    """Python's cyclic garbage collector off while a step is captured, in whatever threads capture.  An engine that was
+    dropped is a cycle: collected in the middle of a capture it destroys its own captures and gives memory back, neither
+    of which CUDA takes while a stream captures, and the step fails."""
+    global _captures_now, _was_enabled
+    with _collector:
+        if _captures_now == 0:
+            _was_enabled = gc.isenabled()
+            gc.disable()
+        _captures_now += 1
+    try:
+        yield
+    finally:
+        with _collector:
+            _captures_now -= 1
+            if _captures_now == 0 and _was_enabled:
+                gc.enable()
 
 
 class GraphCache:
@@ -51,7 +78,8 @@ class GraphCache:
             self.refused += 1
             return None
         try:
-            made = capture()
+            with collector_off():
+                made = capture()
         except self._oom:
             # what the failed capture took is given back; the captures that exist stay usable
             self.full = True

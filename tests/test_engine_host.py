@@ -248,3 +248,46 @@ def test_graph_cache_survives_out_of_memory_inside_a_capture():
     assert g.get(3, capture(mem, 10, log, 3)) is None                 # nothing more is captured
     zero = GraphCache(max_graphs=0, ceiling_bytes=None, in_use=mem)
     assert zero.get(1, capture(mem, 10, log, 1)) is None
+
+
+def test_no_garbage_is_collected_while_a_step_is_captured():
+    """Cycles that became garbage before a capture stay until after it, also where captures of two threads overlap and
+    where one fails; a collector that was off stays off."""
+    import gc
+    from snowllm_b200.engine.graphs import collector_off
+    g = GraphCache(max_graphs=8, ceiling_bytes=None, in_use=lambda: 0)
+    gone = []
+
+    class Cycle:
+        def __init__(self):
+            self.me = self
+
+        def __del__(self):
+            gone.append(1)
+
+    def capture():
+        Cycle()
+        for _ in range(3 * gc.get_threshold()[0]):
+            keep.append([])
+        assert not gone and not gc.isenabled()
+        with collector_off():
+            pass
+        assert not gc.isenabled()
+        return "captured"
+
+    def fails():
+        raise MemoryError
+
+    keep = []
+    assert gc.isenabled()
+    assert g.get("a", capture) == "captured" and gc.isenabled()
+    assert g.get("b", fails) is None and gc.isenabled()
+    gc.collect()
+    assert gone
+    gc.disable()
+    try:
+        with collector_off():
+            assert not gc.isenabled()
+        assert not gc.isenabled()
+    finally:
+        gc.enable()

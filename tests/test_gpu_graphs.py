@@ -62,3 +62,37 @@ def test_decode_tail_through_captured_steps_matches_the_plain_implementation(mod
     for a, b in zip(captured, plainly):
         assert float(((a - b).norm(dim=-1) / b.norm(dim=-1)).max()) < 1e-5
     check_against_plain(d, "bfloat16", reqs, steps, captured, routes)
+
+
+def test_an_engine_dropped_before_a_capture_does_not_fail_it(model_dirs, monkeypatch):
+    """A dropped engine is a cycle that holds captures and memory.  Let the collector run for the first time while the next
+    engine's step is captured: no step fails, and the tokens are the same."""
+    import gc
+    import snowllm_b200
+    from snowllm_b200.engine import Engine, SamplingParams
+    model = snowllm_b200.load(model_dirs("tiny_e", "bfloat16"), "bfloat16")
+    prompt = random_prompt(ALL["tiny_e"]["vocab_size"], 40, 7)
+    forward, threshold, eager = model.forward, gc.get_threshold(), True
+
+    def forward_among_garbage(ctx, cache):
+        if torch.cuda.is_current_stream_capturing() and not eager:
+            gc.set_threshold(1, 1, 1)
+            [[] for _ in range(1000)]                  # containers enough for a collection of every generation
+            gc.set_threshold(10 ** 9)
+        return forward(ctx, cache)
+
+    monkeypatch.setattr(model, "forward", forward_among_garbage)
+    outs = []
+    gc.set_threshold(10 ** 9)
+    try:
+        for eager in (True, False, False):
+            engine = Engine(model, max_num_seqs=2, max_model_len=256)
+            engine.itself = engine
+            outs.append(engine.generate([prompt], SamplingParams(temperature=0, max_new_tokens=20))[0])
+            stats = engine.stats()
+            assert stats.step_errors == 0 and stats.graphs["captures"] > 0, engine.last_error
+            del engine
+    finally:
+        gc.set_threshold(*threshold)
+        gc.collect()
+    assert len(outs[0]) == 20 and outs[1] == outs[0] and outs[2] == outs[0]
