@@ -56,6 +56,7 @@ def statuses_are_clear():
     from snowllm_b200.ops import kernels
     assert kernels.gemm_tc_status() == 0 and kernels.gemm_tc2_status()[0] == 0
     assert kernels.attention_tc_status() == 0 and kernels.attention_decode_status() == 0
+    assert kernels.gemm_skinny_status() == 0
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])

@@ -151,3 +151,42 @@ def test_w_may_come_from_the_kernel_in_front(M, dtype):
         graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+# one row tile and two; one sum a warp and four (K of 2,048 on, up to 2,368 rows of W); one to three rounds of strips;
+# boxes that end in the middle, an odd number of them
+@pytest.mark.parametrize("M,N,K", [(1, 16, 64), (3, 208, 576), (13, 1008, 576), (16, 200, 1088), (5, 2368, 2560), (12, 1776, 4096),
+                                   (16, 2352, 2112), (9, 2384, 2048), (8, 4112, 1600), (16, 4752, 2112)])
+def test_weights_read_ahead_and_stores_with_a_gate(M, N, K):
+    """The streaming product, W read ahead or not, to float, to bfloat16, with a gate and with the square of relu at its
+    store, inside an output that is full of NaN: the same bits as the kernel without a ring, nothing beside them."""
+    from snowllm_b200.ops import kernels
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert kernels.fn("snk_gemm_skinny_streams")(M, N, K, sms)
+    a, w = operands(M, K, seed=20), operands(N, K, seed=21)
+    rows = torch.arange(M, dtype=torch.int32, device="cuda")
+    stores = [dict(out_dtype=torch.float32), {}, dict(act=kernels.UNARY_CODES["relu2"])]
+    stores += [dict(swiglu=code) for code in (1, 2, 3) if N % 16 == 0]
+    for store in stores:
+        want = kernels.gemm_skinny(a, w, a_rows=rows, **store)
+        for ahead in (False, True):
+            room = torch.full((want.numel() + 128,), float("nan"), dtype=want.dtype, device="cuda")
+            out = room[64:-64].view(want.shape)
+            kernels.gemm_skinny(a, w, out=out, w_ahead=ahead, **store)
+            assert torch.equal(out, want)
+            assert bool(room[:64].isnan().all()) and bool(room[-64:].isnan().all())
+    assert kernels.gemm_skinny_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 64, 1024), (64, 2048, 2048), (130, 520, 200), (200, 6144, 576), (2050, 264, 1088)])
+def test_tcgen05_product_with_its_weight_read_ahead(M, N, K):
+    """Split along K and whole, one round of tiles and more, more and fewer k-blocks than the ring has stages."""
+    from snowllm_b200.ops import kernels
+    a, w = operands(M, K, seed=22), operands(N, K, seed=23)
+    for store in (dict(out_dtype=torch.float32), {}, dict(swiglu=1)):
+        if "swiglu" in store and N % 16:
+            continue
+        want = kernels.gemm_tc(a, w, **store)
+        for _ in range(3):
+            assert torch.equal(kernels.gemm_tc(a, w, w_ahead=True, **store), want)
+    assert kernels.gemm_tc_status() == 0
