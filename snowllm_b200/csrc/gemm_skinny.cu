@@ -1,7 +1,8 @@
 // C[M,N] = A[M,K] . W[N,K]^T in bfloat16 for few rows (decode: M up to 64), bound by the read of W.
 //
-// Weights stream from HBM exactly once, straight into tensor-core fragments; nothing of W passes
-// through shared memory.  A block owns 16 rows of W (16 output features).  Its 8 warps split K in
+// Two kernels, which come to the same bits.  The first one's weights stream from HBM exactly once, straight into tensor-core
+// fragments; the second one (further down: plain products of up to 16 rows, where stream_pays says so) brings W through a
+// ring in shared memory.  A block of the first owns 16 rows of W (16 output features).  Its 8 warps split K in
 // interleaved 32-element blocks; a warp multiplies its 16x32 piece of W with up to 64 tokens by
 // mma.sync m16n8k16 (W as the 16-row operand, 8 tokens as the 8-column operand) and the 8 partial
 // sums meet in shared memory, added in warp order: no atomics, the same bits every run, and a
@@ -33,7 +34,8 @@
 #endif
 #ifndef SK_PREFETCH_LINES
 #define SK_PREFETCH_LINES 4    // rounds of 16 lines of 128 bytes per row that a block asks L2 for ahead of its wait
-                               // (measured in the decode step, 0 / 2 / 4 rounds: 1.497 / 1.482 / 1.476 ms at batch 1)
+                               // (measured in the decode step of one request while all its plain products ran here, 0 / 2 / 4
+                               // rounds: 1.497 / 1.482 / 1.476 ms; now its dense gate|up and its head do)
 #endif
 
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {
@@ -265,11 +267,11 @@ static int skinny_split(int N, int K, const int* offsets) {
 
 // ---------------------------------------------------------------------------------------------
 // Plain products of up to 16 rows: the same, with W streamed through shared memory.  What bounds them is the read of W,
-// and most of what a small one takes beside it is the way from the end of the kernel before to the first bytes of W.  W
-// is a constant (the caller says so: w_ahead), so here one block per SM keeps a ring of stages (16 rows x 512 columns each, one TMA box, filled by a
-// ninth warp) that starts to fill while the kernel before still runs, and goes on across the block's strips of 16 rows;
-// eight warps multiply out of it.  Ring and sums take less than half of an SM's shared memory, so that the next product
-// can start beside this one.
+// and most of what a small one takes beside it is the way from the end of the kernel before to the first bytes of W.  Where
+// W is a weight (the caller says so: w_ahead) one block per SM keeps a ring of stages (16 rows x 512 columns each, one TMA
+// box, filled by a ninth warp) that starts to fill while the kernel before still runs, and goes on across the block's
+// strips of 16 rows; eight warps multiply out of it.  Ring and sums take less than half of an SM's shared memory, so that
+// the next product can start beside this one.
 //
 // The numbers are the same bits as above: warp w takes the 32-column runs w, w + 8, .. of a strip in order, the same MMAs,
 // the same order of the warps' sums (SPLIT 4: four sums a warp, as the cluster's blocks held them).  A box brings 64
@@ -277,9 +279,9 @@ static int skinny_split(int N, int K, const int* offsets) {
 // holds row st_row(g), an order in which the eight lanes that read shared memory together find their 16 bytes in
 // different banks.
 //
-// Measured, 1 row, in a replayed chain (the kernel above): 2,048 x 2,048 5.3 -> 3.6 us, 6,144 x 2,048 8.5 -> 7.2, 16,384 x
-// 2,048 17.1 -> 14.5; in the decode steps, where the ring fills ahead, 4.1 -> 2.7 us from the end of the kernel before to
-// the end of 2,048 x 2,048 and 7.0 -> 5.6 of 6,144 x 2,048.
+// Measured, 1 row, in a replayed chain of the product alone (the kernel above): 2,048 x 2,048 5.3 -> 3.0 us, 6,144 x 2,048 8.5 ->
+// 7.0, 4,096 x 4,096 14.0 -> 8.7; in the decode steps, where the ring fills ahead, 4.1 -> 2.7 us from the end of the kernel
+// before to the end of 2,048 x 2,048 and 7.0 -> 5.6 of 6,144 x 2,048.  Sizes at which it loses: see stream_pays.
 // Grouped products stay above: a group's strips are few and each has other rows of A to fetch, so the eight warps of the
 // one block cannot hide that as eight blocks an SM do (20 of 32 experts with a row each: 72 us here, 54 above).
 #define ST_RUNS 16                              // runs of 32 columns of a stage (8 blocks of 64 columns)

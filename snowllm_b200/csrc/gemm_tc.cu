@@ -164,8 +164,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const uint32_t tmem_acc = sh->tmem_base;
   volatile int* aborted = &sh->aborted;
   // w_ahead (plain products): W was there before the kernel in front of this launch began, so its tiles of the first
-  // ring of k-blocks are on their way before the wait, and only A's follow after it
-  // (64 rows, 6,144 x 2,048 in the decode step: 8.2 -> 6.7 us from the end of the norm to the end of the product).
+  // ring of k-blocks are on their way before the wait, and only A's follow after it.  Replayed chains of a norm and the
+  // product, without / with: 17 rows 2,048 x 1,792 11.4 / 10.4 us, 64 rows 2,048 x 2,048 11.6 / 11.5, gate|up and down of 1,024 and 2,816
+  // 23.6 / 22.4, but 6,144 x 2,048 14.1 / 14.5; over 150 sizes of 17 to 1,024 rows 1.2 % less, 9 % at best, 4 % more at worst;
+  // the 64-request decode step of the 8B-A1B sizes 4,890 / 4,868 us.
   int early = 0;
   if (w_ahead && !offsets && threadIdx.x == 0 && *const_cast<volatile int*>(&g_tc_lose_loads) == 0) {
     const int total = row_tiles_bound * ((N + BN - 1) / BN), k_per = (k_tiles + splits - 1) / splits;

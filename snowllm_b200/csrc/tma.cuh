@@ -1,9 +1,9 @@
 // Tensor-map (TMA) loads and mbarriers for the sm_100a kernels: the device helpers, and on the host
-// the encoding of 2-D bfloat16 tensor maps through the driver entry point (no link against the driver
-// library), cached by what they describe.
+// the encoding of bfloat16 tensor maps of a matrix, 2-D or as runs of 64 columns (3-D), through the driver entry point (no
+// link against the driver library), cached by what they describe.
 //
 // Alignment: a tiled TMA copy starts on a 16-byte boundary, so the innermost coordinate is always a
-// multiple of 8 elements here; the other coordinate is free.  Tiles written with the 128-byte swizzle lie
+// multiple of 8 elements here; the other coordinates are free.  Tiles written with the 128-byte swizzle lie
 // on 1024-byte boundaries of shared memory.
 #pragma once
 #include <cuda.h>
@@ -64,8 +64,8 @@ __device__ __forceinline__ void drain_after_abort() {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Tensor maps: 2-D, bfloat16, rows of `k` elements (row pitch k * 2 bytes), box box_cols x box_rows,
-// 128-byte swizzle, zero fill outside.  Cached by (pointer, rows, k, box).
+// Tensor maps: bfloat16, rows of `k` elements (row pitch k * 2 bytes), box box_cols x box_rows (or rows by runs of 64
+// columns, see tensor_map), 128-byte swizzle, zero fill outside.  Cached by (pointer, rows, k, box): a description, no data.
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

@@ -2,7 +2,8 @@
 
 float32: the CUDA-core kernels of csrc/gemm.cu (true 32-bit, sums in k order).
 bfloat16, up to 16 rows (decode; grouped: up to 4 rows per group on average): csrc/gemm_skinny.cu, which
-streams W once into mma.sync fragments (plain products through shared memory, ahead of the kernel in front).
+streams W once into mma.sync fragments (plain products, where that is faster, through shared memory; a weight from ahead
+of the wait for the kernel in front).
 bfloat16, more rows (prefill): csrc/gemm_tc.cu, 128 x 256 tiles on the tcgen05 tensor cores with TMA
 loads and the accumulator in tensor memory; from 4,096 rows on, and for all grouped products, csrc/gemm_tc2.cu
 on pairs of SMs (grouped: W is the 256-row operand and a group's rows the N side, in steps of 16).
