@@ -988,6 +988,8 @@ def gemm_simt(a, w, out_dtype=None, out=None, a_rows=None, a_div=1, offsets=None
     M = rows_out if rows_out is not None else a.shape[0]
     if a_rows is not None:
         _chk(a_rows, "gemm row gather", torch.int32)
+        if a_rows.numel() < M:
+            raise KernelError(f"gemm row gather: {a_rows.numel()} rows for {M} of the output")
     out_dtype = out_dtype or dtype
     if out is None:
         out = torch.empty(M, N, dtype=out_dtype, device=a.device)
@@ -1028,6 +1030,8 @@ def gemm_skinny(a, w, out_dtype=None, out=None, a_rows=None, a_div=1, offsets=No
     M = rows_out if rows_out is not None else a.shape[0]
     if a_rows is not None:
         _chk(a_rows, "gemm row gather", torch.int32)
+        if a_rows.numel() < M:
+            raise KernelError(f"gemm row gather: {a_rows.numel()} rows for {M} of the output")
     out_dtype = out_dtype or torch.bfloat16
     cols = N // 2 if swiglu else N          # swiglu: w rows are gate/up interleaved by 8, out = silu(gate) * up
     if out is None:

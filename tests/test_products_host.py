@@ -3,6 +3,7 @@ The kernels' wrappers are replaced by ones that write down what they are told.""
 import pytest
 import torch
 
+from snowllm_b200.errors import KernelError
 from snowllm_b200.ops import kernels, linear, linear_glu, linear_swiglu
 
 
@@ -87,3 +88,13 @@ def test_which_few_rows_products_stream_w_through_shared_memory():
         for M in (1, 16):
             assert streams(M, N, K, 148) == want, (N, K)
         assert streams(17, N, K, 148) == 0
+
+
+@pytest.mark.parametrize("product", ["gemm_simt", "gemm_skinny"])
+def test_a_row_gather_that_is_too_short_is_refused(monkeypatch, product):
+    monkeypatch.setattr(kernels, "_chk", lambda *a, **kw: None)
+    monkeypatch.setattr(kernels, "fn", lambda name: pytest.fail("launched"))
+    x, w = torch.zeros(9, 64, dtype=torch.bfloat16), torch.zeros(32, 64, dtype=torch.bfloat16)
+    for rows_out, listed in ((None, 8), (12, 11)):
+        with pytest.raises(KernelError, match="row gather"):
+            getattr(kernels, product)(x, w, a_rows=torch.zeros(listed, dtype=torch.int32), rows_out=rows_out)
