@@ -542,7 +542,16 @@ template <int MT>
 static int launch_skinny(const void* A, const void* W, void* C, int M, int N, int K, const int* a_rows,
                          int a_div, const int* offsets, int groups, int out_f32, int swiglu, int split,
                          int w_ahead, cudaStream_t stream) {
-  dim3 grid((N + SK_ROWS - 1) / SK_ROWS, offsets ? (groups < M ? groups : M) : 1, split);
+  // Fewer rows than groups: a block per row and strip, which looks its group up, unless the blocks of all groups are on the SMs
+  // at once (8 to each) and the idle ones cost nothing (8 groups of 512 x 256, one token with two of them: 3.0 / 2.8 us).
+  const int strips = (N + SK_ROWS - 1) / SK_ROWS;
+  int sms = 0, per_group = groups;
+  if (offsets && groups > M) {
+    const int rc = snk_device_sms(&sms);
+    if (rc) return rc;
+    if ((long long)strips * groups > 8ll * sms) per_group = M;
+  }
+  dim3 grid(strips, offsets ? per_group : 1, split);
   const dim3 block(SK_WARPS * 32);
   const bf16 *a = static_cast<const bf16*>(A), *w = static_cast<const bf16*>(W);
   const int unary = swiglu == SNK_ACT_RELU2 ? swiglu : 0;

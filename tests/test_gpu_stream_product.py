@@ -190,3 +190,22 @@ def test_tcgen05_product_with_its_weight_read_ahead(M, N, K):
         for _ in range(3):
             assert torch.equal(kernels.gemm_tc(a, w, w_ahead=True, **store), want)
     assert kernels.gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("counts", [[0] * 40 + [2] + [0] * 30 + [33], [1] * 5 + [0] * 90, [0] * 99 + [7], [3, 0, 9] + [0] * 120])
+def test_grouped_blocks_that_look_their_group_up(counts):
+    """Fewer rows than groups and more blocks than the SMs hold at once: against each group's rows as a product of their own."""
+    from snowllm_b200.ops import kernels
+    G, M, N, K = len(counts), sum(counts), 1024, 256
+    assert G > M and N // 16 * G > 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    x, w = operands(M, K, seed=24), operands(G, N, K, seed=25)
+    offsets = torch.tensor([0] + counts).cumsum(0).to(torch.int32).cuda()
+    for hint in (8, 16):
+        out = kernels.gemm_skinny(x, w, out_dtype=torch.float32, offsets=offsets, rows_out=M, rows_hint=hint)
+        lo = 0
+        for e, n in enumerate(counts):
+            if n:
+                rows = torch.arange(n, dtype=torch.int32, device="cuda")
+                assert torch.equal(out[lo:lo + n], kernels.gemm_skinny(x[lo:lo + n].contiguous(), w[e].contiguous(),
+                                                                       out_dtype=torch.float32, rows_hint=hint, a_rows=rows))
+            lo += n
