@@ -672,10 +672,12 @@ def test_gemm_tc2_grouped_rows_on_the_n_side(K, N, K_):
 
 
 @pytest.mark.parametrize("counts", [[64, 3, 0, 49], [65, 1, 64], [128, 17, 0, 96, 112], [129, 64, 5], [256] + [16] * 40, [257],
+                                    [(11 * e) % 37 * 4 for e in range(32)], [(11 * e) % 37 * 4 for e in range(33)],
                                     [(7 * e) % 23 * (e % 5 != 0) for e in range(200)], [(e % 13) * (e % 29) for e in range(256)]])
 def test_gemm_tc2_grouped_rings_and_plans(K, counts):
     """The grouped pair product where its ring changes (row tiles of up to 64, up to 128 and more rows: 10, 8 and 6 stages),
-    with more than two rounds of the ring (26 k-blocks), and its plan of many groups, longest row tiles first."""
+    with more than two rounds of the ring (26 k-blocks), and both plans: up to 32 groups, longest row tiles first, and
+    more, in their own order."""
     G, M, N, K_ = len(counts), sum(counts), 264, 26 * 64
     gen = torch.Generator(device="cuda").manual_seed(41)
     a = torch.randn(M, K_, device="cuda", generator=gen).to(torch.bfloat16)
