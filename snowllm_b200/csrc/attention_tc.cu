@@ -110,6 +110,11 @@ __device__ __noinline__ bool at_wait_long(uint64_t* bar, uint32_t parity, volati
 __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile int* aborted, int code) {
   return mbar_try_wait(bar, parity) || at_wait_long(bar, parity, aborted, code);
 }
+// The same by all lanes of a warp, which come out together and with one answer (mbar_wait_warp of gemm_tc.cu): here two key tiles
+// apart were enough.
+__device__ __forceinline__ bool at_wait_warp(uint64_t* bar, uint32_t parity, volatile int* aborted, int code) {
+  return __all_sync(0xffffffffu, at_wait(bar, parity, aborted, code));
+}
 
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile(
@@ -274,8 +279,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const int ks = t % AT_KSTAGES;
         const int k0 = tile_k0(t);
         tile_pages(t, fp_k, np_k);
-        const bool free = at_wait(&sh->k_empty[ks], ((t / AT_KSTAGES) & 1) ^ 1, aborted, AT_ERR_KV_FREE);
-        if (!__all_sync(0xffffffffu, free)) break;         // a wait ran out: nothing more is issued
+        if (!at_wait_warp(&sh->k_empty[ks], ((t / AT_KSTAGES) & 1) ^ 1, aborted, AT_ERR_KV_FREE)) break;   // nothing more is issued
         if (lane == 0) mbar_expect_tx(&sh->k_full[ks], (uint32_t)np_k * page_size * 128u);
         __syncwarp();
         if (lane < np_k)
@@ -285,8 +289,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (t >= 1) {
         const int j = t - 1, vs = j % AT_VSTAGES;
         const int k0 = tile_k0(j);
-        const bool free = at_wait(&sh->v_empty[vs], ((j / AT_VSTAGES) & 1) ^ 1, aborted, AT_ERR_KV_FREE);
-        if (!__all_sync(0xffffffffu, free)) break;
+        if (!at_wait_warp(&sh->v_empty[vs], ((j / AT_VSTAGES) & 1) ^ 1, aborted, AT_ERR_KV_FREE)) break;
         if (lane == 0) mbar_expect_tx(&sh->v_full[vs], (uint32_t)np_v * page_size * 128u);
         __syncwarp();
         if (lane < np_v)
@@ -307,8 +310,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     int ks = 0, vs = 0;                                    // the slots of the next tile's keys and values,
     uint32_t k_lap = 0, v_lap = 0;                         // and the parities of the rings' rounds
     auto scores = [&](int j) {
-      if (!at_wait(&sh->k_full[ks], k_lap, aborted, AT_ERR_KV)) return false;
-      if (!at_wait(&sh->s_empty, (j & 1) ^ 1, aborted, AT_ERR_S_FREE)) return false;
+      if (!at_wait_warp(&sh->k_full[ks], k_lap, aborted, AT_ERR_KV)) return false;
+      if (!at_wait_warp(&sh->s_empty, (j & 1) ^ 1, aborted, AT_ERR_S_FREE)) return false;
       tc_fence_after();
       const uint32_t k_lo = k_ring + ks * (AT_KV_BYTES >> 4);
 #pragma unroll
@@ -322,10 +325,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
       return true;
     };
-    if (at_wait(&sh->q_ready, 0, aborted, AT_ERR_Q) && scores(0)) {
+    if (at_wait_warp(&sh->q_ready, 0, aborted, AT_ERR_Q) && scores(0)) {
       for (int j = 0; j < n_kt; ++j) {
         if (j + 1 < n_kt && !scores(j + 1)) break;
-        if (!at_wait(&sh->v_full[vs], v_lap, aborted, AT_ERR_KV) || !at_wait(&sh->p_full, j & 1, aborted, AT_ERR_P)) break;
+        if (!at_wait_warp(&sh->v_full[vs], v_lap, aborted, AT_ERR_KV) || !at_wait_warp(&sh->p_full, j & 1, aborted, AT_ERR_P)) break;
         tc_fence_after();
         const uint32_t v_lo = v_ring + vs * (AT_KV_BYTES >> 4);
 #pragma unroll
@@ -349,7 +352,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
     const int lo_last = window > 0 ? max(0, last_pos - window + 1) : 0;   // the last row's lowest key
     {                                                    // this row of q: shared memory -> tensor memory
-      at_wait(&sh->q_full, 0, aborted, AT_ERR_Q);
+      at_wait_warp(&sh->q_full, 0, aborted, AT_ERR_Q);
       uint32_t qr[32];
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -371,8 +374,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     for (int j = 0; j < n_kt; ++j) {
       const int st = j % AT_VSTAGES;
       const int k0 = tile_k0(j);
-      const bool there = at_wait(&sh->s_full, j & 1, aborted, AT_ERR_S);
-      if (!__all_sync(0xffffffffu, there)) break;          // the whole warp leaves together
+      if (!at_wait_warp(&sh->s_full, j & 1, aborted, AT_ERR_S)) break;
       tc_fence_after();
       uint32_t r[4][32];
 #pragma unroll
@@ -448,7 +450,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
       l = l * alpha + ((sc[0] + sc[1]) + (sc[2] + sc[3]));
       if (j > 0) {                                       // P of the tile before has been read, O holds the tiles before this one
-        at_wait(&sh->pv_done, (j - 1) & 1, aborted, AT_ERR_PV);
+        at_wait_warp(&sh->pv_done, (j - 1) & 1, aborted, AT_ERR_PV);
         tc_fence_after();
       }
       unsigned char* p_row = sm_p + row * 128;
@@ -461,7 +463,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
               make_uint4(r[c][4 * q8], r[c][4 * q8 + 1], r[c][4 * q8 + 2], r[c][4 * q8 + 3]);
         }
       if (k0 < key_lo || k0 + AT_BK - 1 > last_pos) {    // value rows no row sees: zero, whatever they held
-        at_wait(&sh->v_full[st], (j / AT_VSTAGES) & 1, aborted, AT_ERR_KV);
+        at_wait_warp(&sh->v_full[st], (j / AT_VSTAGES) & 1, aborted, AT_ERR_KV);
         const int kp = k0 + row;
         if ((kp < key_lo && kp >= keep) || kp > last_pos) {
           uint4* v_row = reinterpret_cast<uint4*>(sm_v + (size_t)st * AT_KV_BYTES + row * 128);
@@ -484,7 +486,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh->p_full);
     }
-    at_wait(&sh->pv_done, (n_kt - 1) & 1, aborted, AT_ERR_PV);
+    at_wait_warp(&sh->pv_done, (n_kt - 1) & 1, aborted, AT_ERR_PV);
     tc_fence_after();
     float inv = l > 0.f ? 1.f / l : 0.f;
     if (gate && row < rows) inv /= 1.f + expf(-__bfloat162float(gate[(size_t)(row0 + row) * gate_ld + head]));
@@ -505,6 +507,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     }
   }
   if (*aborted) drain_after_abort();
+  __syncwarp();                                          // (the deallocation wants the whole warp)
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

@@ -162,8 +162,10 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // Thread-block clusters: a barrier over all threads of the cluster's blocks, and the shared memory of
-// another block of the cluster (distributed shared memory) by the address the same variable has here.
+// another block of the cluster (distributed shared memory) by the address the same variable has here.  (The aligned form wants whole
+// warps: whatever branch a warp's lanes come out of, they meet first.)
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // The float at the same shared-memory address in block `rank` of this cluster.

@@ -62,6 +62,13 @@ __device__ __noinline__ bool mbar_wait_long(uint64_t* bar, uint32_t parity, vola
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* aborted, int code) {
   return mbar_try_wait(bar, parity) || mbar_wait_long(bar, parity, aborted, code);
 }
+// The same by all lanes of a warp, which come out together and with one answer.  Lanes that waited each for itself could fall
+// apart (nothing joins them again in a loop that is left by a failed wait): one that comes two phases late waits for a phase that
+// never comes, and the aligned instructions behind the loops want whole warps.  Measured, us, 8,192 x 6,144 x 2,048 each for
+// itself / so: XX.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* aborted, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, aborted, code));
+}
 
 #define TC_MAX_STAGES 6
 
@@ -230,12 +237,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (!t.valid) continue;
       const int kt_begin = (item / total) * k_per, kt_end = min(k_tiles, kt_begin + k_per);
       const int buf = local & 1;
-      if (!mbar_wait(&sh->acc_empty[buf], ((local >> 1) & 1) ^ 1, aborted, TC_ERR_WAIT_ACC_FREE)) break;
+      if (!mbar_wait_warp(&sh->acc_empty[buf], ((local >> 1) & 1) ^ 1, aborted, TC_ERR_WAIT_ACC_FREE)) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_acc + (uint32_t)(buf * BN);
       int kt = kt_begin;
       for (; kt < kt_end; ++kt) {
-        if (!mbar_wait(&sh->full[s], lap, aborted, TC_ERR_WAIT_FULL)) break;
+        if (!mbar_wait_warp(&sh->full[s], lap, aborted, TC_ERR_WAIT_FULL)) break;
         tc_fence_after();
         const uint32_t a_lo = ring_lo + s * (STAGE_BYTES >> 4), w_lo = a_lo + (TC_BM * TC_BK * 2 >> 4);
 #pragma unroll
@@ -263,8 +270,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const int buf = local & 1;
       TcOld<ADD> old;
       tc_load_old<ADD>(old, lane, Cp, t.row0 + lane_group * 32, t.row_end, t.n0 + c_begin, N);
-      const bool there = mbar_wait(&sh->acc_full[buf], (local >> 1) & 1, aborted, TC_ERR_WAIT_ACC);
-      if (!__all_sync(0xffffffffu, there)) break;          // the whole warp leaves together
+      if (!mbar_wait_warp(&sh->acc_full[buf], (local >> 1) & 1, aborted, TC_ERR_WAIT_ACC)) break;
       tc_fence_after();
 #pragma unroll 1
       for (int c0 = c_begin; c0 < BN; c0 += 64) {
@@ -283,6 +289,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   }
   if (*aborted) drain_after_abort();
+  __syncwarp();                                          // (the deallocation wants the whole warp)
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

@@ -65,6 +65,10 @@ __device__ __noinline__ bool t2_wait_long(uint64_t* bar, uint32_t parity, volati
 __device__ __forceinline__ bool t2_wait(uint64_t* bar, uint32_t parity, volatile int* aborted, int code) {
   return mbar_try_wait(bar, parity) || t2_wait_long(bar, parity, aborted, code);
 }
+// The same by all lanes of a warp (mbar_wait_warp of gemm_tc.cu).
+__device__ __forceinline__ bool t2_wait_warp(uint64_t* bar, uint32_t parity, volatile int* aborted, int code) {
+  return __all_sync(0xffffffffu, t2_wait(bar, parity, aborted, code));
+}
 
 struct __align__(16) T2Shared {
   uint64_t full[T2_MAX_STAGES];     // (leader) both blocks' stages hold their operands
@@ -177,12 +181,12 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (!t.valid) continue;
         const int buf = local % T2_ACC_BUFFERS;
         const int use = local / T2_ACC_BUFFERS;          // how often this accumulator was used before
-        if (!t2_wait(&sh->acc_empty[buf], (use & 1) ^ 1, aborted, T2_ERR_ACC_FREE)) break;
+        if (!t2_wait_warp(&sh->acc_empty[buf], (use & 1) ^ 1, aborted, T2_ERR_ACC_FREE)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_acc + (uint32_t)(buf * T2_BN);
         int kt = 0;
         for (; kt < k_tiles; ++kt) {
-          if (!t2_wait(&sh->full[s], lap, aborted, T2_ERR_FULL)) break;        // both blocks' stage s
+          if (!t2_wait_warp(&sh->full[s], lap, aborted, T2_ERR_FULL)) break;        // both blocks' stage s
           tc_fence_after();
           const uint32_t a_lo = ring_lo + s * (T2_STAGE_BYTES >> 4), w_lo = a_lo + (T2_BM * T2_BK * 2 >> 4);
 #pragma unroll
@@ -211,8 +215,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const int first_row = t.row0 + (int)rank * T2_BM + lane_group * 32;
       TcOld<ADD> old;
       tc_load_old<ADD>(old, lane, C, first_row, t.row_end, t.n0 + c_begin, N);
-      const bool there = t2_wait(&sh->acc_full[buf], use & 1, aborted, T2_ERR_ACC);
-      if (!__all_sync(0xffffffffu, there)) break;        // the whole warp leaves together
+      if (!t2_wait_warp(&sh->acc_full[buf], use & 1, aborted, T2_ERR_ACC)) break;
       tc_fence_after();
 #pragma unroll 1
       for (int c0 = c_begin; c0 < c_begin + EPI_COLS; c0 += 32) {
@@ -491,12 +494,12 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
         const uint32_t idesc = instr_desc_bf16(2 * T2_BM, t.nt);
         const int buf = local % T2_ACC_BUFFERS;
         const int use = local / T2_ACC_BUFFERS;
-        if (!t2_wait(&sh->acc_empty[buf], (use & 1) ^ 1, aborted, T2_ERR_ACC_FREE)) break;
+        if (!t2_wait_warp(&sh->acc_empty[buf], (use & 1) ^ 1, aborted, T2_ERR_ACC_FREE)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_acc + (uint32_t)(buf * T2_BN);
         int kt = 0;
         for (; kt < k_tiles; ++kt, next_stage()) {
-          if (!t2_wait(&sh->full[s], lap, aborted, T2_ERR_FULL)) break;
+          if (!t2_wait_warp(&sh->full[s], lap, aborted, T2_ERR_FULL)) break;
           tc_fence_after();
           const uint32_t w_lo = ring_lo + s * (stage_bytes >> 4), a_lo = w_lo + (T2G_W_BYTES >> 4);
 #pragma unroll
@@ -516,8 +519,7 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
       const T2GItem t = t2g_item(item, plan, groups, N);
       const int buf = local % T2_ACC_BUFFERS;
       const int use = local / T2_ACC_BUFFERS;
-      const bool there = t2_wait(&sh->acc_full[buf], use & 1, aborted, T2_ERR_ACC);
-      if (!__all_sync(0xffffffffu, there)) break;        // the whole warp leaves together
+      if (!t2_wait_warp(&sh->acc_full[buf], use & 1, aborted, T2_ERR_ACC)) break;
       tc_fence_after();
       const int col0 = t.f0 + (int)rank * T2_BM + lane_group * 32;     // this warp's 32 columns of C: one per lane
       auto release = [&]() {                             // all that this warp reads of the accumulator is in registers

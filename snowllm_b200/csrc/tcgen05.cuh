@@ -19,7 +19,7 @@ __device__ __forceinline__ uint32_t instr_desc_bf16(int m, int n) {
 
 // D += A B, both operands by the low words of their descriptors.  For a loop that a whole warp walks with one lane issuing
 // (`elected`): the instruction carries the lane's predicate, so that no branch stands around it and all that leads up to it is the
-// same in every lane.  An issuing lane of its own, with its branch, descriptors formed for each instruction and three reads of the
+// same in every lane; the loop's waits are the warp's (mbar_wait_warp).  An issuing lane of its own, with its branch, descriptors formed for each instruction and three reads of the
 // abort word a k-block, took 620 cycles per k-block of 64 whatever the tile: more than the 512 that the products of a
 // 256-column tile take.  Measured, such a lane / so, us: 8,192 x 6,144 x 2,048 157 / 137, 8,192 x 2,048 x 8,192 218 / 195, 1,024 x 2,048 x
 // 8,192 50 / 37, experts' gate|up of 64 tokens (32 groups of 3,584 x 2,048) 87.7 / 77.8 = 6.0 TB/s, of 2,048 tokens 150 / 141.
