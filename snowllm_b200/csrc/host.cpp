@@ -89,11 +89,16 @@ inline PyObject* result(int status, int n, const at::Tensor& out) {
   return THPVariable_Wrap(out);
 }
 
-#define LAUNCH(call)               \
-  do {                             \
-    Py_BEGIN_ALLOW_THREADS         \
-    status = (call);               \
-    Py_END_ALLOW_THREADS           \
+// The interpreter's lock given back for as long as this stands, an exception's way out included: a tensor without memory throws
+// where its pointer is asked for, and what catches that speaks to Python.
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+#define LAUNCH(call)   \
+  do {                 \
+    Unlocked unlocked; \
+    status = (call);   \
   } while (0)
 #define GUARD_BEGIN try {
 #define GUARD_END                                      \
@@ -301,11 +306,12 @@ PyObject* route_sort(PyObject*, PyObject* const* a, Py_ssize_t n) {
              pos = empty({pairs}, I32, *x), sorted = empty({pairs}, I32, *x);
   int status, planes = 0;
   const S s = stream();
-  Py_BEGIN_ALLOW_THREADS
-  status = f_tc_parts(ptr(x), ptr(w), ptr(&parts), (int)M, (int)E, (int)H, &planes, ahead, s);
-  if (!status) status = f_topk(ptr(&parts), ptr(bias), ptr(&ids), ptr(&wts), (int)M, (int)E, k, flags, scaling, 0, planes, s);
-  if (!status) status = f_sort(ptr(&ids), ptr(&offsets), ptr(&pos), ptr(&sorted), (int)pairs, (int)E, (int)E - identity, s);
-  Py_END_ALLOW_THREADS
+  {
+    Unlocked unlocked;
+    status = f_tc_parts(ptr(x), ptr(w), ptr(&parts), (int)M, (int)E, (int)H, &planes, ahead, s);
+    if (!status) status = f_topk(ptr(&parts), ptr(bias), ptr(&ids), ptr(&wts), (int)M, (int)E, k, flags, scaling, 0, planes, s);
+    if (!status) status = f_sort(ptr(&ids), ptr(&offsets), ptr(&pos), ptr(&sorted), (int)pairs, (int)E, (int)E - identity, s);
+  }
   if (status) return PyLong_FromLong(status);
   launches += 3;
   PyObject* out = PyTuple_New(5);
