@@ -78,6 +78,12 @@ inline bool is(const at::Tensor* t, at::ScalarType dtype, int64_t m, int64_t n) 
 inline bool small(const at::Tensor* t, at::ScalarType dtype) { return t && (t->scalar_type() == F32 || t->scalar_type() == dtype); }
 inline bool aligned(const at::Tensor* t) { return ((uintptr_t)t->data_ptr() & 15) == 0; }
 inline long to_int(PyObject* o) { return PyLong_AsLong(o); }
+// Whether every number asked for so far was one; if not, the caller's long way meets it again and says so.
+inline bool numbers() {
+  if (!PyErr_Occurred()) return true;
+  PyErr_Clear();
+  return false;
+}
 inline S stream() { return (S)c10::cuda::getCurrentCUDAStream().stream(); }
 inline at::Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, const at::Tensor& like) {
   return at::empty(sizes, at::TensorOptions().dtype(dtype).device(like.device()));
@@ -101,14 +107,8 @@ struct Unlocked {
     status = (call);   \
   } while (0)
 #define GUARD_BEGIN try {
-#define GUARD_END                                      \
-  }                                                    \
-  catch (const std::exception& e) {                    \
-    PyErr_SetString(PyExc_RuntimeError, e.what());     \
-    return nullptr;                                    \
-  }
 // Out of memory has to come out as torch's own error: the caller's long way meets it again and raises that.
-#define GUARD_END_OOM                                  \
+#define GUARD_END                                      \
   }                                                    \
   catch (const c10::OutOfMemoryError&) { Py_RETURN_NONE; } \
   catch (const std::exception& e) {                    \
@@ -136,12 +136,13 @@ PyObject* add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t R = rows ? rows->numel() : M;
   const float eps = (float)PyFloat_AsDouble(a[6]);
   const int ahead = a[9] == Py_True;
+  if (!numbers()) Py_RETURN_NONE;
   at::Tensor out = empty({R, H}, dtype, *res);
   int status;
   LAUNCH(f_norm(ptr(res), ptr(delta), ptr(gamma), gamma->scalar_type() == F32, ptr(&out), ptr(rows), (int)R, (int)H, eps,
                 dtype == BF16, ptr(y), ptr(pos), ptr(w), k, 1.f, nullptr, 0, ahead, stream()));
   return result(status, 1, out);
-  GUARD_END_OOM
+  GUARD_END
 }
 
 // (x, w, out_f32, act, w_ahead, route) -> x . w^T.  route 0: few rows, 1: tcgen05, 2: tcgen05 on pairs of SMs, 3: CUDA cores
@@ -151,7 +152,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   GUARD_BEGIN
   const at::Tensor *x = tensor(a[0]), *w = tensor(a[1]);
   const int f32 = (int)to_int(a[2]), act = (int)to_int(a[3]), ahead = (int)to_int(a[4]), route = (int)to_int(a[5]);
-  if (!x || !w || x->dim() != 2 || w->dim() != 2) Py_RETURN_NONE;
+  if (!numbers() || !x || !w || x->dim() != 2 || w->dim() != 2) Py_RETURN_NONE;
   const at::ScalarType dtype = route == 3 ? F32 : BF16;
   const int64_t M = x->size(0), K = x->size(1), N = w->size(0);
   if (x->scalar_type() != dtype || w->scalar_type() != dtype || w->size(1) != K || M < 1 || (act && f32)) Py_RETURN_NONE;
@@ -178,7 +179,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   else
     LAUNCH(f_simt(ptr(x), ptr(w), ptr(&out), (int)M, (int)N, (int)K, nullptr, 1, nullptr, 1, (int)M, 1, 0, ahead, stream()));
   return result(status, 1, out);
-  GUARD_END_OOM
+  GUARD_END
 }
 
 // (x, w, into, w_ahead, route 1 or 2) -> into, float [M, N], to which x . w^T has been added
@@ -187,7 +188,7 @@ PyObject* linear_add(PyObject*, PyObject* const* a, Py_ssize_t n) {
   GUARD_BEGIN
   const at::Tensor *x = tensor(a[0]), *w = tensor(a[1]), *into = tensor(a[2]);
   const int ahead = (int)to_int(a[3]), route = (int)to_int(a[4]);
-  if (!is(x, BF16) || !is(w, BF16) || x->dim() != 2 || w->dim() != 2 || w->size(1) != x->size(1) ||
+  if (!numbers() || !is(x, BF16) || !is(w, BF16) || x->dim() != 2 || w->dim() != 2 || w->size(1) != x->size(1) ||
       !is(into, F32, x->size(0), w->size(0)) || x->size(0) < 1 || x->size(1) % 8 || !aligned(x) || !aligned(w) || !aligned(into)) Py_RETURN_NONE;
   const int M = (int)x->size(0), K = (int)x->size(1), N = (int)w->size(0);
   if (route == 2 ? !f_tc2 : route == 1 ? !f_tc || !f_tc_scratch : true) Py_RETURN_NONE;
@@ -204,7 +205,7 @@ PyObject* linear_add(PyObject*, PyObject* const* a, Py_ssize_t n) {
     LAUNCH(f_tc(ptr(x), ptr(w), ptr(into), M, N, K, nullptr, 1, (M + 127) / 128, 2, 0, need ? ptr(&scratch) : nullptr, ahead, stream()));
   }
   return result(status, count, *into);
-  GUARD_END_OOM
+  GUARD_END
 }
 
 // (x, w [G, N, K], offsets, rows | None, div, out_f32, act) -> the grouped product on pairs of SMs of x's rows in sorted order
@@ -214,7 +215,7 @@ PyObject* grouped(PyObject*, PyObject* const* a, Py_ssize_t n) {
   GUARD_BEGIN
   const at::Tensor *x = tensor(a[0]), *w = tensor(a[1]), *offsets = tensor(a[2]), *rows = tensor(a[3]);
   const int div = (int)to_int(a[4]), f32 = (int)to_int(a[5]), act = (int)to_int(a[6]);
-  if (!is(x, BF16) || !is(w, BF16) || x->dim() != 2 || w->dim() != 3 || w->size(2) != x->size(1) || !is(offsets, I32, w->size(0) + 1) ||
+  if (!numbers() || !is(x, BF16) || !is(w, BF16) || x->dim() != 2 || w->dim() != 3 || w->size(2) != x->size(1) || !is(offsets, I32, w->size(0) + 1) ||
       (act && f32) || x->size(1) % 8 || !aligned(x) || !aligned(w)) Py_RETURN_NONE;
   const int64_t G = w->size(0), N = w->size(1), K = w->size(2);
   int status = 0, count = 1;
@@ -233,7 +234,7 @@ PyObject* grouped(PyObject*, PyObject* const* a, Py_ssize_t n) {
   at::Tensor out = empty({M, act ? N / 2 : N}, f32 ? F32 : BF16, *x);
   LAUNCH(f_tc2(ptr(x), ptr(w), ptr(&out), (int)M, (int)N, (int)K, ptr(offsets), (int)G, f32, act, stream()));
   return result(status, count, out);
-  GUARD_END_OOM
+  GUARD_END
 }
 
 // (bcx, taps, state, cu_seqlens, seg_start, seg_slot, row_seg, w_ahead) -> y
@@ -255,7 +256,7 @@ PyObject* short_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   LAUNCH(f_conv(ptr(x), ptr(w), w->scalar_type() == F32, ptr(state), ptr(cu), ptr(start), ptr(slot), ptr(seg), ptr(&out), (int)M,
                 (int)B, (int)H, (int)L, dtype == BF16, ahead, stream()));
   return result(status, L > 1 && M != B ? 2 : 1, out);
-  GUARD_END_OOM
+  GUARD_END
 }
 
 // (qkv, q_gamma | None, k_gamma | None, eps, inv_freq | None, rot_dim, positions, row_seg, block_table, page_size, pool, heads,
@@ -278,13 +279,14 @@ PyObject* rope(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!is(at_, I32, M) || !is(seg, I32, M) || !is(table, I32) || table->dim() != 2 || !is(pool, dtype) || pool->dim() != 5 ||
       pool->size(1) != 2 || pool->size(2) != nkv || pool->size(3) != page || pool->size(4) != hd) Py_RETURN_NONE;
   const float eps = (float)PyFloat_AsDouble(a[3]);
+  if (!numbers()) Py_RETURN_NONE;
   at::Tensor q = empty({M, nh, hd}, dtype, *qkv);
   int status;
   LAUNCH(f_rope(ptr(qkv), norm ? ptr(qg) : nullptr, norm ? ptr(kg) : nullptr, norm && qg->scalar_type() == F32, norm, eps, ptr(freq),
                 freq ? rot : 0, ptr(at_), ptr(seg), ptr(table), (int)table->size(1), page, ptr(pool), ptr(&q), (int)M, nh, nkv, hd, write,
                 dtype == BF16, stream()));
   return result(status, 1, q);
-  GUARD_END_OOM
+  GUARD_END
 }
 
 // (x, router, bias | None, top_k, flags, scaling, identity, w_ahead) -> (ids, weights, offsets, pair_pos, sorted_pair): the router of
@@ -301,6 +303,7 @@ PyObject* route_sort(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const long long need = f_tc_scratch((int)M, (int)E, (int)H, 0);
   if (need <= 0) Py_RETURN_NONE;
   const float scaling = (float)PyFloat_AsDouble(a[5]);
+  if (!numbers()) Py_RETURN_NONE;
   at::Tensor parts = empty({(int64_t)need}, at::kByte, *x);
   at::Tensor ids = empty({M, k}, I32, *x), wts = empty({M, k}, F32, *x), offsets = empty({E + 1}, I32, *x),
              pos = empty({pairs}, I32, *x), sorted = empty({pairs}, I32, *x);
@@ -319,7 +322,7 @@ PyObject* route_sort(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Tensor* all[5] = {&ids, &wts, &offsets, &pos, &sorted};
   for (int i = 0; i < 5; ++i) PyTuple_SET_ITEM(out, i, THPVariable_Wrap(*all[i]));
   return out;
-  GUARD_END_OOM
+  GUARD_END
 }
 
 // (gate_up, interleaved) -> silu(gate) * up
@@ -332,7 +335,7 @@ PyObject* swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int status;
   LAUNCH(f_swiglu(ptr(h), ptr(&out), (int)h->size(0), (int)(h->size(1) / 2), a[1] == Py_True, h->scalar_type() == BF16, stream()));
   return result(status, 1, out);
-  GUARD_END_OOM
+  GUARD_END
 }
 
 // (name, address): an entry point of a loaded library; names that nothing here calls are ignored

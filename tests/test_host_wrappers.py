@@ -28,9 +28,42 @@ with FakeTensorMode():
                 print("raised")
 """
 
+NOT_A_NUMBER = """
+import ctypes, torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from snowllm_b200.csrc import build
+host = build.load_host()
+NOTHING = ctypes.CFUNCTYPE(ctypes.c_int)(lambda: 0)
+SCRATCH = ctypes.CFUNCTYPE(ctypes.c_longlong)(lambda: 64)
+for name in ("snk_gemm_simt", "snk_gemm_tc2", "snk_gemm_tc", "snk_add_rmsnorm", "snk_qk_norm_rope_cache", "snk_gemm_tc_parts",
+             "snk_moe_topk", "snk_moe_sort"):
+    host.bind(name, ctypes.cast(NOTHING, ctypes.c_void_p).value)
+host.bind("snk_gemm_tc_scratch_bytes", ctypes.cast(SCRATCH, ctypes.c_void_p).value)
+with FakeTensorMode():
+    f32 = lambda *s: torch.empty(*s, device="cuda")
+    bf = lambda *s: torch.empty(*s, device="cuda", dtype=torch.bfloat16)
+    i32 = lambda *s: torch.empty(*s, device="cuda", dtype=torch.int32)
+    for out in (host.linear(f32(4, 32), f32(8, 32), 1, 0, None, 3),
+                host.linear_add(bf(32, 32), bf(8, 32), f32(32, 8), None, 2),
+                host.grouped(bf(32, 32), bf(2, 8, 32), i32(3), None, "1", 1, 0),
+                host.add_rmsnorm(f32(4, 32), None, None, None, None, f32(32), "eps", False, None, False),
+                host.rope(f32(4, 64), None, None, None, None, 0, i32(4), i32(4), i32(1, 1), 4, f32(1, 2, 1, 4, 16), 2, 1, 16, True),
+                host.route_sort(bf(70, 32), bf(8, 32), None, 2, 1, "1", 0, 0)):
+        print(out)
+"""
+
+
+def run(program: str) -> list:
+    done = subprocess.run([sys.executable, "-c", program], cwd=CSRC.parent.parent, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
+    return done.stdout.split()
+
 
 def test_a_tensor_without_memory_raises():
     """A tensor that has no pointer to give (here one that stands for a CUDA tensor) is an error, and the process goes on."""
-    done = subprocess.run([sys.executable, "-c", PROGRAM], cwd=CSRC.parent.parent, capture_output=True, text=True, timeout=300)
-    assert done.returncode == 0, done.stderr[-2000:]
-    assert done.stdout.split() == ["raised"] * 6
+    assert run(PROGRAM) == ["raised"] * 6
+
+
+def test_what_is_no_number_goes_the_long_way():
+    """The wrappers in Python say what is wrong with it; these return None for that, and leave no error behind them."""
+    assert run(NOT_A_NUMBER) == ["None"] * 6
