@@ -19,6 +19,13 @@ Interfaces (duck-typed; these base classes only hold what is common):
 * block:       ``forward(ctx, residual, delta, cache, owns_cache) -> delta`` (how mixer, feed-
                forward and norms are arranged around the residual stream)
 
+Optional, of a mixer or feed-forward whose ``forward`` is written for it, and of no part that derives from it with a ``forward`` of
+its own (``offered``):
+* ``adds_to_stream = True``: where the block lends the residual stream (``ctx.stream``), ``forward`` may add its output to it and
+  return None;
+* ``reads_pending_norm(*args) -> w | None``: the weight of the product that alone reads x; ``forward`` may then be given a
+  ``kernels.PendingNorm`` for x.  Its counterpart in a norm is ``before(ctx, residual, delta, w)``.
+
 No part knows which model it is in: what it needs comes through its parameters, its tensors
 and the step context.
 """
@@ -29,6 +36,17 @@ from typing import Callable, Mapping
 import torch
 
 from .spec import TensorSpec
+
+
+def offered(part, name: str):
+    """``part``'s optional ``name``, where it belongs to the ``forward`` that the part has; else None.  A part that derives from
+    another one and brings a ``forward`` of its own has not said that this one may be given what the other's may."""
+    for space in (getattr(part, "__dict__", {}), *map(vars, type(part).__mro__)):
+        if name in space:
+            return getattr(part, name)
+        if "forward" in space:
+            return None
+    return None
 
 
 class Part:

@@ -23,7 +23,7 @@ import torch
 from ..errors import ConfigError
 from ..ops import kernels
 from ..trace import span
-from .base import Part
+from .base import Part, offered
 from ..ops import linear
 from .registry import lookup, register_block
 from .spec import INIT_BIAS, KEEP_F32, TensorSpec
@@ -62,8 +62,7 @@ class PreNormBlock:
     def _normed(norm, part, ctx, residual, delta, *args):
         """The norm's rows for ``part``, or the norm left to the part's first product."""
         if ctx.M <= kernels.PENDING_NORM_ROWS:
-            reads = getattr(part, "reads_pending_norm", None)
-            before = getattr(norm, "before", None)
+            reads, before = offered(part, "reads_pending_norm"), offered(norm, "before")
             if reads is not None and before is not None:
                 return before(ctx, residual, delta, reads(*args))
         return norm.forward(ctx, residual, delta)
@@ -76,7 +75,7 @@ class PreNormBlock:
         # comes in again.  (Nobody may read the delta then, and nothing may stand between it and the stream.)
         lend = residual if ctx.taps is None and self.residual_scale == 1.0 and self.side is None else None
         with span(self._names[1]):
-            ctx.stream = lend if getattr(self.mixer, "adds_to_stream", False) else None
+            ctx.stream = lend if offered(self.mixer, "adds_to_stream") else None
             delta = self.mixer.forward(ctx, x, cache, owns_cache)
             ctx.stream = None
         ctx.tap("mixer_out", delta)
@@ -99,7 +98,7 @@ class PreNormBlock:
             x = self._normed(self.ffn_norm, self.ffn, ctx, residual, delta)
         ctx.tap("ffn_in", x)
         with span(self._names[3]):
-            ctx.stream = lend if getattr(self.ffn, "adds_to_stream", False) else None
+            ctx.stream = lend if offered(self.ffn, "adds_to_stream") else None
             delta = self.ffn.forward(ctx, x)
             ctx.stream = None
         ctx.tap("ffn_out", delta)

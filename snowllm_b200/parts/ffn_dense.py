@@ -49,6 +49,8 @@ class GatedFFN(SwiGLU):
     bfloat16 products apply the gate at their store (gate and up rows interleaved by 8); float32, and widths
     that are no multiple of 8, run the product and then one elementwise kernel."""
     libraries = SwiGLU.libraries + ("sublayer",)
+    adds_to_stream = True
+    reads_pending_norm = SwiGLU.reads_pending_norm
 
     def __init__(self, dtype, names, *, hidden_size: int, intermediate_size: int, activation: str = "silu",
                  limit: float | None = None):

@@ -1,0 +1,92 @@
+"""What a block hands to parts that offer to take it (the residual stream to add to, a norm that is still to be formed), and that a
+part which derives from such a one with a ``forward`` of its own is given neither."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from snowllm_b200.ops import kernels
+from snowllm_b200.parts.attention import Attention
+from snowllm_b200.parts.base import offered
+from snowllm_b200.parts.block import PreNormBlock
+from snowllm_b200.parts.ffn_dense import GatedFFN, SwiGLU
+from snowllm_b200.parts.norm import RMSNorm
+from snowllm_b200.parts.short_conv import ShortConv
+
+PENDING = object()
+
+
+class Norm:
+    def forward(self, ctx, residual, delta=None, rows=None):
+        if delta is not None:
+            residual += delta
+        return residual.clone()
+
+    def before(self, ctx, residual, delta, w):
+        self.forward(ctx, residual, delta)
+        return PENDING
+
+
+class Doubles:
+    adds_to_stream = True
+
+    def reads_pending_norm(self, *args):
+        return torch.ones(1)
+
+    def forward(self, ctx, x, *args):
+        self.seen = (x is PENDING, ctx.stream is not None)
+        out = torch.ones(ctx.M, 4) if x is PENDING else 2 * x
+        if ctx.stream is not None:
+            ctx.stream += out
+            return None
+        return out
+
+
+class DoublesAndHalves(Doubles):
+    """Works on what the part above returns."""
+
+    def forward(self, ctx, x, *args):
+        return super().forward(ctx, x, *args) * 0.25
+
+
+class LoudNorm(Norm):
+    def forward(self, ctx, residual, delta=None, rows=None):
+        return super().forward(ctx, residual, delta) + 1
+
+
+def step(part, M, norm=Norm):
+    ctx = SimpleNamespace(M=M, taps=None, stream=None, tap=lambda *a: None)
+    residual = torch.ones(M, 4)
+    delta = PreNormBlock(part, part, norm(), norm()).forward(ctx, residual, None, None)
+    assert ctx.stream is None
+    return residual if delta is None else residual + delta
+
+
+def test_a_part_is_given_what_it_offers_to_take():
+    part = Doubles()
+    assert torch.equal(step(part, 40), torch.full((40, 4), 9.0)) and part.seen == (False, True)
+    step(part, kernels.PENDING_NORM_ROWS)
+    assert part.seen == (True, True)
+
+
+@pytest.mark.parametrize("M", [1, 40])
+def test_a_part_with_a_forward_of_its_own_is_not(M):
+    part = DoublesAndHalves()
+    assert torch.equal(step(part, M), torch.full((M, 4), 2.25)) and part.seen == (False, False)
+    loose = Doubles()
+    loose.forward = lambda ctx, x, *args: torch.zeros(ctx.M, 4) if ctx.stream is None and x is not PENDING else None
+    assert torch.equal(step(loose, M), torch.ones(M, 4))
+    step(loose, M)
+
+
+def test_nor_is_a_norm_asked_for_what_another_one_offers():
+    part = Doubles()
+    step(part, 1, LoudNorm)
+    assert part.seen == (False, True)
+
+
+def test_what_the_framework_s_own_parts_offer():
+    for cls in (Attention, ShortConv, SwiGLU, GatedFFN):
+        part = cls.__new__(cls)
+        assert offered(part, "adds_to_stream") and offered(part, "reads_pending_norm")
+    assert offered(RMSNorm.__new__(RMSNorm), "before")
