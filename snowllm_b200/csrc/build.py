@@ -137,7 +137,10 @@ def build_host() -> pathlib.Path:
     if not out.exists():
         tmp = out.with_suffix(f".tmp{os.getpid()}.so")
         print("[snowllm_b200] compiling host.cpp ...", file=sys.stderr, flush=True)
-        proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        try:
+            proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        except OSError as e:
+            raise KernelError(f"the C++ compiler did not run: {e}") from e
         if proc.returncode != 0:
             tmp.unlink(missing_ok=True)
             raise KernelError(f"the C++ compiler failed on host.cpp:\n{proc.stdout}")

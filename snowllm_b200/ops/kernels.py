@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import os
+import warnings
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
@@ -184,17 +185,24 @@ def fn(name: str):
 
 
 _native = None
+_native_missing = False
 
 
 def native():
     """The extension module that holds the launch wrappers in C++ (csrc/host.cpp), or None while the ledger is on, which only
-    the wrappers here keep.  One of its functions returns None where its checks are not met, or where nobody has called the
+    the wrappers here keep, and where the module cannot be compiled or loaded (a warning says so once: everything still runs, with
+    more host time a launch).  One of its functions returns None where its checks are not met, or where nobody has called the
     library's entry point from here yet: the wrapper here then does the call, or says what is wrong."""
-    global _native
-    if ledger is not None:
+    global _native, _native_missing
+    if ledger is not None or _native_missing:
         return None
     if _native is None:
-        module = build.load_host()
+        try:
+            module = build.load_host()
+        except KernelError as e:
+            _native_missing = True
+            warnings.warn(f"the launch wrappers in C++ are not there, the ones in Python do their work: {e}", RuntimeWarning)
+            return None
         for name, f in _functions.items():
             module.bind(name, ctypes.cast(f, c_void_p).value)
         _native = module

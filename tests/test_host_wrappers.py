@@ -4,7 +4,11 @@ import pathlib
 import re
 import subprocess
 import sys
+import warnings
 
+import pytest
+
+from snowllm_b200.csrc import build
 from snowllm_b200.ops import kernels
 
 CSRC = pathlib.Path(kernels.__file__).resolve().parent.parent / "csrc"
@@ -67,3 +71,18 @@ def test_a_tensor_without_memory_raises():
 def test_what_is_no_number_goes_the_long_way():
     """The wrappers in Python say what is wrong with it; these return None for that, and leave no error behind them."""
     assert run(NOT_A_NUMBER) == ["None"] * 6
+
+
+def test_without_the_module_the_wrappers_in_python_do_the_work(monkeypatch):
+    """No compiler, or no headers for it: said once, and every call goes the Python wrapper's way."""
+    monkeypatch.setattr(kernels, "_native", None)
+    monkeypatch.setattr(kernels, "_native_missing", False, raising=False)
+    monkeypatch.setattr(build, "_host", None)
+    monkeypatch.setattr(build, "host_path", lambda: pathlib.Path("/nowhere/libsnk_host_0.so"))
+    monkeypatch.setenv("CXX", "/nowhere/no-such-compiler")
+    with pytest.warns(RuntimeWarning, match="wrappers in C\\+\\+"):
+        assert kernels.native() is None
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert kernels.native() is None
+    assert kernels.launch_count() == kernels._launches
