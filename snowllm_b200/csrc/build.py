@@ -107,6 +107,13 @@ def _compile(name: str, out: pathlib.Path) -> None:
 # --- host.cpp: a Python extension of the launch wrappers -----------------------------------------------------
 
 _host = None
+HOST_FLAGS = ["-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
+HOST_LIBS = ["-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"]
+
+
+def _host_flags() -> list[str]:
+    import torch
+    return [*HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
 
 
 def _host_command(out: pathlib.Path) -> list[str]:
@@ -115,19 +122,18 @@ def _host_command(out: pathlib.Path) -> list[str]:
     import torch
     root = pathlib.Path(torch.__file__).resolve().parent
     cuda = pathlib.Path(_nvcc()).resolve().parent.parent
-    cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
-    return [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    return [os.environ.get("CXX") or shutil.which("g++") or "g++", *_host_flags(),
             "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"), "-I", str(cuda / "include"),
             "-I", sysconfig.get_paths()["include"], str(HERE / "host.cpp"), "-o", str(out), "-L", str(root / "lib"),
-            "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"]
+            *HOST_LIBS]
 
 
 def host_path() -> pathlib.Path:
     import torch
     h = hashlib.sha256()
     h.update((HERE / "host.cpp").read_bytes())
-    h.update(f"{torch.__version__} {sys.version}".encode())
+    # (the compiler's name where one was chosen: a build that is there serves without any)
+    h.update(" ".join([torch.__version__, sys.version, os.environ.get("CXX", ""), *_host_flags(), *HOST_LIBS]).encode())
     return _build_dir() / f"libsnk_host_{h.hexdigest()[:16]}.so"
 
 

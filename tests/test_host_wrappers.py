@@ -86,3 +86,14 @@ def test_without_the_module_the_wrappers_in_python_do_the_work(monkeypatch):
         warnings.simplefilter("error")
         assert kernels.native() is None
     assert kernels.launch_count() == kernels._launches
+
+
+def test_another_compiler_or_other_flags_are_another_build(monkeypatch):
+    paths = {build.host_path()}
+    monkeypatch.setenv("CXX", "some-other-c++")
+    paths.add(build.host_path())
+    monkeypatch.setattr(build, "HOST_FLAGS", ["-O3"], raising=False)
+    paths.add(build.host_path())
+    monkeypatch.setattr(build.subprocess, "run", lambda *a, **kw: pytest.fail("ran"))        # a path costs no compiler
+    monkeypatch.setattr(build, "_nvcc", lambda: pytest.fail("asked for nvcc"))
+    assert build.host_path() in paths and len(paths) == 3
