@@ -548,22 +548,20 @@ static int at_launch(const void* q, long long M, const void* pool, const void* v
     if (rc) return rc;
   }
   const size_t smem = (size_t)(AT_KSTAGES + AT_VSTAGES) * AT_KV_BYTES + AT_P_BYTES + sizeof(AtShared);
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(attention_prefill_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(attention_prefill_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(attention_prefill_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(attention_prefill_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    configured = true;
-  }
   const float log2e = 1.4426950408889634f;
   const float scale_log2 = softcap > 0.f ? softcap * log2e : scale * log2e;      // of what enters the softmax
   const float cap_in = softcap > 0.f ? 2.f * log2e * scale / softcap : 0.f;
-#define AT_LAUNCH(EXTRA_, CAP_)                                                                                  \
-  snk_launch(attention_prefill_tc_kernel<EXTRA_, CAP_>, dim3(n_tiles, nh), dim3(AT_THREADS), smem, stream, map_q, \
-             map_kv, map_v, k_mul, v_add, block_table, max_pages, page_size, tiles, n_tiles,                     \
-             static_cast<bf16*>(out), nh, nkv, window, scale_log2, keep, slopes, sink,                           \
-             static_cast<const bf16*>(gate), gate_ld, cap_in)
+#define AT_LAUNCH(EXTRA_, CAP_)                                                                                    \
+  do {                                                                                                             \
+    static std::atomic<int> ready[SNK_MAX_DEVICES];                                                                \
+    int sms = 0;                                                                                                   \
+    rc = snk_kernel_ready(ready, attention_prefill_tc_kernel<EXTRA_, CAP_>, smem, &sms);                           \
+    if (rc) return rc;                                                                                             \
+    snk_launch(attention_prefill_tc_kernel<EXTRA_, CAP_>, dim3(n_tiles, nh), dim3(AT_THREADS), smem, stream, map_q, \
+               map_kv, map_v, k_mul, v_add, block_table, max_pages, page_size, tiles, n_tiles,                     \
+               static_cast<bf16*>(out), nh, nkv, window, scale_log2, keep, slopes, sink,                           \
+               static_cast<const bf16*>(gate), gate_ld, cap_in);                                                   \
+  } while (0)
   const bool extra = keep || slopes || sink || gate;
   if (softcap > 0.f) {
     if (extra) AT_LAUNCH(true, true);

@@ -262,6 +262,20 @@ inline int snk_device_sms(int* sms) {
   });
 }
 
+// Before a launch of `kernel` with `smem` bytes of dynamic shared memory: its limit is set on the current device, whose SMs come
+// back in *sms.  `ready` is the kernel's own (SNK_MAX_DEVICES zeros at first).
+template <typename Kernel>
+inline int snk_kernel_ready(std::atomic<int>* ready, Kernel kernel, size_t smem, int* sms) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  return snk_per_device(ready, device, sms, [&](int* n) {
+    const cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (set != cudaSuccess) return (int)set;
+    return (int)cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, device);
+  });
+}
+
 #define SNK_LAUNCH_CHECK()                       \
   do {                                           \
     cudaError_t e_ = cudaGetLastError();         \

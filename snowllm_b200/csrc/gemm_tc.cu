@@ -306,13 +306,10 @@ static int launch_tc(const CUtensorMap& map_a, const CUtensorMap& map_w, void* C
   constexpr int STAGE_BYTES = (TC_BM + BN) * TC_BK * 2;
   constexpr int STAGES = TC_SMEM_TILES / STAGE_BYTES < TC_MAX_STAGES ? TC_SMEM_TILES / STAGE_BYTES : TC_MAX_STAGES;
   const size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + sizeof(TcShared);
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(gemm_tc_kernel<BN, OutT, SWIGLU, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
+  static std::atomic<int> ready[SNK_MAX_DEVICES];
+  int sms = 0;
+  const int rc = snk_kernel_ready(ready, gemm_tc_kernel<BN, OutT, SWIGLU, ADD>, smem, &sms);
+  if (rc) return rc;
   const long long tiles = (long long)row_tiles * ((N + BN - 1) / BN) * splits;
   const int blocks = (int)(tiles < sms ? tiles : sms);     // one block per SM (shared memory), persistent
   snk_launch(gemm_tc_kernel<BN, OutT, SWIGLU, ADD>, dim3(blocks), dim3(TC_THREADS), smem, stream, map_a, map_w, static_cast<OutT*>(C), M, N, K,
@@ -370,16 +367,12 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ parts, OutT* __re
 
 // How many parts along K a plain product of these sizes is split into (1: none).
 static int tc_splits(int M, int N, int K, const int* offsets) {
-  static int sms = 0;
-  static int off = -1;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  static const bool off = [] {
     const char* e = getenv("SNOWLLM_B200_TC_SPLIT");
-    off = (e && e[0] == '0') ? 1 : 0;
-  }
-  if (offsets || off || N % 16) return 1;
+    return e && e[0] == '0';
+  }();
+  int sms = 0;
+  if (offsets || off || N % 16 || snk_device_sms(&sms)) return 1;
   const int k_tiles = (K + TC_BK - 1) / TC_BK;
   const int tiles = ((M + TC_BM - 1) / TC_BM) * ((N + 127) / 128);
   int splits = sms / tiles;                                   // parts that still find an SM each

@@ -250,13 +250,10 @@ template <typename OutT, bool SWIGLU, bool ADD = false>
 static int launch_tc2(const CUtensorMap& map_a, const CUtensorMap& map_w, void* C, int M, int N, int K,
                       int row_tiles, cudaStream_t stream, int act) {
   const size_t smem = 1024 + (size_t)T2_STAGES * T2_STAGE_BYTES + sizeof(T2Shared) + sizeof(T2Staging);
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(gemm_tc2_kernel<OutT, SWIGLU, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
+  static std::atomic<int> ready[SNK_MAX_DEVICES];
+  int sms = 0;
+  const int rc = snk_kernel_ready(ready, gemm_tc2_kernel<OutT, SWIGLU, ADD>, smem, &sms);
+  if (rc) return rc;
   const long long tiles = (long long)row_tiles * ((N + T2_BN - 1) / T2_BN);
   const int pairs = (int)(tiles < sms / 2 ? tiles : sms / 2);
   const dim3 block(64 + 32 * (SWIGLU ? T2_EPI_WARPS : T2_PLAIN_EPI_WARPS));
@@ -584,13 +581,10 @@ template <typename OutT, bool SWIGLU>
 static int launch_tc2_grouped(const T2GMaps& maps, const CUtensorMap& map_w, void* C, int M, int N, int K,
                               const int* offsets, int groups, cudaStream_t stream, int act) {
   const size_t smem = 1024 + T2G_RING_BYTES + sizeof(T2Shared) + sizeof(T2GPlan);
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(gemm_tc2_grouped_kernel<OutT, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
+  static std::atomic<int> ready[SNK_MAX_DEVICES];
+  int sms = 0;
+  const int rc = snk_kernel_ready(ready, gemm_tc2_grouped_kernel<OutT, SWIGLU>, smem, &sms);
+  if (rc) return rc;
   // at most M / 256 full row tiles and one partial tile per group
   const long long items = ((long long)M / (2 * T2_BM) + groups) * ((N + T2_BN - 1) / T2_BN);
   const int pairs = (int)(items < sms / 2 ? items : sms / 2);

@@ -1111,8 +1111,17 @@ def gemm_skinny(a, w, out_dtype=None, out=None, a_rows=None, a_div=1, offsets=No
 
 
 @functools.lru_cache(maxsize=4096)
+def _on_device(entry: str, device: int, *sizes: int) -> int:
+    """What an entry point says of sizes on ``device``, the current one (its SMs are part of the answer)."""
+    return int(fn(entry)(*sizes))
+
+
+def _of_sizes(entry: str, *sizes: int) -> int:
+    return _on_device(entry, torch._C._cuda_getDevice(), *sizes)
+
+
 def _conv_step_sizes_ok(M: int, K: int, H: int, L: int) -> bool:
-    return bool(fn("snk_conv_step_ok")(M, K, H, L))
+    return bool(_of_sizes("snk_conv_step_ok", M, K, H, L))
 
 
 def conv_step_ok(x, in_proj, weight, M: int, segments: int) -> bool:
@@ -1152,9 +1161,8 @@ def conv_step(x, in_proj, weight, state, seg_start, seg_slot, w_ahead: bool = Fa
     return out
 
 
-@functools.lru_cache(maxsize=4096)
 def _norm_product_sizes_ok(M: int, N: int, K: int, pieces: int) -> bool:
-    return bool(fn("snk_norm_product_ok")(M, N, K, pieces))
+    return bool(_of_sizes("snk_norm_product_ok", M, N, K, pieces))
 
 
 PENDING_NORM_ROWS = 2          # rows up to which a product may form a norm for itself (csrc/gemm_skinny.cu: norm_pays)
@@ -1237,10 +1245,9 @@ def gemm_tc_ok(a, w) -> bool:
             and w.data_ptr() % 16 == 0)
 
 
-@functools.lru_cache(maxsize=4096)
 def _tc_scratch_bytes(M: int, N: int, K: int, grouped: bool) -> int:
     """Bytes of float planes that a tcgen05 product of these sizes is split into along K (0: not split)."""
-    return int(fn("snk_gemm_tc_scratch_bytes")(M, N, K, int(grouped)))
+    return _of_sizes("snk_gemm_tc_scratch_bytes", M, N, K, int(grouped))
 
 
 def gemm_tc(a, w, out_dtype=None, out=None, offsets=None, swiglu=False, w_ahead: bool = False):
