@@ -161,6 +161,11 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return red[32];
 }
 
+// Threads among which the RMS norm's kernel deals the vectors of a row of H floats (thread t sums the squares of vectors t, t + threads,
+// .., and block_sum adds the threads): whoever forms a norm's rows adds in this order, so that a row's statistics never depend on
+// how many rows a step has.
+__host__ __device__ __forceinline__ int norm_threads(int H) { return H >= 2048 ? 512 : H >= 512 ? 256 : 128; }
+
 // Thread-block clusters: a barrier over all threads of the cluster's blocks, and the shared memory of
 // another block of the cluster (distributed shared memory) by the address the same variable has here.  (The aligned form wants whole
 // warps: whatever branch a warp's lanes come out of, they meet first.)

@@ -319,7 +319,7 @@ SNK_API int snk_add_rmsnorm(float* residual, const float* delta, const void* gam
   if (moe_y && (H % 4 || (uintptr_t)moe_y % 16 || (uintptr_t)residual % 16 || (uintptr_t)out % 16 || k <= 0))
     return SNK_ERR_ALIGN;
   // The block size depends on H alone, so a row's statistics never depend on the batch.
-  const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
+  const int threads = norm_threads(H);
   const size_t smem = (size_t)(((H + 3) & ~3) + 33) * sizeof(float);
   SmallVec g{gamma, gamma_is_f32};
   const int vec4 = H % 4 == 0 && (uintptr_t)residual % 16 == 0 && (uintptr_t)delta % 16 == 0 &&

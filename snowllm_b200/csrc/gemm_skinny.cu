@@ -316,14 +316,16 @@ __device__ __forceinline__ void st_wait(uint64_t* bar, uint32_t parity, volatile
 // a chain of small launches, and from the end of one kernel to the end of a next that does next to nothing are 3 to 4 us.
 //
 // ST_NORM: the rows of A are not there yet, but a residual, what is added to it, and the weight of an RMS norm.  Every block
-// forms the rows for itself in shared memory (the sum, its mean square, the rounded row: add_rmsnorm_kernel's arithmetic) and
+// forms the rows for itself in shared memory (the sum, its mean square, the rounded row: add_rmsnorm_kernel's arithmetic in its
+// order, so that a request's rows are the same bits whether one, two or more requests are in the step) and
 // writes its share of the new residual, to other memory than it is read from, as other blocks may still be reading.
 // ST_CONV: W is [B | C | x], three times H rows, and every row of A is one token of a request of its own.  A unit of 16
 // channels is their three strips, one after the other by the same block, whose threads keep the strips' sums, and the store is
 // the gated convolution over the channel's history (short_conv_decode_kernel's arithmetic), which it brings up to date.
 // Measured, a decode step before / with both, us: 1.2B sizes 1 request 759 / 672, 2 requests 780 / 692; 2.6B sizes 1 request 1,502 / 1,365;
 // 8B-A1B sizes 1 request 1,288 / 1,219, 2 requests 1,637 / 1,613.  With the norm's weight loaded behind the sum 707 of 759; the
-// convolution alone gains nothing at 8 rows.
+// convolution alone gains nothing at 8 rows.  The squares summed in an order of the block's own / in the norm's: 670.1 / 670.6 and 1,226 /
+// 1,215.
 enum { ST_NORM = 1, ST_CONV = 2 };
 #define ST_FUSE_ROWS 2                          // rows a launch may have
 #define ST_NORM_VECS 4                          // vectors of four a thread may hold of a row
@@ -366,10 +368,11 @@ __device__ __forceinline__ void st_gamma(const StFuse& f, const StNormPart& p, f
 }
 __device__ __forceinline__ void st_norm_rows(const StFuse& f, const StNormPart& p, const float4 (&g)[ST_NORM_VECS], bf16* xs, int pitch,
                                              float* red, int M, int K) {
-  const int warp = threadIdx.x >> 5, per_row = p.threads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per_row = p.threads / 32;
+  const int chains = max(norm_threads(K) / p.threads, 1);                   // 1, 2 or 4
   const bool mine = p.row < M;
   float4 v[ST_NORM_VECS];
-  float ss = 0.f;
+  float squares[ST_NORM_VECS] = {};
   if (mine) {
     const float4* res4 = reinterpret_cast<const float4*>(f.residual + (size_t)p.row * K);
 #pragma unroll
@@ -411,17 +414,25 @@ __device__ __forceinline__ void st_norm_rows(const StFuse& f, const StNormPart& 
       }
     }
 #pragma unroll
-    for (int j = 0; j < ST_NORM_VECS; ++j) {
+    for (int j = 0; j < ST_NORM_VECS; ++j) {             // a thread here is `chains` of the norm's kernel, of every chains-th vector each
+      float ss = 0.f;
+      if (j >= 1 && chains == 1) ss = squares[j - (j >= 1)];
+      if (j >= 2 && chains == 2) ss = squares[j - 2 * (j >= 2)];
       ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
       ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+      squares[j] = ss;
     }
   }
-  ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) red[warp] = ss;
+  // block_sum of those threads: a sum a warp of theirs, and then the warps'
+#pragma unroll
+  for (int j = 0; j < ST_NORM_VECS; ++j) {
+    if (j < ST_NORM_VECS - chains) continue;             // (continued by a later vector's)
+    const float ss = warp_sum(squares[j]);
+    if (lane == 0) red[p.row * 16 + (j - (ST_NORM_VECS - chains)) * per_row + warp - p.row * per_row] = ss;
+  }
   asm volatile("bar.sync 1, %0;" ::"n"(SK_WARPS * 32) : "memory");
   if (mine) {
-    float sum = 0.f;
-    for (int w = 0; w < per_row; ++w) sum += red[p.row * per_row + w];
+    const float sum = warp_sum(lane < chains * per_row ? red[p.row * 16 + lane] : 0.f);
     const float inv = rsqrtf(sum / (float)K + f.eps);
 #pragma unroll
     for (int j = 0; j < ST_NORM_VECS; ++j) {

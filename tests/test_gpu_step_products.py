@@ -98,3 +98,30 @@ def test_norm_and_conv(M, L):
     assert torch.equal(residual, other)
     assert torch.equal(y, conv_plain(bcx, weight, plain_state, start, slot))
     assert torch.equal(state, plain_state)
+
+
+# Widths at which a thread of the product stands for one, two and four threads of the norm's kernel, whole and in part
+@pytest.mark.parametrize("M,K", [(m, k) for m in (1, 2) for k in (64, 448, 512, 960, 1024, 2048)] + [(1, 2624), (1, 4096)])
+@pytest.mark.parametrize("pieces", [0, 1, 3])
+def test_norm_in_front_is_the_norms_own(M, K, pieces):
+    """The rows of a norm that a product forms for itself are the norm's own kernel's, bit for bit: what a request's rows are does not
+    depend on how many requests a step has."""
+    from snowllm_b200.ops import kernels
+    gamma = draw(K, seed=42)
+    w = torch.eye(max(K, 2560), K, device="cuda", dtype=BF)                 # the product hands the norm's rows on as they are
+    differ = torch.zeros((), dtype=torch.int64, device="cuda")
+    for seed in range(100):                              # (another order of the sum shows in the last bit of one row in thirty)
+        residual, delta = draw(M, K, seed=seed, scale=3.0, dtype=torch.float32), None
+        if pieces == 1:
+            delta = draw(M, K, seed=1000 + seed, dtype=torch.float32)
+        elif pieces:
+            pos = torch.randperm(M * pieces, generator=torch.Generator().manual_seed(seed)).to(torch.int32).cuda()
+            delta = kernels.ExpertSum(draw(M * pieces, K, seed=2000 + seed, dtype=torch.float32), pos,
+                                      draw(M, pieces, seed=3000 + seed, dtype=torch.float32))
+        if not kernels.PendingNorm.ok(residual, delta, gamma, BF, w):
+            pytest.skip("not a size for this device")
+        other = residual.clone()
+        out = kernels.PendingNorm(residual, delta, gamma, 1e-5).product(w)
+        rows = kernels.add_rmsnorm(other, delta, gamma, 1e-5, BF)
+        differ += (residual != other).sum() + (out[:, :K] != rows).sum()
+    assert int(differ) == 0
