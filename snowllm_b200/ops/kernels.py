@@ -1168,11 +1168,16 @@ def _norm_product_sizes_ok(M: int, N: int, K: int, pieces: int) -> bool:
 PENDING_NORM_ROWS = 2          # rows up to which a product may form a norm for itself (csrc/gemm_skinny.cu: norm_pays)
 
 
+def _alone(t: torch.Tensor) -> bool:
+    """Whether no other tensor looks at the memory of ``t`` (the count has ``t`` and the storage object that asks)."""
+    return torch._C._storage_Use_Count(t.untyped_storage()._cdata) <= 2
+
+
 class PendingNorm:
     """The rows of an RMS norm that have not been formed: ``residual`` (float [M, K]), what is added to it (None, a float
     tensor or an ``ExpertSum``), the norm's weight and eps.  ``product`` forms them inside the product that reads them
-    (few rows: a launch less) and gives ``residual`` the memory that holds the sum; ``dense()`` forms them by a kernel of
-    their own.  One of the two is called, once."""
+    (few rows: a launch less) and gives ``residual`` the memory that holds the sum, so nobody else may be looking at what it
+    had; ``dense()`` forms them by a kernel of their own.  One of the two is called, once."""
     dtype = torch.bfloat16
 
     def __init__(self, residual, delta, gamma, eps: float):
@@ -1187,6 +1192,8 @@ class PendingNorm:
             return False
         pieces = 0
         if delta is not None:
+            if not _alone(residual):
+                return False
             if _pieces_with_rows(delta):
                 pieces = delta.weights.shape[1]
             elif isinstance(delta, torch.Tensor):

@@ -90,3 +90,22 @@ def test_what_the_framework_s_own_parts_offer():
         part = cls.__new__(cls)
         assert offered(part, "adds_to_stream") and offered(part, "reads_pending_norm")
     assert offered(RMSNorm.__new__(RMSNorm), "before")
+
+
+def test_a_stream_that_somebody_else_looks_at_stays_where_it_is(monkeypatch):
+    """A product that forms the norm in front of it moves the stream to other memory: not while a view of it is held."""
+    monkeypatch.setattr(kernels, "_norm_product_sizes_ok", lambda *sizes: True)
+    residual, delta, gamma = torch.zeros(2, 64), torch.ones(2, 64), torch.ones(64, dtype=torch.bfloat16)
+    w = torch.zeros(4096, 64, dtype=torch.bfloat16)
+
+    def ok(delta):
+        return kernels.PendingNorm.ok(residual, delta, gamma, torch.bfloat16, w)
+
+    experts = kernels.ExpertSum(torch.ones(4, 64), torch.arange(4, dtype=torch.int32), torch.ones(2, 2))
+    assert ok(delta) and ok(experts)
+    for look in (lambda: residual[0], lambda: residual.view(-1), lambda: residual.detach()):
+        held = look()
+        assert not ok(delta) and not ok(experts)
+        assert ok(None)                                  # nothing is added: the stream is not moved
+        del held
+        assert ok(delta)
