@@ -800,24 +800,51 @@ SNK_API int snk_attention_decode_mma(const void* q, const void* pool, const int*
 // first chunk; `gate`: the head's output times sigmoid(gate[m * gate_ld + head]) (one chunk; with several the
 // merge applies it).
 //
-// A long launch holds the blocks that are on the SMs at once, and every block walks items of one (row, chunk, kv head) each,
-// counted from the rows' positions (up to FD_ROWS rows), so that chunks which a row does not reach cost nothing: a captured
-// step is launched for the longest sequence it may ever serve, and of the 32,768 blocks of 64 requests of 127 to 8,380 positions
-// 24,000 left at once.  Measured, us a launch, a block per possible chunk / so: those 64 requests 124.6 / 103.1, 64 requests of 32,700 positions
-// (every chunk reached) 718 / 681 = 6.3 TB/s; walking without the look ahead 114 and 774.  A short launch keeps a block per possible chunk
-// (8 requests of 8,192 positions, 4,096 blocks, with the merge behind it 37.0 / 38.9).
+// WALK: a long launch holds the blocks that are on the SMs at once, and every block walks items of one (row, chunk, kv head) each,
+// counted from the rows' positions, so that chunks which a row does not reach cost nothing (a captured step is launched for the longest
+// sequence it may ever serve).  Where: fd_walks, plain launches of head size 64 and up to 256 rows, from 32 possible chunks a row and 16
+// rounds of possible blocks over the SMs on.  Measured, us a launch, a block per possible chunk / walking, rows at random positions up to
+// the longest, and all at it: 28 rows of 32 chunks (16.1 rounds, the line) 54.9 / 53.0 and 83.0 / 81.9; 64 rows of 33 107 / 101 and 187 / 179; 64
+// of 128 360 / 315 and 702 / 655 = 6.6 TB/s; 256 of 32 388 / 341 and 724 / 663; 64 rows in the first tenth of 33 chunks 29.9 / 19.0.  Fewer rounds: 24
+// rows of 32 (13.8) 48.8 / 49.0 and 72.1 / 71.9.  Fewer chunks: 28 rows of 24 38.9 / 40.0 and 64.5 / 64.8, 32 rows of 24 41.0 / 42.1.  Head size 128 (a
+// block an SM) was up to 11 % slower walking, launches with options up to 44 %, more than 256 rows, whose items are not
+// counted, up to 22 %.
+// Else a block per possible chunk, which leaves ahead of all else where there is nothing to do: 300 rows in the first tenth of 33 chunks
+// 137 us, 167 with the block's number taken apart by divisions.
+// Registers: three blocks of 67 KB are on an SM whatever they take up to 168, one of 133 KB up to all.  Left to itself the compiler kept 64 wide heads to 75
+// and 128 wide ones to 101: 64 rows of 33 chunks, all at the longest, 186.7 / 184.1 and 512 / 501 us with the bounds.
 #define FD_WAIT_NS 1000000000ull
 #define FD_ROWS 256
-#define FD_WALK_ROUNDS 12            // rounds of possible blocks over the SMs from which a launch walks
+#define FD_WALK_ROUNDS 16            // rounds of possible blocks over the SMs from which a launch walks,
+#define FD_WALK_CHUNKS 32            // and chunks that a row may have
 __device__ int g_fd_status;
 
 struct FdItem {
   int m, kvh, x, z;                  // the row of the batch, kv head, row of the launch and its chunk
-  int pos, k0, k_begin, k_end, valid;
+  int pos, k0, k_begin, k_end;       // the row's position, the chunk's first position, its keys that the row reaches
 };
+// Fills in the keys of an item whose position and chunk are known; false: the row has no such chunk.
+template <bool EXTRA>
+__device__ __forceinline__ bool fd_keys(FdItem& it, int window, int keep) {
+  if (EXTRA) {
+    int first, last;
+    bool inside;
+    if (!chunk_keys(it.pos, window, keep, FD_CHUNK, it.z, first, last, it.k0, inside)) return false;
+    it.k_begin = first;
+    it.k_end = last + 1;
+    return true;
+  }
+  const int lo = window > 0 ? max(0, it.pos - window + 1) : 0;
+  const int c = lo / FD_CHUNK + it.z;
+  if ((long long)c * FD_CHUNK > it.pos) return false;
+  it.k0 = c * FD_CHUNK;
+  it.k_begin = max(lo, it.k0);
+  it.k_end = min(it.pos + 1, it.k0 + FD_CHUNK);
+  return true;
+}
 
 template <int HD, bool EXTRA, bool WALK>
-__global__ void __launch_bounds__(FA_WARPS * 32)
+__global__ void __launch_bounds__(FA_WARPS * 32, HD == 64 ? 3 : 1)
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_v,
                             int k_mul, int v_add, const bf16* __restrict__ q,
                             const int* __restrict__ block_table, int max_pages, int page_size,
@@ -826,7 +853,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const __
                             float* __restrict__ part_o, float* __restrict__ part_ml, int nh, int nkv,
                             int window, int num_chunks, float scale_log2, int keep,
                             const float* __restrict__ slopes, const float* __restrict__ sink,
-                            const bf16* __restrict__ gate, long long gate_ld, float cap_in, int M, int counted) {
+                            const bf16* __restrict__ gate, long long gate_ld, float cap_in, int M) {
   // the map is a kernel parameter: fetching it does not have to wait for the kernel in front
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_kv)) : "memory");
@@ -839,6 +866,15 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const __
     cap_in = 0.f;
   }
   pdl_begin();
+  FdItem now;
+  if (!WALK) {                                            // (ahead of all else: most blocks may find nothing to do)
+    now.x = blockIdx.x;
+    now.kvh = blockIdx.y;
+    now.z = blockIdx.z;
+    now.m = row_list ? row_list[now.x] : now.x;
+    now.pos = positions[now.m];
+    if (!fd_keys<EXTRA>(now, window, keep)) return;
+  }
   constexpr int CH = HD / 8, KT = HD / 16, NT = HD / 8, PANELS = HD / 64;
   constexpr uint32_t PANEL = FD_CHUNK * 128;              // bytes of one 64-element panel of the chunk's rows
   extern __shared__ unsigned char fd_raw[];
@@ -859,111 +895,97 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const __
     mbar_init(&bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    gave_up = 0;
+    if (WALK) gave_up = 0;
   }
-  if (WALK && counted && warp == 0) {
-    int before = 0;
-    for (int r0 = 0; r0 < M; r0 += 32) {
-      const int r = r0 + lane;
-      const int mine = r < M ? min(row_chunks(positions[row_list ? row_list[r] : r], EXTRA ? window : max(window, 0), keep, FD_CHUNK), num_chunks) : 0;
-      int upto = mine;
+  int items = 1;                                          // (this block's own)
+  if (WALK) {
+    if (warp == 0) {
+      int before = 0;
+      for (int r0 = 0; r0 < M; r0 += 32) {
+        const int r = r0 + lane;
+        const int mine = r < M ? min(row_chunks(positions[row_list ? row_list[r] : r], max(window, 0), 0, FD_CHUNK), num_chunks) : 0;
+        int upto = mine;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int left = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += left;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int left = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += left;
+        }
+        if (r < M) row_first[r] = before + upto - mine;
+        before += __shfl_sync(0xffffffffu, upto, 31);
       }
-      if (r < M) row_first[r] = before + upto - mine;
-      before += __shfl_sync(0xffffffffu, upto, 31);
+      if (lane == 0) row_first[M] = before;
     }
-    if (lane == 0) row_first[M] = before;
+    __syncthreads();                                      // the items are counted
+    items = row_first[M] * nkv;
   }
-  if (WALK) __syncthreads();                              // the items are counted
-  const long long items = (WALK && counted ? (long long)row_first[M] : (long long)M * num_chunks) * nkv;
   // Warp 0 works an item out one ahead, while the copies of the one before are on their way (its lanes keep the pages: a
   // chunk has 32 at the most): behind them the row, its position and its pages were a chain of trips to L2.
-  auto plan = [&](long long item, FdItem& it) {
-    int page = 0;
-    if (item < items) {
-      it.kvh = (int)(item % nkv);
-      if (WALK && counted) {
-        const int w = (int)(item / nkv);
-        int lo = 0, hi = M;                               // the last row whose items begin at w or before
-        while (hi - lo > 1) {
-          const int mid = (lo + hi) >> 1;
-          if (row_first[mid] <= w) lo = mid; else hi = mid;
-        }
-        it.x = lo;
-        it.z = w - row_first[lo];
-      } else {
-        it.x = (int)(item / nkv % M);
-        it.z = (int)(item / nkv / M);
-      }
-      it.m = row_list ? row_list[it.x] : it.x;
-      it.pos = positions[it.m];
-      const int seg = row_seg[it.m];
-      if (EXTRA) {
-        int first = 0, last = 0;
-        bool inside;
-        it.valid = chunk_keys(it.pos, window, keep, FD_CHUNK, it.z, first, last, it.k0, inside);
-        it.k_begin = first;
-        it.k_end = last + 1;
-      } else {
-        const int lo = window > 0 ? max(0, it.pos - window + 1) : 0;
-        const int c = lo / FD_CHUNK + it.z;
-        it.valid = (long long)c * FD_CHUNK <= it.pos;
-        it.k0 = c * FD_CHUNK;
-        it.k_begin = max(lo, it.k0);
-        it.k_end = min(it.pos + 1, it.k0 + FD_CHUNK);
-      }
-      const int first_page = it.k_begin / page_size;
-      if (it.valid && lane <= (it.k_end - 1) / page_size - first_page)
-        page = block_table[(size_t)seg * max_pages + first_page + lane];
+  auto pages_of = [&](const FdItem& it) {
+    const int first_page = it.k_begin / page_size;
+    return lane <= (it.k_end - 1) / page_size - first_page
+        ? block_table[(size_t)row_seg[it.m] * max_pages + first_page + lane] : 0;
+  };
+  auto plan = [&](int item, FdItem& it) {
+    if (item >= items) return 0;
+    const int w = item / nkv;
+    it.kvh = item - w * nkv;
+    int lo = 0, hi = M;                                   // the last row whose items begin at w or before
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (row_first[mid] <= w) lo = mid; else hi = mid;
     }
-    return page;
+    it.x = lo;
+    it.z = w - row_first[lo];
+    it.m = row_list ? row_list[it.x] : it.x;
+    it.pos = positions[it.m];
+    fd_keys<EXTRA>(it, window, keep);
+    return pages_of(it);
+  };
+  auto load_q = [&]() {
+    for (int v = threadIdx.x; v < 16 * CH; v += FA_WARPS * 32) {
+      const int r = v / CH, cc = v % CH;
+      fa_cp_async16(sm_q + swz<CH>(r, cc), q + ((size_t)now.m * nh + now.kvh * group + min(r, group - 1)) * HD + cc * 8,
+                    r < group);
+    }
+    fa_commit();
   };
   int page = 0;
-  FdItem now;
-  if (!WALK || warp == 0) page = plan(blockIdx.x, now);
-  if (WALK && threadIdx.x == 0) planned[0] = now;
-  if (!WALK && !now.valid) return;                        // (the same for all threads)
+  if (WALK) {
+    if (warp == 0) {
+      page = plan(blockIdx.x, now);
+      if (lane == 0) planned[0] = now;
+    }
+  } else {
+    if (warp == 0) page = pages_of(now);
+    load_q();
+  }
   __syncthreads();                                        // the barrier is initialised
   uint32_t phase = 0;
   int turn = 0;
-  for (long long item = blockIdx.x; item < items; item += gridDim.x, turn ^= 1) {
+  for (int item = WALK ? blockIdx.x : 0; item < items; item += gridDim.x, turn ^= 1) {
   if (WALK) now = planned[turn];
   const int m = now.m, kvh = now.kvh, x = now.x, z = now.z, pos = now.pos, k0 = now.k0, k_begin = now.k_begin, k_end = now.k_end;
   if (warp == 0) {
-    if (now.valid) {
-      const int first_page = k_begin / page_size, n_pages = (k_end - 1) / page_size - first_page + 1;
-      if (lane == 0) mbar_expect_tx(&bar, (uint32_t)n_pages * page_size * 128u * 2u * PANELS);
-      __syncwarp();
-      if (lane < n_pages) {
-        const int row = (first_page + lane) * page_size - k0;               // the page's first row in the chunk
-        const int y_k = ((page * k_mul) * nkv + kvh) * page_size, y_v = ((page * k_mul + v_add) * nkv + kvh) * page_size;
+    const int first_page = k_begin / page_size, n_pages = (k_end - 1) / page_size - first_page + 1;
+    if (lane == 0) mbar_expect_tx(&bar, (uint32_t)n_pages * page_size * 128u * 2u * PANELS);
+    __syncwarp();
+    if (lane < n_pages) {
+      const int row = (first_page + lane) * page_size - k0;                 // the page's first row in the chunk
+      const int y_k = ((page * k_mul) * nkv + kvh) * page_size, y_v = ((page * k_mul + v_add) * nkv + kvh) * page_size;
 #pragma unroll
-        for (int p = 0; p < PANELS; ++p) {
-          tma_load_2d(fd_smem + p * PANEL + row * 128, &map_kv, &bar, p * 64, y_k);
-          tma_load_2d(fd_smem + (PANELS + p) * PANEL + row * 128, &map_v, &bar, p * 64, y_v);
-        }
+      for (int p = 0; p < PANELS; ++p) {
+        tma_load_2d(fd_smem + p * PANEL + row * 128, &map_kv, &bar, p * 64, y_k);
+        tma_load_2d(fd_smem + (PANELS + p) * PANEL + row * 128, &map_v, &bar, p * 64, y_v);
       }
-      __syncwarp();
     }
+    __syncwarp();
     if (WALK) {
       FdItem it;
       page = plan(item + gridDim.x, it);
       if (lane == 0) planned[turn ^ 1] = it;
     }
   }
-  if (!now.valid) {
-    __syncthreads();
-    continue;
-  }
-  for (int v = threadIdx.x; v < 16 * CH; v += FA_WARPS * 32) {
-    const int r = v / CH, cc = v % CH;
-    fa_cp_async16(sm_q + swz<CH>(r, cc), q + ((size_t)m * nh + kvh * group + min(r, group - 1)) * HD + cc * 8,
-                  r < group);
-  }
-  fa_commit();
+  if (WALK) load_q();
   fa_wait<0>();
   if (!mbar_try_wait(&bar, phase)) {
     const uint64_t start = global_ns();
@@ -971,7 +993,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const __
       if (global_ns() - start > FD_WAIT_NS) {
         atomicCAS(&g_fd_status, 0, 1);
         drain_after_abort();                              // the copies in flight land before the block goes on and returns
-        gave_up = 1;
+        if (WALK) gave_up = 1;
         break;
       }
     }
@@ -991,7 +1013,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const __
     }
   }
   __syncthreads();
-  if (gave_up) return;                                    // (the same for all threads: it was written before the barrier)
+  if (WALK && gave_up) return;                            // (the same for all threads: it was written before the barrier)
   // byte offset of 16-byte chunk cc of row r in a [PANELS][256][64] tile written by TMA
   auto tile_off = [](int r, int cc) -> uint32_t {
     return (uint32_t)(cc >> 3) * PANEL + (uint32_t)r * 128u + (uint32_t)(((cc & 7) ^ (r & 7)) << 4);
@@ -1144,6 +1166,16 @@ static bool decode_tma_page_ok(int page_size) {
   return page_size >= 8 && page_size <= FD_CHUNK && page_size % 8 == 0 && FD_CHUNK % page_size == 0;
 }
 
+static long long fd_at_once(int sms) { return 3ll * sms; }       // blocks of 67 KB that are on the SMs at once
+static bool fd_walks(int M, int nkv, int num_chunks, int hd, bool extra, int sms) {
+  const long long most = (long long)M * nkv * num_chunks;
+  return hd == 64 && !extra && M <= FD_ROWS && num_chunks >= FD_WALK_CHUNKS && most >= FD_WALK_ROUNDS * fd_at_once(sms) && most < (1ll << 30);
+}
+// For tests: whether a launch of these sizes walks on a device of that many SMs.
+SNK_API int snk_attention_decode_walks(int M, int nkv, int num_chunks, int hd, int extra, int sms) {
+  return fd_walks(M, nkv, num_chunks, hd, extra != 0, sms);
+}
+
 // num_pages: pages in the pool (it is [num_pages, 2, nkv, page_size, hd]).  Page sizes the TMA kernel does
 // not take give SNK_ERR_SIZE (the caller then uses snk_attention_decode_mma).
 static int fd_launch(const void* q, const void* pool, const void* vpool, long long num_pages, const int* block_table,
@@ -1174,13 +1206,11 @@ static int fd_launch(const void* q, const void* pool, const void* vpool, long lo
   // with a cap c the scores become c tanh(scale q . k / c): the tangent's argument, and what then takes the scale's place
   const float cap_in = softcap > 0.f ? 2.f * 1.4426950408889634f * scale / softcap : 0.f;
   const float scale_log2 = (softcap > 0.f ? softcap : scale) * 1.4426950408889634f;
-  // the blocks that are on the SMs at once: three of 67 KB, one of 133
   int sms = 0;
   rc = snk_device_sms(&sms);
   if (rc) return rc;
-  const long long most = (long long)M * nkv * num_chunks, at_once = (long long)sms * (hd == 64 ? 3 : 1);
-  const bool walk = most > FD_WALK_ROUNDS * at_once;
-  const dim3 grid((unsigned)(walk ? at_once : most));
+  const bool walk = fd_walks(M, nkv, num_chunks, hd, extra, sms);
+  const dim3 grid = walk ? dim3((unsigned)fd_at_once(sms)) : dim3(M, nkv, num_chunks);
   const size_t smem = 1024 + (size_t)2 * (hd / 64) * FD_CHUNK * 128 + (size_t)16 * hd * 2;
   float* part_o = static_cast<float*>(scratch);
   float* part_ml = part_o ? part_o + (size_t)M * nh * num_chunks * hd : nullptr;
@@ -1193,21 +1223,16 @@ static int fd_launch(const void* q, const void* pool, const void* vpool, long lo
     snk_launch(attention_decode_tma_kernel<HD_, EXTRA_, WALK_>, dim3(grid), dim3(FA_WARPS * 32), smem, stream, map,     \
                map_v, k_mul, v_add, qp, block_table, max_pages, page_size, positions, row_seg, row_list, op,            \
                part_o, part_ml, nh, nkv, window, num_chunks, scale_log2, keep, slopes, sink, gp, gate_ld,               \
-               cap_in, M, M <= FD_ROWS);                                                                                \
-  } while (0)
-#define FD_EITHER(HD_, EXTRA_)                 \
-  do {                                         \
-    if (walk) FD_LAUNCH(HD_, EXTRA_, true);    \
-    else FD_LAUNCH(HD_, EXTRA_, false);        \
+               cap_in, M);                                                                                              \
   } while (0)
   if (hd == 64) {
-    if (extra) FD_EITHER(64, true);
-    else FD_EITHER(64, false);
+    if (walk) FD_LAUNCH(64, false, true);
+    else if (extra) FD_LAUNCH(64, true, false);
+    else FD_LAUNCH(64, false, false);
   } else {
-    if (extra) FD_EITHER(128, true);
-    else FD_EITHER(128, false);
+    if (extra) FD_LAUNCH(128, true, false);
+    else FD_LAUNCH(128, false, false);
   }
-#undef FD_EITHER
 #undef FD_LAUNCH
   SNK_LAUNCH_CHECK();
   return 0;

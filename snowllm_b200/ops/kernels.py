@@ -50,6 +50,7 @@ _SIGNATURES = {
         "snk_attention_prefill_tma": [P, P, LL, P, I, I, P, I, P, I, I, I, I, F, P],
         "snk_attention_decode_tma": [P, P, LL, P, I, I, P, P, P, P, P, I, I, I, I, I, I, F, P],
         "snk_attention_decode_tma_split": [P, P, P, LL, P, I, I, P, P, P, P, P, I, I, I, I, I, I, F, I, P, P, P, LL, F, P],
+        "snk_attention_decode_walks": [I, I, I, I, I, I],
         "snk_attention_decode_status": [],
         "snk_attention_decode_status_peek": [P, P],
     },

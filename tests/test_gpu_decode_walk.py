@@ -36,3 +36,11 @@ def test_walk(M, chunks, hd, P, window):
     served = torch.zeros(M + 4, dtype=torch.bool)
     served[rows.cpu().long()] = True
     assert (outs[0][~served.cuda()] == 7).all() and outs[0].isfinite().all()
+
+
+# the line from which a launch walks (32 chunks a row, 16 rounds of possible blocks, up to 256 rows of head size 64), its sides, and
+# rows with and without a window; some rows reach one chunk, some nearly all, the last chunk nobody
+@pytest.mark.parametrize("M,chunks", [(27, 32), (28, 32), (64, 31), (64, 33), (256, 32), (257, 32)])
+@pytest.mark.parametrize("P,window", [(64, None), (8, 300), (256, None)])
+def test_walk_at_its_line(M, chunks, P, window):
+    test_walk(M, chunks, 64, P, window)

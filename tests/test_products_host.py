@@ -98,3 +98,12 @@ def test_a_row_gather_that_is_too_short_is_refused(monkeypatch, product):
     for rows_out, listed in ((None, 8), (12, 11)):
         with pytest.raises(KernelError, match="row gather"):
             getattr(kernels, product)(x, w, a_rows=torch.zeros(listed, dtype=torch.int32), rows_out=rows_out)
+
+
+def test_which_decode_attention_launches_walk():
+    """148 SMs hold 444 blocks at once: 16 rounds of them are 7,104 possible blocks."""
+    walks = kernels.fn("snk_attention_decode_walks")
+    for (M, nkv, chunks, hd), want in {(28, 8, 32, 64): 1, (27, 8, 32, 64): 0, (64, 8, 31, 64): 0, (64, 8, 32, 64): 1, (256, 8, 32, 64): 1,
+                                       (257, 8, 32, 64): 0, (64, 8, 64, 128): 0, (1, 8, 888, 64): 1, (1, 8, 887, 64): 0}.items():
+        assert walks(M, nkv, chunks, hd, 0, 148) == want, (M, nkv, chunks, hd)
+        assert not walks(M, nkv, chunks, hd, 1, 148)                # launches with options do not
