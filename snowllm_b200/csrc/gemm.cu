@@ -374,10 +374,13 @@ static int launch_few(const SimtArgs& p) {
     if (e != cudaSuccess) return (int)e;
   }
   // Fewer rows than groups: a block per row and strip, which looks its group up, unless the blocks of all groups are on the SMs at
-  // once (five to each) and the idle ones cost nothing.
+  // once (five to each) and the idle ones cost nothing.  Measured, us, a block per group / per row: 32 groups of 2,048 x 1,792, 4 rows 19.7 / 14.3, 8
+  // 26.7 / 24.2, 16 42.0 / 39.4, 28 59.8 / 58.3; of 3,584 x 2,048, 16 rows 75.4 / 73.1; of 384 x 512 (768 blocks, just above the line), 4 rows 4.4 /
+  // 3.5, 16 5.4 / 5.4; 128 groups of 768 x 512, 4 rows 9.3 / 4.2, 64 24.1 / 21.8; 256 of 256 x 512, 8 rows 7.0 / 4.8, 128 18.6 / 17.7, but 248, with
+  // nearly a row to a group, 25.9 / 26.5.
   const long long strips = (p.N + FR_COLS - 1) / FR_COLS;
   int sms = 0, per_group = p.offsets ? p.groups : 1;
-  if (p.offsets && p.groups > p.M) {
+  if (p.offsets && p.M <= p.groups - (p.groups + 15) / 16) {
     const int rc = snk_device_sms(&sms);
     if (rc) return rc;
     if (strips * p.groups > 5ll * sms) per_group = p.M;

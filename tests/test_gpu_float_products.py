@@ -40,6 +40,31 @@ def test_groups(counts):
         lo += n
 
 
+# Fewer rows than groups, and more strips of 16 columns over all groups than the SMs hold blocks (five each): a block looks the group
+# up that its number stands for (up to 15 rows to 16 groups).  One group of 32 and several of them; empty ones first, last and between; rows in
+# one group alone; 30 rows of 32 groups are the last to be looked up, 31 have a block per group.
+@pytest.mark.parametrize("N,counts", [
+    (3584, [0, 1, 0, 2] * 3 + [0] * 20), (3584, [0] * 31 + [1]), (3584, [1] + [0] * 31), (3584, [0] * 31 + [31]),
+    (3584, [1] * 31 + [0]), (3584, [0] + [1] * 30 + [0]), (3584, [0, 17] + [0] * 29 + [9]), (384, [0, 1] * 16),
+    (260, [0] * 33 + [1, 0, 3] + [0] * 33 + [2]), (260, [0] * 69 + [1]), (112, [(e % 5 == 3) * (1 + e % 3) for e in range(128)])])
+@pytest.mark.parametrize("K", [64, 260])
+def test_fewer_rows_than_groups(N, counts, K):
+    from snowllm_b200.ops import kernels
+    G, M = len(counts), sum(counts)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert M < G and -(-N // 16) * G > 5 * sms
+    x, w = operands(M, K, seed=13), operands(G, N, K, seed=14)
+    rows = torch.randperm(2 * M, generator=torch.Generator().manual_seed(15))[:M].to(torch.int32).cuda()
+    offsets = torch.tensor([0] + counts).cumsum(0).to(torch.int32).cuda()
+    out = torch.full((M, N), float("nan"), device="cuda")
+    kernels.gemm_simt(x, w, a_rows=rows, a_div=2, offsets=offsets, rows_out=M, max_rows_per_group=M, out=out)
+    lo = 0
+    for e, n in enumerate(counts):
+        if n:
+            assert torch.equal(out[lo:lo + n], kernels.gemm_simt(x[(rows[lo:lo + n] // 2).long()].contiguous(), w[e]))
+        lo += n
+
+
 def tile_of(M, N, groups, rows):
     from snowllm_b200.ops import kernels
     sms = torch.cuda.get_device_properties(0).multi_processor_count
