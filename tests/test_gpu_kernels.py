@@ -675,7 +675,7 @@ def test_gemm_tc2_grouped_rows_on_the_n_side(K, N, K_):
                                     [(11 * e) % 37 * 4 for e in range(32)], [(11 * e) % 37 * 4 for e in range(33)],
                                     [(7 * e) % 23 * (e % 5 != 0) for e in range(200)], [(e % 13) * (e % 29) for e in range(256)]])
 def test_gemm_tc2_grouped_rings_and_plans(K, counts):
-    """The grouped pair product where its ring changes (row tiles of up to 64, up to 128 and more rows: 10, 8 and 6 stages),
+    """The grouped pair product where its ring changes (row tiles of up to 64, up to 128 and more rows: 11, 9 and 6 stages),
     with more than two rounds of the ring (26 k-blocks), and both plans: up to 32 groups, longest row tiles first, and
     more, in their own order."""
     G, M, N, K_ = len(counts), sum(counts), 264, 26 * 64

@@ -97,3 +97,34 @@ def test_another_compiler_or_other_flags_are_another_build(monkeypatch):
     monkeypatch.setattr(build.subprocess, "run", lambda *a, **kw: pytest.fail("ran"))        # a path costs no compiler
     monkeypatch.setattr(build, "_nvcc", lambda: pytest.fail("asked for nvcc"))
     assert build.host_path() in paths and len(paths) == 3
+
+
+def kinds(arguments: str) -> list:
+    """The kinds of a C argument list, as ops/kernels.py has them."""
+    out = []
+    if arguments.strip() in ("", "void"):
+        return out
+    for a in re.sub(r"\s+", " ", arguments).split(","):
+        a = a.strip()
+        if "*" in a or re.match(r"(cudaStream_t|S)\b", a):
+            out.append(kernels.P)
+        else:
+            out.append({"long long": kernels.LL, "int": kernels.I, "float": kernels.F}[re.match(r"(?:const )?(long long|int|float)\b", a)[1]])
+    return out
+
+
+def test_every_entry_point_is_declared_as_it_is_defined():
+    """The sources, the table that ctypes goes by, and the types that host.cpp calls through: the same arguments everywhere."""
+    defined = {}
+    for source in CSRC.glob("*.cu"):
+        for name, arguments in re.findall(r"SNK_API (?:int|long long|void) (snk_\w+)\(([^)]*)\)\s*{", source.read_text()):
+            defined[name] = kinds(arguments)
+    declared = {name: args for table in kernels._SIGNATURES.values() for name, args in table.items()}
+    assert len(declared) > 80 and {n: defined.get(n) for n in declared} == declared
+    host = (CSRC / "host.cpp").read_text()
+    types = {t: kinds(a) for t, a in re.findall(r"typedef (?:int|long long) \(\*(\w+)\)\(([^)]*)\);", host)}
+    variables = dict((v, t) for t, v in re.findall(r"^(\w+) (f_\w+);$", host, re.M))
+    entries = re.findall(r'{"(snk_\w+)", \(void\*\*\)&(f_\w+)}', host)
+    assert len(entries) == len(variables) > 10
+    for name, variable in entries:
+        assert types[variables[variable]] == declared[name], name
