@@ -93,7 +93,7 @@ _SIGNATURES = {
         "snk_gemm_tc2_test_lose_loads": [I],
     },
     "moe": {
-        "snk_moe_route": [P, P, I, P, P, P, I, I, I, I, I, F, I, I, P],
+        "snk_moe_route": [P, P, I, P, P, P, I, I, I, I, I, F, I, P],
         "snk_moe_topk": [P, P, P, P, I, I, I, I, F, I, I, P],
         "snk_moe_route_sort": [P, P, I, P, P, P, P, P, P, P, I, I, I, I, I, I, F, I, I, P],
         "snk_moe_sort": [P, P, P, P, I, I, I, P],
@@ -1476,7 +1476,7 @@ def moe_route(x, router_w, bias, top_k, norm_topk_prob, scaling, scoring: str = 
                                  flags, float(scaling), 1, 1, _stream()), "moe_topk")
         return ids, wts
     check(fn("snk_moe_route")(_ptr(x), _ptr(router_w), w32, _ptr(bias), _ptr(ids), _ptr(wts), M, H, E,
-                              top_k, flags, float(scaling), code_of(dtype), int(w_ahead), _stream()),
+                              top_k, flags, float(scaling), code_of(dtype), _stream()),
           "moe_route", work=lambda: (_nbytes(x, router_w, ids, wts), 2 * M * E * H))
     return ids, wts
 
