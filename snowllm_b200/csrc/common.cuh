@@ -168,9 +168,8 @@ __host__ __device__ __forceinline__ int norm_threads(int H) { return H >= 2048 ?
 
 // Thread-block clusters: a barrier over all threads of the cluster's blocks, and the shared memory of
 // another block of the cluster (distributed shared memory) by the address the same variable has here.  (The aligned form wants whole
-// warps: whatever branch a warp's lanes come out of, they meet first.)
+// warps: behind a branch or a wait that a warp's lanes may have left one by one, a __syncwarp comes first.)
 __device__ __forceinline__ void cluster_sync() {
-  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // The float at the same shared-memory address in block `rank` of this cluster.

@@ -140,6 +140,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
+  __syncwarp();
   cluster_sync();                                        // both blocks' barriers and tensor memory are set up
   tc_fence_after();
   // the accumulator's address is the leader's: the MMA writes rows 128..255 at the same columns of the peer
@@ -238,6 +239,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   }
   if (*aborted) drain_after_abort();
   tc_fence_before();
+  __syncwarp();
   cluster_sync();                                        // nobody of the pair touches tensor memory or barriers any more
   if (warp == 1) {
     tc_fence_after();
@@ -443,6 +445,7 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
+  __syncwarp();
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem_acc = rank == 0 ? sh->tmem_base : ld_cluster_u32(&sh->tmem_base, 0);
@@ -569,6 +572,7 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
   }
   if (*aborted) drain_after_abort();
   tc_fence_before();
+  __syncwarp();
   cluster_sync();
   if (warp == 1) {
     tc_fence_after();
