@@ -412,6 +412,36 @@ __device__ __forceinline__ int t2g_box(int half_rows) {
   return b;
 }
 
+// The gated store of a grouped piece of `rows` (up to 32) rows.  Lanes 0..7 and 16..23 hold a column of gates each, the eight behind each
+// their ups: of rows 2 j and 2 j + 1 a gate's lane gives the second for its up's first, and each then has both of one row.  A store
+// writes 16 neighbouring columns of two rows.  Four pairs of rows at a time, their exchanges ahead of their activations and those ahead of
+// their stores, and no more than there are rows: with halves of 16 rows exchanged, activated and stored one after the other
+// an item's epilogue was one chain of 16, and longer than its products where K or the rows were few.  Measured, us, so before / now, 128
+// groups of 768 x 512 and the top 8 of them: 200 tokens 38.2 / 31.7, 1,024 46.8 / 41.3; 32 groups of 3,584 x 2,048, top 4: 64 tokens 84 /
+// 82, 276 92.9 / 88.4, 2,048 195 / 161, 4,096 304 / 272.  Eight pairs at a time 83.8 and 167 instead of 83.6 and 161 (100 and 2,048
+// tokens), all sixteen 86.5 and 172.
+template <typename OutT>
+__device__ __forceinline__ void t2g_glu_store(uint32_t (&r)[32], int lane, OutT* __restrict__ dst, int ld, int mine, int rows, int act) {
+  const int up = (lane >> 3) & 1;
+  dst += (size_t)up * ld + (lane & 7) + ((lane >> 4) << 3);
+  mine -= up;
+#pragma unroll
+  for (int j0 = 0; j0 < 16; j0 += 4) {
+    if (2 * j0 >= rows) break;                           // (the same for all lanes)
+#pragma unroll
+    for (int j = j0; j < j0 + 4; ++j) {
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, up ? r[2 * j] : r[2 * j + 1], 8);
+      if (up) r[2 * j] = other;
+      else r[2 * j + 1] = other;
+    }
+#pragma unroll
+    for (int j = j0; j < j0 + 4; ++j) r[2 * j] = __float_as_uint(glu_out(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]), act));
+#pragma unroll
+    for (int j = j0; j < j0 + 4; ++j)
+      if (2 * j < mine) dst[(size_t)(2 * j) * ld] = from_f<OutT>(__uint_as_float(r[2 * j]));
+  }
+}
+
 template <typename OutT, bool SWIGLU>
 __global__ void __launch_bounds__(64 + 32 * T2_EPI_WARPS)
 gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_constant__ CUtensorMap map_w,
@@ -538,18 +568,7 @@ gemm_tc2_grouped_kernel(const __grid_constant__ T2GMaps maps, const __grid_const
         if (c0 + 64 >= t.nt) release();
         const int rows = t.row_end - (t.row0 + c0);      // of this piece and the ones behind it
         if constexpr (SWIGLU) {
-          // Lanes 0..7 and 16..23 hold gates, the eight behind each their ups: a gate's lane gives its rows 16..31 for its
-          // up's rows 0..15, and each then has both of 16 rows.  A store writes 16 neighbouring columns of two rows.
-          const bool up = lane & 8;
-          const int f = (lane & 7) + ((lane >> 4) << 3), ahead = up ? 16 : 0;
-          const bool ok = col0 + (lane & 16) + 16 <= N;
-          OutT* dst = C + (size_t)(t.row0 + c0 + ahead) * (N / 2) + col0 / 2 + f;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float other = __uint_as_float(__shfl_xor_sync(0xffffffffu, up ? r[j] : r[16 + j], 8));
-            const float gate = up ? other : __uint_as_float(r[j]), upv = up ? __uint_as_float(r[16 + j]) : other;
-            if (ok && ahead + j < rows) dst[(size_t)j * (N / 2)] = from_f<OutT>(glu_out(gate, upv, act));
-          }
+          t2g_glu_store(r, lane, C + (size_t)(t.row0 + c0) * (N / 2) + col0 / 2, N / 2, col0 + (lane & 16) + 16 <= N ? rows : 0, rows, act);
         } else if (col0 + lane < N) {
           // a warp's store writes 32 neighbouring columns of one row
           OutT* dst = C + (size_t)(t.row0 + c0) * N + col0 + lane;
