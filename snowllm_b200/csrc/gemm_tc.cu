@@ -9,7 +9,7 @@
 //                      memory into a float accumulator in tensor memory; tcgen05.commit hands the stage
 //                      back to the producer and, after the last k-block, the accumulator to the epilogue
 //   warps 2..9         epilogue: tcgen05.ld of the accumulator (each warp its 32 lanes = 32 rows of C, and one half of
-//                      the columns), conversion, guarded stores
+//                      the columns; warps 2..5 of a split product all of them), conversion, guarded stores
 //
 // There are two accumulators in tensor memory (2 x BN columns): the epilogue of one tile runs while
 // the next tile's products are issued.
@@ -33,8 +33,12 @@
 
 #define TC_BM 128
 #define TC_BK 64
-#define TC_EPI_WARPS 8                 // two to each 32 lanes of tensor memory, which share a tile's columns
-#define TC_THREADS (64 + 32 * TC_EPI_WARPS)
+// Epilogue warps: two to each 32 lanes of tensor memory, which share a tile's columns; one where a product is split along K, whose
+// blocks have one short tile each and are soon followed by other kernels' on the same SMs (with two the kernel alone is as fast, but
+// in a chain of norm, gated product and product, us, two / one: 2,048 x 1,536 200 rows 26.1 / 23.8, 2,048 x 1,024 129 rows 24.1 / 22.0, 1,024 x
+// 1,408 64 rows 17.3 / 18.1).
+#define TC_EPI_WARPS 8
+#define TC_SPLIT_EPI_WARPS 4
 #define TC_SMEM_TILES (192 * 1024)    // bytes of shared memory given to the operand stages
 #ifndef TC_BAND
 #define TC_BAND 8                     // n-tiles in a band of the tile order (8, 16 and 28 measured; 8 is best or equal everywhere)
@@ -72,6 +76,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 
 #define TC_MAX_STAGES 6
 
+template <int EPI>
 struct __align__(16) TcShared {
   uint64_t full[TC_MAX_STAGES];
   uint64_t empty[TC_MAX_STAGES];
@@ -79,7 +84,7 @@ struct __align__(16) TcShared {
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   int aborted;
-  __align__(16) float stage_out[TC_EPI_WARPS][TC_STAGE_FLOATS];    // one staging tile per epilogue warp (tc_store_piece)
+  __align__(16) float stage_out[EPI][TC_STAGE_FLOATS];    // one staging tile per epilogue warp (tc_store_piece)
 };
 
 // Rows of C and rows of W that tile `tile` covers.  Plain: tiles = row_tiles * n_tiles, row tile fastest.
@@ -134,8 +139,8 @@ __device__ __forceinline__ TcTile tc_tile(int tile, int row_tiles, int M, int N,
 // 8j..8j+7, rows 16j+8..16j+15: their up rows); the store is act(gate) * up into C[M, N/2], act by the code
 // that the entry point's `swiglu` argument carries (1 silu, 2 relu, 3 gelu in its tanh form).
 // ADD (float): the product is added to what C holds (the stream that a sublayer's output belongs to).
-template <int BN, typename OutT, bool SWIGLU, bool ADD>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+template <int BN, typename OutT, bool SWIGLU, bool ADD, int EPI>
+__global__ void __launch_bounds__(64 + 32 * EPI, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                OutT* __restrict__ C, int M, int N, int K, const int* __restrict__ offsets, int groups,
                int row_tiles_bound, int splits, int act, int w_ahead) {
@@ -146,7 +151,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   extern __shared__ unsigned char smem_raw[];
   // tiles need 1024-byte alignment for the 128-byte swizzle
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  TcShared* sh = reinterpret_cast<TcShared*>(tiles + (size_t)STAGES * STAGE_BYTES);
+  TcShared<EPI>* sh = reinterpret_cast<TcShared<EPI>*>(tiles + (size_t)STAGES * STAGE_BYTES);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k_tiles = (K + TC_BK - 1) / TC_BK;
@@ -160,7 +165,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sh->acc_full[b], 1);
-      mbar_init(&sh->acc_empty[b], TC_EPI_WARPS);        // one arrival per epilogue warp
+      mbar_init(&sh->acc_empty[b], EPI);                 // one arrival per epilogue warp
     }
     sh->aborted = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -260,7 +265,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else {
     const int lane_group = warp & 3;                     // a warp reads the 32 tensor-memory lanes 32*(warp%4)..
-    const int c_begin = (warp - 2) / 4 * 32;             // the two warps of 32 lanes take the tile's pieces in turns
+    constexpr int STEP = EPI * 8;                        // the warps of 32 lanes take the tile's pieces of 32 columns in turns
+    const int c_begin = (warp - 2) / 4 * 32;
     float* stage_out = sh->stage_out[warp - 2];
     int local = 0;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
@@ -273,17 +279,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (!mbar_wait_warp(&sh->acc_full[buf], (local >> 1) & 1, aborted, TC_ERR_WAIT_ACC)) break;
       tc_fence_after();
 #pragma unroll 1
-      for (int c0 = c_begin; c0 < BN; c0 += 64) {
+      for (int c0 = c_begin; c0 < BN; c0 += STEP) {
         uint32_t r[32];
         tmem_ld32(tmem_acc + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)(buf * BN + c0), r);
-        if (c0 + 64 >= BN) {                             // everything of this warp's part is in registers
+        if (c0 + STEP >= BN) {                            // everything of this warp's part is in registers
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&sh->acc_empty[buf]);
         }
         if (!*aborted)
           tc_store_piece<OutT, SWIGLU, ADD>(r, stage_out, lane, Cp, t.row0 + lane_group * 32, t.row_end, t.n0 + c0, N, act, old);
-        if (c0 + 64 < BN) tc_load_old<ADD>(old, lane, Cp, t.row0 + lane_group * 32, t.row_end, t.n0 + c0 + 64, N);
+        if (c0 + STEP < BN) tc_load_old<ADD>(old, lane, Cp, t.row0 + lane_group * 32, t.row_end, t.n0 + c0 + STEP, N);
       }
       ++local;
     }
@@ -299,20 +305,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
-template <int BN, typename OutT, bool SWIGLU, bool ADD = false>
+template <int BN, typename OutT, bool SWIGLU, bool ADD = false, int EPI = TC_EPI_WARPS>
 static int launch_tc(const CUtensorMap& map_a, const CUtensorMap& map_w, void* C, int M, int N, int K,
                      const int* offsets, int groups, int row_tiles, int splits, int w_ahead, cudaStream_t stream,
                      int act = SNK_GLU_SILU) {
   constexpr int STAGE_BYTES = (TC_BM + BN) * TC_BK * 2;
   constexpr int STAGES = TC_SMEM_TILES / STAGE_BYTES < TC_MAX_STAGES ? TC_SMEM_TILES / STAGE_BYTES : TC_MAX_STAGES;
-  const size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + sizeof(TcShared);
+  const size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + sizeof(TcShared<EPI>);
   static std::atomic<int> ready[SNK_MAX_DEVICES];
   int sms = 0;
-  const int rc = snk_kernel_ready(ready, gemm_tc_kernel<BN, OutT, SWIGLU, ADD>, smem, &sms);
+  const int rc = snk_kernel_ready(ready, gemm_tc_kernel<BN, OutT, SWIGLU, ADD, EPI>, smem, &sms);
   if (rc) return rc;
   const long long tiles = (long long)row_tiles * ((N + BN - 1) / BN) * splits;
   const int blocks = (int)(tiles < sms ? tiles : sms);     // one block per SM (shared memory), persistent
-  snk_launch(gemm_tc_kernel<BN, OutT, SWIGLU, ADD>, dim3(blocks), dim3(TC_THREADS), smem, stream, map_a, map_w, static_cast<OutT*>(C), M, N, K,
+  snk_launch(gemm_tc_kernel<BN, OutT, SWIGLU, ADD, EPI>, dim3(blocks), dim3(64 + 32 * EPI), smem, stream, map_a, map_w, static_cast<OutT*>(C), M, N, K,
                                                                  offsets, groups, row_tiles, splits, act, w_ahead);
   SNK_LAUNCH_CHECK();
   return 0;
@@ -334,6 +340,8 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ parts, OutT* __re
     const size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= blocks) return;
     float g[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, u[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    // four planes' vectors on their way at a time (one by one 64 rows of 3,072 columns came to 15.2 us, product and this, 13.5 so)
+#pragma unroll 4
     for (int p = 0; p < splits; ++p) {
       const float4* src = reinterpret_cast<const float4*>(parts + (size_t)p * plane + b * 16);
       const float4 g0 = src[0], g1 = src[1], u0 = src[2], u1 = src[3];
@@ -464,7 +472,7 @@ SNK_API int snk_gemm_tc(const void* A, const void* W, void* C, int M, int N, int
   rc = tensor_map(W, (long long)(offsets ? groups : 1) * N, K, bn, TC_BK, &map_w);
   if (rc) return rc;
   if (splits > 1) {
-    rc = launch_tc<128, float, false>(map_a, map_w, scratch, M, N, K, nullptr, 1, row_tiles, splits, w_ahead, stream);
+    rc = launch_tc<128, float, false, false, TC_SPLIT_EPI_WARPS>(map_a, map_w, scratch, M, N, K, nullptr, 1, row_tiles, splits, w_ahead, stream);
     if (rc) return rc;
     const float* parts = static_cast<const float*>(scratch);
     const size_t work = swiglu ? (size_t)M * N / 16 : (size_t)M * N / 4;
@@ -502,7 +510,7 @@ SNK_API int snk_gemm_tc_parts(const void* A, const void* W, void* parts, int M, 
   rc = tensor_map(W, N, K, 128, TC_BK, &map_w);
   if (rc) return rc;
   *splits_out = splits;
-  return launch_tc<128, float, false>(map_a, map_w, parts, M, N, K, nullptr, 1, (M + TC_BM - 1) / TC_BM, splits, w_ahead, stream);
+  return launch_tc<128, float, false, false, TC_SPLIT_EPI_WARPS>(map_a, map_w, parts, M, N, K, nullptr, 1, (M + TC_BM - 1) / TC_BM, splits, w_ahead, stream);
 }
 
 // Test hook: with on != 0 the producers of later launches issue no loads, so that the bounded waits run out
