@@ -89,8 +89,9 @@ struct __align__(16) AtShared {
   int aborted;
 };
 
-// False: the wait ran out, or another one of the block has.
-__device__ __noinline__ bool at_wait_long(uint64_t* bar, uint32_t parity, volatile int* aborted, int code) {
+// False: the wait ran out, or another one of the block has.  (Part of the code around it: as a call, beside the 128 scores that a
+// softmax thread holds, it cost 2,048 rows at 30,720 842 us instead of 820.)
+__device__ __forceinline__ bool at_wait_long(uint64_t* bar, uint32_t parity, volatile int* aborted, int code) {
   // the clock is read once in 64 polls: reading it costs more than a poll, and a waiter that is busy
   // reading it sees the barrier late
   uint64_t start = 0;
@@ -317,8 +318,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
       for (int k = 0; k < AT_HD / 16; ++k)                 // 16 elements of q = 8 columns of tensor memory
         umma_bf16_ta(tmem, tmem + AT_TMEM_Q + k * 8, k_lo + 2 * k, idesc_s, k > 0 ? 1u : 0u, elected);
-      umma_commit_if(smem_u32(&sh->s_full), elected);
       umma_commit_if(smem_u32(&sh->k_empty[ks]), elected);
+      umma_commit_if(smem_u32(&sh->s_full), elected);
       if (++ks == AT_KSTAGES) {
         ks = 0;
         k_lap ^= 1;
@@ -328,7 +329,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     if (at_wait_warp(&sh->q_ready, 0, aborted, AT_ERR_Q) && scores(0)) {
       for (int j = 0; j < n_kt; ++j) {
         if (j + 1 < n_kt && !scores(j + 1)) break;
-        if (!at_wait_warp(&sh->v_full[vs], v_lap, aborted, AT_ERR_KV) || !at_wait_warp(&sh->p_full, j & 1, aborted, AT_ERR_P)) break;
+        if (!at_wait_warp(&sh->p_full, j & 1, aborted, AT_ERR_P) || !at_wait_warp(&sh->v_full[vs], v_lap, aborted, AT_ERR_KV)) break;
         tc_fence_after();
         const uint32_t v_lo = v_ring + vs * (AT_KV_BYTES >> 4);
 #pragma unroll
@@ -336,8 +337,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           // P: panel kk / 4 (64 keys), 32 bytes per k-step inside it; V: 16 keys = 16 rows of 128 bytes further
           umma_bf16_lo(tmem + AT_TMEM_O, p_lo + (kk >> 2) * (AT_BQ * 128 >> 4) + (kk & 3) * 2, v_lo + kk * (16 * 128 >> 4),
                        idesc_o, (j > 0 || kk > 0) ? 1u : 0u, elected);
-        umma_commit_if(smem_u32(&sh->pv_done), elected);
         umma_commit_if(smem_u32(&sh->v_empty[vs]), elected);
+        umma_commit_if(smem_u32(&sh->pv_done), elected);
         if (++vs == AT_VSTAGES) {
           vs = 0;
           v_lap ^= 1;
