@@ -6,6 +6,7 @@ be mixed and cut anywhere (the role of runner.forward, snowllm/engine/runner.py:
 its split into prefill-only and decode-only batches)."""
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass, field
 from typing import Sequence
 
@@ -52,7 +53,7 @@ class ModelRunner:
         self.tokens = 0
         self.taps = None       # set to a list to collect what parts tap (tests and debugging)
         self.use_graphs = use_graphs
-        self.graphs = GraphCache(max_graphs, graph_ceiling_bytes, in_use=self._bytes_in_use,
+        self.graphs = GraphCache(max_graphs, graph_ceiling_bytes, in_use=functools.partial(_bytes_in_use, self.device),
                                  release=torch.cuda.empty_cache, oom_errors=(torch.OutOfMemoryError,))
         self.graph_pool = None
         self.graph_replays = 0
@@ -86,10 +87,6 @@ class ModelRunner:
                              pending_tokens=self.pending_tokens, **kw)
 
     # -- decode steps as CUDA graphs ------------------------------------------------------------
-    def _bytes_in_use(self) -> int:
-        free, total = torch.cuda.mem_get_info(self.device)
-        return total - free
-
     def _graph_step(self, entries):
         """Replay the capture that serves this step (made now, if there is room for it); None when the
         step has to run launch by launch."""
@@ -131,6 +128,13 @@ class ModelRunner:
             graph.logits = self.model.forward(ctx, self.cache)
         graph.graph = g
         return graph
+
+
+def _bytes_in_use(device) -> int:
+    """Device memory in use.  (No method: what the runner's captures keep would then keep the runner, and with it the model and the
+    cache, until the collector comes by.)"""
+    free, total = torch.cuda.mem_get_info(device)
+    return total - free
 
 
 def _pow2_at_least(n: int) -> int:

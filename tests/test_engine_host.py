@@ -291,3 +291,30 @@ def test_no_garbage_is_collected_while_a_step_is_captured():
         assert not gc.isenabled()
     finally:
         gc.enable()
+
+
+def test_a_dropped_runner_lets_go_at_once(monkeypatch):
+    """The model and the cache behind a runner are gigabytes: they go with the last reference, not when the collector comes by."""
+    import gc
+    import weakref
+    import torch
+    from snowllm_b200.cache import CacheManager
+    from snowllm_b200.engine import ModelRunner
+    from snowllm_b200.loader import build_model
+    from snowllm_b200.ops import kernels
+    from tiny_configs import ALL
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(kernels, "libraries_for", lambda names: None)
+    model = build_model(ALL["tiny_a"], "float32")
+    model.bound = True
+    cache = CacheManager(model.cache_specs(), 16, 8, 2, model.dtype, "cpu")
+    runner = ModelRunner(model, cache, "cpu", use_graphs=True)
+    alive = [weakref.ref(x) for x in (runner, model, cache)]
+    enabled = gc.isenabled()
+    gc.disable()
+    try:
+        del runner, model, cache
+        assert [x() for x in alive] == [None] * 3
+    finally:
+        if enabled:
+            gc.enable()
