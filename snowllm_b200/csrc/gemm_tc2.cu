@@ -23,7 +23,7 @@
 #define T2_BN 256                     // columns of C per pair; each block loads T2_BN / 2 rows of W
 #define T2_BK 64
 // Epilogue warps of each block: two to each 32 lanes of tensor memory, which share a tile's columns, where one was what a tile
-// waited for: the gated store (8,192 x 16,384 x 2,048, one / two warps: 405 / 342 us = 1.6 PFLOP/s) and the grouped products (2,048
+// waited for: the gated store (8,192 x 16,384 x 2,048, one / two warps: 405 / 342 us alone) and the grouped products (2,048
 // tokens, down 78.4 / 73.4 us).  The plain stores of the ungrouped product stay behind its products with one (8,192 x 6,144 x 2,048
 // 136.5 / 136.7 us).
 #define T2_EPI_WARPS 8
@@ -286,10 +286,11 @@ static int launch_tc2(const CUtensorMap& map_a, const CUtensorMap& map_w, void* 
 // Groups of few rows are bound by the read of W, and that by the bytes an SM keeps on their way: a stage's part for A
 // is as large as the longest row tile of the launch needs, and the ring has as many stages as then fit (11 of 20 KB,
 // 9 of 24 KB, 6 of 32 KB; a plain TMA read loop: 5.3 TB/s with 64 KB of an SM in flight, 6.4 with 128 KB).
-// Measured, 32 groups, gate|up of 2,048 x 3,584, tokens with the top 4 of 32, us (an issuing lane, one epilogue warp to 32 lanes and
-// the offsets read for each item / so): 16 tokens 78 / 74 = 6.3 TB/s, 64 87.7 / 78.4, 276 89.5 / 81.4, 1,024 103 / 95, 2,048 150 / 140, 4,096
-// 236 / 221; down 48.7 / 42.3, 49.4 / 44.3, 51.7 / 46.4, 62 / 54, 83.6 / 73.4, 127 / 114.  (Also tried: tiles of 224 or 240 columns where they fill the last round better, 89.5 us at 8 rows and
-// slower from 256 rows on, where an item costs its full M of 256 whatever it keeps.)
+// Measured in turn, 32 groups, gate|up of 2,048 x 3,584 with its gate, tokens with the top 4 of 32, us (an issuing lane, one epilogue
+// warp to 32 lanes, the offsets read for each item / so): 16 tokens 64.9 / 62.1, 64 87.0 / 80.4 = 5.8 TB/s, 276 89.0 / 83.3, 1,024 121 / 99.8, 2,048 210 /
+// 155, 4,096 349 / 254; down of 1,792 x 2,048 37.5 / 35.2, 47.7 / 45.4, 49.9 / 47.1, 59.7 / 52.9, 83.4 / 74.4, 129 / 116.  (Also tried: tiles of 224
+// or 240 columns where they fill the last round better, 89.5 us at 8 rows and slower from 256 rows on, where an item costs its
+// full M of 256 whatever it keeps.)
 #define T2G_MAX_GROUPS 256
 #define T2G_W_BYTES (T2_BM * T2_BK * 2)               // of a stage: 128 rows of W, then 128, 64 or 32 of the tile's rows of A
 #define T2G_RING_BYTES (11 * (T2G_W_BYTES + 32 * T2_BK * 2))     // the largest of the three rings

@@ -18,11 +18,11 @@ __device__ __forceinline__ uint32_t instr_desc_bf16(int m, int n) {
 }
 
 // D += A B, both operands by the low words of their descriptors.  For a loop that a whole warp walks with one lane issuing
-// (`elected`): the instruction carries the lane's predicate, so that no branch stands around it and all that leads up to it is the
-// same in every lane; the loop's waits are the warp's (mbar_wait_warp).  An issuing lane of its own, with its branch, descriptors formed for each instruction and three reads of the
-// abort word a k-block, took 620 cycles per k-block of 64 whatever the tile: more than the 512 that the products of a
-// 256-column tile take.  Measured, such a lane / so, us: 8,192 x 6,144 x 2,048 157 / 137, 8,192 x 2,048 x 8,192 218 / 195, 1,024 x 2,048 x
-// 8,192 50 / 37, experts' gate|up of 64 tokens (32 groups of 3,584 x 2,048) 87.7 / 77.8 = 6.0 TB/s, of 2,048 tokens 150 / 141.
+// (`elected`): the instruction carries the lane's predicate, so that no branch stands around it, and all that leads up to it is the
+// same in every lane; the loop's waits are the warp's (mbar_wait_warp).  An issuing lane of its own, with its branch, descriptors
+// formed for each instruction and three reads of the abort word a k-block, took 620 cycles per k-block of 64 whatever the tile: more than
+// the 512 that the products of a 256-column tile take.  Measured in turn, us, such a lane / so, on pairs of SMs: 8,192 x 6,144 x 2,048 160 /
+// 142, 8,192 x 2,048 x 8,192 207 / 191, 4,096 x 6,144 x 2,048 86.8 / 83.4; on one: 8,192 x 6,144 x 2,048 169 / 159, 1,024 x 2,048 x 8,192 54.1 / 49.2.
 __device__ __forceinline__ void umma_bf16_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate,
                                              uint32_t elected) {
   asm volatile(
