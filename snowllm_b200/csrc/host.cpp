@@ -327,7 +327,7 @@ PyObject* route_sort(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // (gate_up, interleaved) -> silu(gate) * up
 PyObject* swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 2 || !f_swiglu) Py_RETURN_NONE;
+  if (n != 2 || !f_swiglu || !PyBool_Check(a[1])) Py_RETURN_NONE;       // (1 for True is the long way's)
   GUARD_BEGIN
   const at::Tensor* h = tensor(a[0]);
   if (!h || (h->scalar_type() != F32 && h->scalar_type() != BF16) || h->dim() != 2 || h->size(1) % 2) Py_RETURN_NONE;

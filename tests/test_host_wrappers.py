@@ -56,6 +56,17 @@ with FakeTensorMode():
         print(out)
 """
 
+LAYOUT_AS_A_NUMBER = """
+import ctypes, torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from snowllm_b200.csrc import build
+host = build.load_host()
+host.bind("snk_swiglu", ctypes.cast(ctypes.CFUNCTYPE(ctypes.c_int)(lambda: 0), ctypes.c_void_p).value)
+with FakeTensorMode():
+    for interleaved in (1, 0, None):
+        print(host.swiglu(torch.empty(4, 32, device="cuda"), interleaved))
+"""
+
 
 def run(program: str) -> list:
     done = subprocess.run([sys.executable, "-c", program], cwd=CSRC.parent.parent, capture_output=True, text=True, timeout=300)
@@ -71,6 +82,11 @@ def test_a_tensor_without_memory_raises():
 def test_what_is_no_number_goes_the_long_way():
     """The wrappers in Python say what is wrong with it; these return None for that, and leave no error behind them."""
     assert run(NOT_A_NUMBER) == ["None"] * 6
+
+
+def test_a_layout_that_is_no_truth_value_goes_the_long_way():
+    """Only True meant interleaved columns to the short way, where the wrapper in Python takes any number for one."""
+    assert run(LAYOUT_AS_A_NUMBER) == ["None"] * 3
 
 
 def test_without_the_module_the_wrappers_in_python_do_the_work(monkeypatch):
