@@ -1196,10 +1196,12 @@ class PendingNorm:
             if not _alone(residual):
                 return False
             if _pieces_with_rows(delta):
-                pieces = delta.weights.shape[1]
+                pieces, rows = delta.weights.shape[1], delta.y
             elif isinstance(delta, torch.Tensor):
-                pieces = 1
+                pieces, rows = 1, delta
             else:
+                return False
+            if rows.data_ptr() % 16:         # the norm's own kernel takes a delta as it lies
                 return False
         return (w.data_ptr() % 16 == 0 and residual.data_ptr() % 16 == 0
                 and _norm_product_sizes_ok(M, w.shape[0], K, pieces))

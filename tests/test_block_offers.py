@@ -109,3 +109,12 @@ def test_a_stream_that_somebody_else_looks_at_stays_where_it_is(monkeypatch):
         assert ok(None)                                  # nothing is added: the stream is not moved
         del held
         assert ok(delta)
+
+
+def test_a_delta_off_a_16_byte_boundary_is_left_to_the_norm_s_kernel(monkeypatch):
+    """The norm's kernel takes such a delta an element at a time; a product that forms the norm reads 16 bytes and refuses it."""
+    monkeypatch.setattr(kernels, "_norm_product_sizes_ok", lambda *sizes: True)
+    residual, gamma, w = torch.zeros(2, 64), torch.ones(64, dtype=torch.bfloat16), torch.zeros(4096, 64, dtype=torch.bfloat16)
+    for lead in range(5):
+        delta = torch.ones(lead + 128)[lead:].view(2, 64)
+        assert kernels.PendingNorm.ok(residual, delta, gamma, torch.bfloat16, w) == (lead % 4 == 0)
