@@ -62,7 +62,9 @@ class ModelRunner:
     def step(self, entries: Sequence[StepEntry]) -> torch.Tensor:
         """Run one batch; returns float logits [wanted rows, vocab] in entry order, then ``want``
         order.  Every entry's pages must have been taken already (``CacheManager.ensure``).  The
-        tensor may be overwritten by the next step."""
+        tensor may be overwritten by the next step.  A kernel whose bounded wait ran out is not looked for here, as that takes
+        a wait for the step: whoever reads the logits queues a ``kernels.StatusWatch``'s ``peek()`` behind the step and calls its
+        ``check()`` once they are there (``Engine`` and ``Replay`` do)."""
         entries = [e for e in entries if len(e.tokens) > 0]
         if not entries:
             return torch.empty(0, self.model.vocab_size, dtype=torch.float32, device=self.device)
